@@ -66,9 +66,8 @@ struct BatchTask {
     long long unit0, units;    // first work unit, number of units
     long long grid_off;        // doubles: nch * dims * (bins+1)
     long long hist_off;        // doubles: nch * dims * bins
-    long long hint_off;        // bin-search hints (uint32): nch * dims * kHintPerBin * bins
-    long long width_off;       // bin widths (doubles): nch * dims * bins
-    long long sorted_off;      // monotone flags (bytes): nch * dims
+    long long cell_off;        // search entries (uint32): nch * dims * grid_cells(bins)
+    long long width_off;       // scaled bin widths (doubles): nch * dims * width_row(bins)
     int32_t ch_off;            // first ChannelProgram / channel-weight slot
     int32_t desc;              // IntegrandDesc index
     int32_t pp;                // PointProgram index, -1: per-channel weights
@@ -111,9 +110,8 @@ struct BatchDev {
     const PointProgram *pps;
     const IntegrandDesc *descs;
     double *grids, *grids_new, *hist, *atrain;  // atrain per channel slot
-    uint32_t *hints;                            // bin-search tables of the grids (BatchTask offsets)
+    uint32_t *cells;                            // search tables of the grids (BatchTask offsets)
     double *widths;
-    uint8_t *sorted;
     double *alpha, *best, *mindiff, *cp;        // per channel slot; mindiff per task
     double *part;                              // [nunits][6], task-contiguous
     double *stats;                             // [iter slot][ntasks][6]
@@ -323,7 +321,7 @@ __device__ __forceinline__ void bt_accum_block(const BatchDev &B, int ti, long l
                                                const double *__restrict__ rec_val,
                                                const double *__restrict__ rec_wgt,
                                                const uint8_t *__restrict__ rec_ok,
-                                               const int32_t *__restrict__ rec_slot,
+                                               const uint4 *__restrict__ rec_bins,
                                                const double *__restrict__ rec_dens, long long mr, long long bx,
                                                const RoundCtl *__restrict__ ctl = nullptr,
                                                RetryState *__restrict__ R = nullptr) {
@@ -360,10 +358,9 @@ __device__ __forceinline__ void bt_accum_block(const BatchDev &B, int ti, long l
         if (val != 0) {
             const double v2 = val * val;
             double *H = B.hist + T.hist_off;
-            for (int j = 0; j < T.dims; ++j) {
-                const int s = rec_slot[j * mr + r];
+            for_each_train_slot(rec_bins, r, T.dims, T.bins, [&](int s) {
                 if (s >= 0) atomicAdd(H + s, v2);
-            }
+            });
             vw = v2 * rec_wgt[r];
         }
     }
@@ -416,9 +413,9 @@ __global__ void __launch_bounds__(kFwdBlock) k_bt_accum(BatchDev B, int ti, long
                                                         const double *__restrict__ rec_val,
                                                         const double *__restrict__ rec_wgt,
                                                         const uint8_t *__restrict__ rec_ok,
-                                                        const int32_t *__restrict__ rec_slot,
+                                                        const uint4 *__restrict__ rec_bins,
                                                         const double *__restrict__ rec_dens, long long mr) {
-    bt_accum_block(B, ti, p0, mm, block_count, block_off, rec_val, rec_wgt, rec_ok, rec_slot, rec_dens, mr,
+    bt_accum_block(B, ti, p0, mm, block_count, block_off, rec_val, rec_wgt, rec_ok, rec_bins, rec_dens, mr,
                    blockIdx.x);
 }
 
@@ -436,10 +433,8 @@ struct Piece {
     int32_t n_items[3], n_chains, nch, dims, bins;
     long long p0, mm, ms;
     const PointProgram *pp;
-    const double *grids, *alpha;
-    const uint32_t *hints;  // the task's bin-search tables (rows of its grids)
-    const double *widths;
-    const uint8_t *sorted;
+    GridTables tables;  // the task's grids and their search tables
+    const double *alpha;
     const IntegrandDesc *f;
     double *mom;
     int32_t *ich;
@@ -448,12 +443,12 @@ struct Piece {
     long long *boff;
     RoundCtl *ctl;
     int32_t *list;
-    double *node, *memo, *dcv, *vwv;
+    double *node, *memo, *vwv;
     uint8_t *cfail;
     int32_t *ich_tile;
     double *val, *wgt;
     uint8_t *ok;
-    int32_t *slot;
+    uint4 *bin_rec;
     double *dens;
 };
 enum { GS_FWD, GS_COMPACT, GS_NODES, GS_ITEM0, GS_ITEM1, GS_ITEM2, GS_CHAINS, GS_CHANNEL, GS_COMBINE, GS_ACCUM,
@@ -559,62 +554,37 @@ __global__ void __launch_bounds__(256) k_g_chains(WaveDev W, int lo, int hi, lon
                     lb / P.n_chains);
 }
 
-// Pieces [lo, hi) of the wave have DIMS dimensions. A block works on one
-// channel c of one piece; TAB: the block first stages channel c's edges,
-// bin widths, hint tables and monotone flags (dynamic shared memory) and runs
-// the hinted bin search of the single-integrand path on them, instead of a
-// plain binary search through L1 on the edges in global memory.
+// Pieces [lo, hi) of the wave have DIMS dimensions. A block works on W.ch_pts
+// points of one channel c of one piece (pp_channel_block; TAB: the channel's
+// tables in dynamic shared memory).
 template <int DIMS, bool TAB>
-__global__ void __launch_bounds__(128) k_g_channel(WaveDev W, int lo, int hi, long long blk0) {
+__global__ void __launch_bounds__(256) k_g_channel(WaveDev W, int lo, int hi, long long blk0) {
+    extern __shared__ __align__(16) char smem[];
     CHILI_PIECE(GS_CHANNEL)
     const int c = static_cast<int>(lb % P.nch);
     const long long i0 = (lb / P.nch) * W.ch_pts;  // W.ch_pts points per block: one table copy for all of them
-    const long long n = P.ctl->n_acc;
-    if constexpr (TAB) {
-        extern __shared__ double se[];
-        const int bins = P.bins, H = kHintPerBin * bins;
-        const int ne = DIMS * (bins + 1), nw = DIMS * bins, nh = DIMS * H;
-        double *sw = se + ne;
-        uint32_t *sh = reinterpret_cast<uint32_t *>(sw + nw);
-        uint8_t *ss = reinterpret_cast<uint8_t *>(sh + nh);
-        const size_t row0 = static_cast<size_t>(c) * DIMS;
-        const double *ge = P.grids + row0 * (bins + 1);
-        const double *gw = P.widths + row0 * bins;
-        const uint32_t *gh = P.hints + row0 * H;
-        for (int k = threadIdx.x; k < ne; k += 128) se[k] = __ldg(ge + k);
-        for (int k = threadIdx.x; k < nw; k += 128) sw[k] = __ldg(gw + k);
-        for (int k = threadIdx.x; k < nh; k += 128) sh[k] = __ldg(gh + k);
-        if (threadIdx.x < DIMS) ss[threadIdx.x] = __ldg(P.sorted + row0 + threadIdx.x);
-        __syncthreads();
-#pragma unroll 1
-        for (int j = 0; j < W.ch_pts; j += 128) {
-            const long long i = i0 + j + threadIdx.x;
-            if (i < P.ms && i < n)
-                pp_channel_point<DIMS, true, true>(P.pp, se, sh, ss, sw, bins, P.memo, P.cfail, P.ich_tile, P.ms,
-                                                   P.ms, 1, P.dcv, P.vwv, P.slot, P.dens, i, i, c);
-        }
-    } else {
-#pragma unroll 1
-        for (int j = 0; j < W.ch_pts; j += 128) {
-            const long long i = i0 + j + threadIdx.x;
-            if (i < P.ms && i < n)
-                pp_channel_point<DIMS, false>(P.pp, P.grids, nullptr, nullptr, nullptr, P.bins, P.memo, P.cfail,
-                                              P.ich_tile, P.ms, P.ms, 1, P.dcv, P.vwv, P.slot, P.dens, i, i, c);
-        }
-    }
+    const long long n = P.ctl->n_acc, end = n < P.ms ? n : P.ms;
+    if (i0 >= end) return;
+    const long long i1 = i0 + W.ch_pts < end ? i0 + W.ch_pts : end;
+    if (cell_fbits(P.bins) == 11)
+        pp_channel_block<DIMS, TAB, 11>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms, 1,
+                                        Densities{P.dens, P.ms}, P.vwv, P.bin_rec, 0, i0, i1, c, smem);
+    else
+        pp_channel_block<DIMS, TAB, 9>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms, 1,
+                                        Densities{P.dens, P.ms}, P.vwv, P.bin_rec, 0, i0, i1, c, smem);
 }
 
 __global__ void __launch_bounds__(256) k_g_combine(WaveDev W, int lo, int hi, long long blk0) {
     CHILI_PIECE(GS_COMBINE)
     const long long i = lb * 256 + threadIdx.x;
     if (i < P.ms && i < P.ctl->n_acc)
-        pp_combine_point(P.pp, P.alpha, P.dcv, P.vwv, P.node, P.ms, i, i, P.f, P.val, P.wgt, P.ok, false);
+        pp_combine_point(P.pp, P.alpha, Densities{P.dens, P.ms}, P.vwv, P.node, P.ms, i, i, P.f, P.val, P.wgt, P.ok);
 }
 
 __global__ void __launch_bounds__(kFwdBlock) k_g_accum(BatchDev B, WaveDev W, int lo, int hi, long long blk0) {
     CHILI_PIECE(GS_ACCUM)
     const bool retry = B.tasks[P.ti].retry != 0;
-    bt_accum_block(B, P.ti, P.p0, P.mm, P.bcount, P.boff, P.val, P.wgt, P.ok, P.slot, P.dens, P.ms, lb,
+    bt_accum_block(B, P.ti, P.p0, P.mm, P.bcount, P.boff, P.val, P.wgt, P.ok, P.bin_rec, P.dens, P.ms, lb,
                    retry ? P.ctl : nullptr, retry ? B.retry + P.ti : nullptr);
 }
 #undef CHILI_PIECE
@@ -787,21 +757,20 @@ __global__ void k_batch_commit(BatchDev B, const AdaptJob *__restrict__ jobs, in
     for (int k = threadIdx.x; k <= T.bins; k += blockDim.x) B.grids[off + k] = B.grids_new[off + k];
     __syncthreads();
     // the row's bin-search tables for the next iteration's channel step
-    build_hint_row(B.grids + off, T.bins, B.hints + T.hint_off + row * (kHintPerBin * T.bins),
-                   B.sorted + T.sorted_off + row, B.widths + T.width_off + row * T.bins);
+    build_cell_row(B.grids_new + T.grid_off + static_cast<size_t>(J.ch) * T.dims * (T.bins + 1), T.dims, T.bins, J.dim,
+                   B.cells + T.cell_off + row * grid_cells(T.bins), B.widths + T.width_off + row * width_row(T.bins));
 }
 
 // The bin-search tables of every (task, channel, dimension) row, one block
 // per row (after the grids are set).
-__global__ void k_batch_hints(BatchDev B, const AdaptJob *__restrict__ jobs, int njobs) {
+__global__ void k_batch_cells(BatchDev B, const AdaptJob *__restrict__ jobs, int njobs) {
     const int j = blockIdx.x;
     if (j >= njobs) return;
     const AdaptJob J = jobs[j];
     const BatchTask T = B.tasks[J.task];
     const size_t row = static_cast<size_t>(J.ch) * T.dims + J.dim;
-    build_hint_row(B.grids + T.grid_off + row * (T.bins + 1), T.bins,
-                   B.hints + T.hint_off + row * (kHintPerBin * T.bins), B.sorted + T.sorted_off + row,
-                   B.widths + T.width_off + row * T.bins);
+    build_cell_row(B.grids + T.grid_off + static_cast<size_t>(J.ch) * T.dims * (T.bins + 1), T.dims, T.bins, J.dim,
+                   B.cells + T.cell_off + row * grid_cells(T.bins), B.widths + T.width_off + row * width_row(T.bins));
 }
 
 __global__ void k_batch_next(BatchDev B) {
@@ -820,7 +789,7 @@ struct BatchState {
     int max_bins = 2, nslots = 0;
     long long total_points = 0, nunits = 0;
     DevBuf d_tasks, d_umap, d_pps, d_progs, d_descs, d_grids, d_grids_new, d_hist, d_atrain, d_alpha, d_best, d_mindiff,
-        d_cp, d_part, d_stats, d_counters, d_jobs, d_status, d_hints, d_widths, d_sorted;
+        d_cp, d_part, d_stats, d_counters, d_jobs, d_status, d_cells, d_widths;
     int block = 0, ppt = 0, grid_blocks = 0;
     long long n_pulled = 0;  // units k_batch_eval pulls (the tasks that are not phased)
     // phased multichannel tasks: host copies of the point programs (launch
@@ -828,7 +797,7 @@ struct BatchState {
     std::vector<PointProgram> pps_host;
     long long ph_tile = 0;
     struct PhBufs {
-        DevBuf mom, ich, flag, list, bcount, boff, ctl, node, memo, cfail, dcv, vwv, ich_tile, val, wgt, ok, slot, dens;
+        DevBuf mom, ich, flag, list, bcount, boff, ctl, node, memo, cfail, vwv, ich_tile, val, wgt, ok, slot, dens;
     };
     // the task chains run as kPhBranches parallel branches of the graph,
     // each with its own stream (at capture) and tile buffers
@@ -891,9 +860,8 @@ BatchDev batch_dev(chili_ctx *ctx) {
     B.descs = S.d_descs.as<IntegrandDesc>();
     B.grids = S.d_grids.as<double>();
     B.grids_new = S.d_grids_new.as<double>();
-    B.hints = S.d_hints.as<uint32_t>();
+    B.cells = S.d_cells.as<uint32_t>();
     B.widths = S.d_widths.as<double>();
-    B.sorted = S.d_sorted.as<uint8_t>();
     B.hist = S.d_hist.as<double>();
     B.atrain = S.d_atrain.as<double>();
     B.alpha = S.d_alpha.as<double>();
@@ -984,14 +952,13 @@ int enqueue_phased_task(chili_ctx *ctx, const BatchDev &B, int ti, BatchState::P
         a.T = mm;
         a.mr = ms;
         a.bins = T.bins;
-        a.grids = B.grids + T.grid_off;
+        a.tables = GridTables{B.grids + T.grid_off, B.cells + T.cell_off, B.widths + T.width_off};
         a.node_soa = b.node.as<double>();
         a.memo = b.memo.as<double>();
-        a.dcv = b.dcv.as<double>();
         a.vwv = b.vwv.as<double>();
         a.cfail = b.cfail.as<uint8_t>();
         a.ich_tile = b.ich_tile.as<int32_t>();
-        a.rec_slot = b.slot.as<int32_t>();
+        a.rec_bins = b.slot.as<uint4>();
         a.rec_dens = b.dens.as<double>();
         a.alpha = B.alpha + T.ch_off;
         a.f = B.descs + T.desc;
@@ -1001,7 +968,7 @@ int enqueue_phased_task(chili_ctx *ctx, const BatchDev &B, int ti, BatchState::P
         if (int rc = pp_pass_launch(ctx, a)) return rc;
         k_bt_accum<<<nb, kFwdBlock, 0, ctx->stream>>>(B, ti, p0, mm, b.bcount.as<int32_t>(), b.boff.as<long long>(),
                                                      b.val.as<double>(), b.wgt.as<double>(), b.ok.as<uint8_t>(),
-                                                     b.slot.as<int32_t>(), b.dens.as<double>(), ms);
+                                                     b.slot.as<uint4>(), b.dens.as<double>(), ms);
         LAUNCHED();
     }
     return CHILI_OK;
@@ -1047,18 +1014,17 @@ int enqueue_waves(chili_ctx *ctx, const BatchDev &B, const std::vector<BatchStat
         for (const auto &g : w.dgroups) {
             const long long b0 = pc[g[1]], nbk = pc[g[2]] - b0;
             if (nbk <= 0) continue;
-            // one channel's edges, widths, hints and flags in shared memory
-            // when they fit the default 48 KB
-            const size_t tab = sizeof(double) * static_cast<size_t>(g[0]) * (2 * g[3] + 1) +
-                               sizeof(uint32_t) * static_cast<size_t>(g[0]) * kHintPerBin * g[3] + g[0];
-            const bool use_tab = ctx->channel_tables && tab <= 48 * 1024;
+            // one channel's entries and widths in shared memory when they
+            // fit the default 48 KB
+            const bool use_tab = ctx->channel_tables && channel_smem_bytes(g[0], g[3], true) <= 48 * 1024;
+            const size_t smem = channel_smem_bytes(g[0], g[3], use_tab);
             switch (g[0]) {
-#define CHILI_GCH(D)                                                                                        \
-    case D:                                                                                                 \
-        if (use_tab)                                                                                        \
-            k_g_channel<D, true><<<static_cast<unsigned>(nbk), 128, tab, ctx->stream>>>(W, g[1], g[2], b0); \
-        else                                                                                                \
-            k_g_channel<D, false><<<static_cast<unsigned>(nbk), 128, 0, ctx->stream>>>(W, g[1], g[2], b0);  \
+#define CHILI_GCH(D)                                                                                         \
+    case D:                                                                                                  \
+        if (use_tab)                                                                                         \
+            k_g_channel<D, true><<<static_cast<unsigned>(nbk), 256, smem, ctx->stream>>>(W, g[1], g[2], b0);  \
+        else                                                                                                 \
+            k_g_channel<D, false><<<static_cast<unsigned>(nbk), 256, smem, ctx->stream>>>(W, g[1], g[2], b0); \
         break;
                 CHILI_GCH(1) CHILI_GCH(4) CHILI_GCH(7) CHILI_GCH(10) CHILI_GCH(13) CHILI_GCH(16) CHILI_GCH(19)
                 CHILI_GCH(22)
@@ -1430,9 +1396,9 @@ int plan_waves(chili_ctx *ctx, const std::vector<PointProgram> &pps) {
                             sizeof(long long) * nb, sizeof(RoundCtl), sizeof(int32_t) * ms,
                             sizeof(double) * 4 * PP.n_nodes * ms, sizeof(double) * std::max(1, PP.n_memo) * ms,
                             static_cast<size_t>(std::max(1, PP.n_chains)) * ms, sizeof(double) * PP.nch * ms,
-                            sizeof(double) * PP.nch * ms, sizeof(int32_t) * ms, sizeof(double) * ms,
-                            sizeof(double) * ms, ms, sizeof(int32_t) * PP.ndims * ms, sizeof(double) * PP.nch * ms};
-        for (int q = 0; q < 18; ++q) out[q] = (v[q] + 255) / 256 * 256;
+                            sizeof(int32_t) * ms, sizeof(double) * ms,
+                            sizeof(double) * ms, ms, sizeof(uint4) * bin_rec_vecs(PP.ndims) * ms, sizeof(double) * PP.nch * ms};
+        for (int q = 0; q < 17; ++q) out[q] = (v[q] + 255) / 256 * 256;
     };
     S.wave_streams = static_cast<int>(std::min<long long>(std::max<long long>(ctx->batch_wave_streams, 1),
                                                           kMaxWaveStreams));
@@ -1441,7 +1407,7 @@ int plan_waves(chili_ctx *ctx, const std::vector<PointProgram> &pps) {
     for (size_t wi = 0; wi < waves.size(); ++wi) {
         size_t tot = 0;
         for (const Piece &P : waves[wi]) {
-            size_t sz[18];
+            size_t sz[17];
             sizes(P, pps[static_cast<size_t>(S.tasks[static_cast<size_t>(P.ti)].pp)], sz);
             for (size_t q : sz) tot += q;
         }
@@ -1477,16 +1443,14 @@ int plan_waves(chili_ctx *ctx, const std::vector<PointProgram> &pps) {
             P.dims = T.dims;
             P.bins = T.bins;
             P.pp = S.d_pps.as<PointProgram>() + T.pp;
-            P.grids = S.d_grids.as<double>() + T.grid_off;
-            P.hints = S.d_hints.as<uint32_t>() + T.hint_off;
-            P.widths = S.d_widths.as<double>() + T.width_off;
-            P.sorted = S.d_sorted.as<uint8_t>() + T.sorted_off;
+            P.tables = GridTables{S.d_grids.as<double>() + T.grid_off, S.d_cells.as<uint32_t>() + T.cell_off,
+                                  S.d_widths.as<double>() + T.width_off};
             P.alpha = S.d_alpha.as<double>() + T.ch_off;
             P.f = S.d_descs.as<IntegrandDesc>() + T.desc;
-            size_t sz[18];
+            size_t sz[17];
             sizes(P, PP, sz);
-            void *ptr[18];
-            for (int q = 0; q < 18; ++q) {
+            void *ptr[17];
+            for (int q = 0; q < 17; ++q) {
                 ptr[q] = base + off;
                 off += sz[q];
             }
@@ -1500,14 +1464,13 @@ int plan_waves(chili_ctx *ctx, const std::vector<PointProgram> &pps) {
             P.node = static_cast<double *>(ptr[7]);
             P.memo = static_cast<double *>(ptr[8]);
             P.cfail = static_cast<uint8_t *>(ptr[9]);
-            P.dcv = static_cast<double *>(ptr[10]);
-            P.vwv = static_cast<double *>(ptr[11]);
-            P.ich_tile = static_cast<int32_t *>(ptr[12]);
-            P.val = static_cast<double *>(ptr[13]);
-            P.wgt = static_cast<double *>(ptr[14]);
-            P.ok = static_cast<uint8_t *>(ptr[15]);
-            P.slot = static_cast<int32_t *>(ptr[16]);
-            P.dens = static_cast<double *>(ptr[17]);
+            P.vwv = static_cast<double *>(ptr[10]);
+            P.ich_tile = static_cast<int32_t *>(ptr[11]);
+            P.val = static_cast<double *>(ptr[12]);
+            P.wgt = static_cast<double *>(ptr[13]);
+            P.ok = static_cast<uint8_t *>(ptr[14]);
+            P.bin_rec = static_cast<uint4 *>(ptr[15]);
+            P.dens = static_cast<double *>(ptr[16]);
             const long long gx = (P.ms + 255) / 256, gy = (P.ms + S.ch_pts - 1) / S.ch_pts;
             const long long nblk[kGroupSteps] = {P.nb, P.nb, gx, P.n_items[0] * gx, P.n_items[1] * gx,
                                                  P.n_items[2] * gx, P.n_chains * gx, P.nch * gy, gx, P.nb};
@@ -1561,14 +1524,14 @@ void batch_release(chili_ctx *ctx) {
     S.d_top_pieces.release();
     S.d_top_prefix.release();
     for (DevBuf *b : {&S.d_tasks, &S.d_umap, &S.d_pps, &S.d_progs, &S.d_descs, &S.d_grids, &S.d_grids_new, &S.d_hist,
-                      &S.d_hints, &S.d_widths, &S.d_sorted,
+                      &S.d_cells, &S.d_widths,
                       &S.d_atrain, &S.d_alpha, &S.d_best, &S.d_mindiff, &S.d_cp, &S.d_part, &S.d_stats,
                       &S.d_counters, &S.d_jobs, &S.d_status, &S.d_pieces, &S.d_prefix, &S.d_arena[0],
                       &S.d_arena[1], &S.d_arena[2], &S.d_arena[3]})
         b->release();
     for (auto &b : S.ph)
         for (DevBuf *d : {&b.mom, &b.ich, &b.flag, &b.list, &b.bcount, &b.boff, &b.ctl, &b.node, &b.memo, &b.cfail,
-                          &b.dcv, &b.vwv, &b.ich_tile, &b.val, &b.wgt, &b.ok, &b.slot, &b.dens})
+                          &b.vwv, &b.ich_tile, &b.val, &b.wgt, &b.ok, &b.slot, &b.dens})
             d->release();
     for (cudaStream_t st : S.ph_streams) cudaStreamDestroy(st);
     for (cudaEvent_t e : S.ph_events) cudaEventDestroy(e);
@@ -1588,7 +1551,7 @@ int chili_gpu_batch_set(chili_ctx *ctx, const chili_task *tasks, int ntasks) {
     std::vector<PointProgram> pps;
     std::vector<IntegrandDesc> descs;
     std::vector<double> grids, alpha;
-    long long goff = 0, hoff = 0, hnoff = 0, woff = 0, soff = 0;
+    long long goff = 0, hoff = 0, coff = 0, woff = 0;
     for (int k = 0; k < ntasks; ++k) {
         const chili_task &t = tasks[k];
         BatchTask T{};
@@ -1670,12 +1633,10 @@ int chili_gpu_batch_set(chili_ctx *ctx, const chili_task *tasks, int ntasks) {
         T.before = edge_before_table(T.dims, T.bins);
         T.grid_off = goff;
         T.hist_off = hoff;
-        T.hint_off = hnoff;
+        T.cell_off = coff;
         T.width_off = woff;
-        T.sorted_off = soff;
-        hnoff += static_cast<long long>(T.nch) * T.dims * kHintPerBin * T.bins;
-        woff += static_cast<long long>(T.nch) * T.dims * T.bins;
-        soff += static_cast<long long>(T.nch) * T.dims;
+        coff += static_cast<long long>(T.nch) * T.dims * grid_cells(T.bins);
+        woff += static_cast<long long>(T.nch) * T.dims * width_row(T.bins);
         const long long per = static_cast<long long>(T.dims) * (T.bins + 1);
         for (int c = 0; c < T.nch; ++c)
             for (int dd = 0; dd < T.dims; ++dd)
@@ -1738,13 +1699,12 @@ int chili_gpu_batch_set(chili_ctx *ctx, const chili_task *tasks, int ntasks) {
                 CK(b.node.ensure(sizeof(double) * 4 * nn * T));
                 CK(b.memo.ensure(sizeof(double) * nmemo * T));
                 CK(b.cfail.ensure(static_cast<size_t>(nchain) * T));
-                CK(b.dcv.ensure(sizeof(double) * nch * T));
                 CK(b.vwv.ensure(sizeof(double) * nch * T));
                 CK(b.ich_tile.ensure(sizeof(int32_t) * T));
                 CK(b.val.ensure(sizeof(double) * T));
                 CK(b.wgt.ensure(sizeof(double) * T));
                 CK(b.ok.ensure(T));
-                CK(b.slot.ensure(sizeof(int32_t) * dims * T));
+                CK(b.slot.ensure(sizeof(uint4) * bin_rec_vecs(dims) * T));
                 CK(b.dens.ensure(sizeof(double) * nch * T));
             }
             for (int k = 0; k < kPhBranches; ++k) {
@@ -1777,9 +1737,8 @@ int chili_gpu_batch_set(chili_ctx *ctx, const chili_task *tasks, int ntasks) {
     CK(S.d_grids.ensure(sizeof(double) * grids.size()));
     CK(S.d_grids_new.ensure(sizeof(double) * grids.size()));
     CK(cudaMemcpyAsync(S.d_grids.p, grids.data(), sizeof(double) * grids.size(), cudaMemcpyHostToDevice, ctx->stream));
-    CK(S.d_hints.ensure(sizeof(uint32_t) * std::max<long long>(hnoff, 1)));
+    CK(S.d_cells.ensure(sizeof(uint32_t) * std::max<long long>(coff, 1)));
     CK(S.d_widths.ensure(sizeof(double) * std::max<long long>(woff, 1)));
-    CK(S.d_sorted.ensure(std::max<long long>(soff, 1)));
     CK(S.d_hist.ensure(sizeof(double) * std::max<size_t>(S.hist_doubles, 1)));
     CK(S.d_atrain.ensure(sizeof(double) * nslot));
     CK(S.d_alpha.ensure(sizeof(double) * nslot));
@@ -1823,7 +1782,7 @@ int chili_gpu_batch_set(chili_ctx *ctx, const chili_task *tasks, int ntasks) {
     // the bin-search tables of the initial grids (k_batch_commit keeps them
     // current after every adaptation)
     if (!S.jobs.empty()) {
-        k_batch_hints<<<static_cast<unsigned>(S.jobs.size()), 128, 0, ctx->stream>>>(
+        k_batch_cells<<<static_cast<unsigned>(S.jobs.size()), 128, 0, ctx->stream>>>(
             batch_dev(ctx), S.d_jobs.as<AdaptJob>(), static_cast<int>(S.jobs.size()));
         LAUNCHED();
     }

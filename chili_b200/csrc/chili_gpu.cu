@@ -35,43 +35,55 @@ namespace {
 
 int rebuild_hints(chili_ctx *ctx);
 
-// Largest table (one channel's edges, widths, hints) staged in shared memory
-// by k_pp_channel_tab; larger channel tables take k_pp_channel.
-constexpr size_t kMaxChannelTab = 112 * 1024;
+// Largest table of one channel (entries and widths) staged in shared memory
+// by the channel step; larger ones are read from global memory.
+constexpr size_t kMaxChannelTab = 200 * 1024;
 
+GridTables grid_tables(const chili_ctx *ctx) {
+    return GridTables{ctx->edges.as<double>(), ctx->cells.as<uint32_t>(), ctx->widths.as<double>()};
+}
+
+// The channel step over the T-point tile (n of them listed, as far as the
+// host knows).
 template <int D>
-void launch_channel(chili_ctx *ctx, long long base, long long T, long long mr, int bins, int opt,
-                    const long long *n_list, int32_t *rec_slot, double *rec_dens, const PPCombine *fuse) {
-    const dim3 grid(ctx->nch, static_cast<unsigned>((T + 127) / 128));
-    if (fuse) {
-        k_pp_channel<D, true, true><<<grid, 128, 0, ctx->stream>>>(
-            ctx->point_prog.as<PointProgram>(), ctx->edges.as<double>(), ctx->hints.as<uint32_t>(),
-            ctx->sorted.as<uint8_t>(), ctx->widths.as<double>(), bins, ctx->memo.as<double>(),
-            ctx->cfail.as<uint8_t>(), ctx->ich_tile.as<int32_t>(), n_list, base, T, mr, opt, ctx->dcv.as<double>(),
-            ctx->vwv.as<double>(), rec_slot, rec_dens, *fuse);
-        return;
+int launch_channel(chili_ctx *ctx, const PointProgram *pp, const GridTables &G, int bins, const double *memo,
+                   const uint8_t *cfail, const int32_t *ich_tile, const long long *n_list, long long base, long long T,
+                   int opt, Densities dens, double *vwv, uint4 *rec_bins, int nch, long long n) {
+    const bool tab = ctx->channel_tables && channel_smem_bytes(D, bins, true) <= kMaxChannelTab;
+    const size_t smem = channel_smem_bytes(D, bins, tab);
+    // as many threads per block as keep 32 warps on an SM beside the tables
+    const int threads = !tab || smem <= 54 * 1024 ? 256 : (smem <= 110 * 1024 ? 512 : channel_max_threads(D));
+    // points per block: enough for the table copy to be small beside them,
+    // few enough for about four blocks per SM
+    long long points = n * nch / (4 * ctx->sms);
+    points = std::min<long long>(8192, std::max<long long>(threads, (points + threads - 1) / threads * threads));
+    points = std::max(points, (T / 65535 / threads + 1) * threads);  // gridDim.y stays below 65536
+    const dim3 grid(static_cast<unsigned>(nch), static_cast<unsigned>((T + points - 1) / points));
+    const bool f11 = cell_fbits(bins) == 11;
+    auto kern = tab ? (f11 ? k_pp_channel<D, true, 11> : k_pp_channel<D, true, 9>)
+                    : (f11 ? k_pp_channel<D, false, 11> : k_pp_channel<D, false, 9>);
+    if (smem > 48 * 1024)
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    kern<<<grid, threads, smem, ctx->stream>>>(pp, G, bins, memo, cfail, ich_tile, n_list, base, T, opt, dens, vwv,
+                                               rec_bins, static_cast<int>(points));
+    LAUNCHED();
+    return CHILI_OK;
+}
+
+// launch_channel<D> for the dimensions the phased kernels are built for.
+template <class... A>
+int launch_channel_dims(chili_ctx *ctx, int dims, A... a) {
+    switch (dims) {
+    case 1: return launch_channel<1>(ctx, a...);
+    case 4: return launch_channel<4>(ctx, a...);
+    case 7: return launch_channel<7>(ctx, a...);
+    case 10: return launch_channel<10>(ctx, a...);
+    case 13: return launch_channel<13>(ctx, a...);
+    case 16: return launch_channel<16>(ctx, a...);
+    case 19: return launch_channel<19>(ctx, a...);
+    case 22: return launch_channel<22>(ctx, a...);
+    default: return fail(ctx, CHILI_ERR_STATE, "no phased weight kernel for this dimension");
     }
-    const size_t tab = channel_tab_bytes(D, bins);
-    if (ctx->channel_tables && tab <= kMaxChannelTab) {
-        static size_t attr = 0;  // dynamic shared memory granted so far
-        if (tab > attr) {
-            cudaFuncSetAttribute(k_pp_channel_tab<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kMaxChannelTab));
-            attr = kMaxChannelTab;
-        }
-        const dim3 gt(ctx->nch, static_cast<unsigned>((T + kTabPoints - 1) / kTabPoints));
-        k_pp_channel_tab<D><<<gt, kTabThreads, tab, ctx->stream>>>(
-            ctx->point_prog.as<PointProgram>(), ctx->edges.as<double>(), ctx->hints.as<uint32_t>(),
-            ctx->sorted.as<uint8_t>(), ctx->widths.as<double>(), bins, ctx->memo.as<double>(),
-            ctx->cfail.as<uint8_t>(), ctx->ich_tile.as<int32_t>(), n_list, base, T, mr, opt, ctx->dcv.as<double>(),
-            ctx->vwv.as<double>(), rec_slot, rec_dens);
-        return;
-    }
-    k_pp_channel<D><<<grid, 128, 0, ctx->stream>>>(
-        ctx->point_prog.as<PointProgram>(), ctx->edges.as<double>(), ctx->hints.as<uint32_t>(),
-        ctx->sorted.as<uint8_t>(), ctx->widths.as<double>(), bins, ctx->memo.as<double>(),
-        ctx->cfail.as<uint8_t>(), ctx->ich_tile.as<int32_t>(), n_list, base, T, mr, opt, ctx->dcv.as<double>(),
-        ctx->vwv.as<double>(), rec_slot, rec_dens);
 }
 
 }  // namespace
@@ -83,11 +95,11 @@ void launch_channel(chili_ctx *ctx, long long base, long long T, long long mr, i
 // intermediates go through HBM: tiles small enough for their buffers to stay
 // in L2 were measured slower, every launch's tail growing with the launch
 // count); `combine` launches the last step of
-// each tile (it reads the per-channel densities ctx->dcv, ctx->vwv and the
+// each tile (it reads the per-channel densities it is given, ctx->vwv and the
 // nodes ctx->node_soa of the tile).
 int pipeline_run(chili_ctx *ctx, const double *mom_soa, long long m, const int32_t *list, const int32_t *ich,
-                 const long long *n_list, long long n_pre, int bins, bool opt, int32_t *rec_slot, double *rec_dens,
-                 const TileFn &combine, const PPFusedOut *fused) {
+                 const long long *n_list, long long n_pre, int bins, bool opt, uint4 *rec_bins, double *rec_dens,
+                 const TileFn &combine) {
     if (ctx->hints_stale)
         if (int rc = rebuild_hints(ctx)) return rc;
     const PointProgram &P = ctx->pp_host;
@@ -102,24 +114,15 @@ int pipeline_run(chili_ctx *ctx, const double *mom_soa, long long m, const int32
     CK(ctx->node_soa.ensure(sizeof(double) * 4 * P.n_nodes * Ta));
     CK(ctx->memo.ensure(sizeof(double) * std::max(1, P.n_memo) * Ta));
     CK(ctx->cfail.ensure(static_cast<size_t>(std::max(1, P.n_chains)) * Ta));
-    CK(ctx->dcv.ensure(sizeof(double) * ctx->nch * Ta));
+    if (!rec_dens) CK(ctx->dcv.ensure(sizeof(double) * ctx->nch * Ta));
     CK(ctx->ich_tile.ensure(sizeof(int32_t) * Ta));
     CK(ctx->vwv.ensure(sizeof(double) * ctx->nch * Ta));
-    PPCombine comb{};
-    const bool fuse = fused && ctx->fuse_combine;
-    if (fuse) {
-        const size_t nblk = static_cast<size_t>((Ta + 127) / 128);
-        if (ctx->arrivals.cap < sizeof(unsigned) * nblk) {
-            CK(ctx->arrivals.ensure(sizeof(unsigned) * nblk));
-            CK(cudaMemsetAsync(ctx->arrivals.p, 0, ctx->arrivals.cap, ctx->stream));
-        }
-        comb = PPCombine{alpha_ptr(ctx), ctx->node_soa.as<double>(), ctx->f_dev.as<IntegrandDesc>(), fused->rec_val,
-                         fused->rec_wgt, fused->rec_ok, ctx->arrivals.as<unsigned>()};
-    }
     const unsigned gx = static_cast<unsigned>((T + 255) / 256);
     const int n_items = P.n_tents + P.n_dws + P.n_sws;
     const int o = opt ? 1 : 0;
     for (long long base = 0; base < n_pre; base += T) {
+        // the densities go straight to the records, or to a tile buffer
+        const Densities dens = rec_dens ? Densities{rec_dens + base, m} : Densities{ctx->dcv.as<double>(), T};
         { KTimer kt_(ctx, KT_NODES);
         k_pp_nodes<<<gx, 256, 0, ctx->stream>>>(pp, mom_soa, m, list, ich, n_list, base, ctx->node_soa.as<double>(),
                                                  ctx->ich_tile.as<int32_t>(), T); }
@@ -146,16 +149,15 @@ int pipeline_run(chili_ctx *ctx, const double *mom_soa, long long m, const int32
         k_pp_chains<<<dim3(P.n_chains, gx), 256, 0, ctx->stream>>>(pp, ctx->node_soa.as<double>(), n_list, base, T,
                                                                     ctx->memo.as<double>(), ctx->cfail.as<uint8_t>()); }
         LAUNCHED();
-        switch (P.ndims) {
-#define CHILI_CH(D) \
-    case D: { KTimer kt_(ctx, KT_CHANNEL); launch_channel<D>(ctx, base, T, m, bins, o, n_list, rec_slot, rec_dens, fuse ? &comb : nullptr); } break;
-            CHILI_CH(1) CHILI_CH(4) CHILI_CH(7) CHILI_CH(10) CHILI_CH(13) CHILI_CH(16) CHILI_CH(19) CHILI_CH(22)
-#undef CHILI_CH
-        default: return fail(ctx, CHILI_ERR_STATE, "no phased weight kernel for this dimension");
+        {
+            KTimer kt_(ctx, KT_CHANNEL);
+            if (int rc = launch_channel_dims(ctx, P.ndims, pp, grid_tables(ctx), bins, ctx->memo.as<double>(),
+                                             ctx->cfail.as<uint8_t>(), ctx->ich_tile.as<int32_t>(), n_list, base, T, o,
+                                             dens, ctx->vwv.as<double>(), rec_bins, ctx->nch,
+                                             std::min(T, n_pre - base)))
+                return rc;
         }
-        LAUNCHED();
-        if (!fuse)
-            if (int rc = combine(base, T)) return rc;
+        if (int rc = combine(base, T, dens)) return rc;
     }
     return CHILI_OK;
 }
@@ -184,25 +186,10 @@ int pp_pass_launch(chili_ctx *ctx, const PPPass &a) {
         k_pp_chains<<<dim3(P.n_chains, gx), 256, 0, ctx->stream>>>(a.pp, a.node_soa, a.n_list, 0, T, a.memo, a.cfail);
         LAUNCHED();
     }
-    const dim3 gc(static_cast<unsigned>(P.nch), static_cast<unsigned>((T + 127) / 128));
-    switch (P.ndims) {
-#define CHILI_CH(D)                                                                                          \
-    case D:                                                                                                  \
-        if (a.hints)                                                                                         \
-            k_pp_channel<D, true><<<gc, 128, 0, ctx->stream>>>(                                              \
-                a.pp, a.grids, a.hints, a.sorted, a.widths, a.bins, a.memo, a.cfail, a.ich_tile, a.n_list,        \
-                0, T, a.mr, 1, a.dcv, a.vwv, a.rec_slot, a.rec_dens);                                        \
-        else                                                                                                 \
-            k_pp_channel<D, false><<<gc, 128, 0, ctx->stream>>>(                                             \
-                a.pp, a.grids, a.hints, a.sorted, a.widths, a.bins, a.memo, a.cfail, a.ich_tile,              \
-                a.n_list, 0, T, a.mr, 1, a.dcv, a.vwv, a.rec_slot, a.rec_dens);                              \
-        break;
-        CHILI_CH(1) CHILI_CH(4) CHILI_CH(7) CHILI_CH(10) CHILI_CH(13) CHILI_CH(16) CHILI_CH(19) CHILI_CH(22)
-#undef CHILI_CH
-    default: return fail(ctx, CHILI_ERR_STATE, "no phased weight kernel for this dimension");
-    }
-    LAUNCHED();
-    k_pp_combine<<<gx, 256, 0, ctx->stream>>>(a.pp, a.alpha, a.dcv, a.vwv, a.node_soa, a.n_list, 0, T, a.f,
+    if (int rc = launch_channel_dims(ctx, P.ndims, a.pp, a.tables, a.bins, a.memo, a.cfail, a.ich_tile, a.n_list, 0ll, T,
+                                     1, Densities{a.rec_dens, a.mr}, a.vwv, a.rec_bins, static_cast<int>(P.nch), T))
+        return rc;
+    k_pp_combine<<<gx, 256, 0, ctx->stream>>>(a.pp, a.alpha, Densities{a.rec_dens, a.mr}, a.vwv, a.node_soa, a.n_list, 0, T, a.f,
                                                a.rec_val, a.rec_wgt, a.rec_ok);
     LAUNCHED();
     return CHILI_OK;
@@ -269,39 +256,35 @@ int upload_host(chili_ctx *ctx, const double *u, long long m, const std::vector<
 // The phased weight pass of a multichannel chunk: records of the n_pre
 // PreProcess-accepted points of the chunk of m counters.
 int launch_pipeline(chili_ctx *ctx, const double *mom_soa, const int32_t *ich, long long m, long long n_pre, int bins,
-                    bool opt, RoundCtl *ctl_pre, double *rec_val, double *rec_wgt, uint8_t *rec_ok, int32_t *rec_slot,
+                    bool opt, RoundCtl *ctl_pre, double *rec_val, double *rec_wgt, uint8_t *rec_ok, uint4 *rec_bins,
                     double *rec_dens) {
     const PointProgram *pp = ctx->point_prog.as<PointProgram>();
     const long long *n_list = reinterpret_cast<const long long *>(
         reinterpret_cast<const char *>(ctl_pre) + offsetof(RoundCtl, n_acc));
-    const PPFusedOut fused{rec_val, rec_wgt, rec_ok};
     return pipeline_run(ctx, mom_soa, m, ctx->list.as<int32_t>(), ich, n_list,
-                        n_pre, bins, opt, rec_slot, rec_dens, [&](long long base, long long T) -> int {
+                        n_pre, bins, opt, rec_bins, rec_dens, [&](long long base, long long T, Densities dens) -> int {
                             const unsigned gx = static_cast<unsigned>((T + 255) / 256);
                             {
                                 KTimer kt_(ctx, KT_COMBINE);
                                 k_pp_combine<<<gx, 256, 0, ctx->stream>>>(
-                                    pp, alpha_ptr(ctx), ctx->dcv.as<double>(), ctx->vwv.as<double>(),
+                                    pp, alpha_ptr(ctx), dens, ctx->vwv.as<double>(),
                                     ctx->node_soa.as<double>(), n_list, base, T, ctx->f_dev.as<IntegrandDesc>(),
                                     rec_val, rec_wgt, rec_ok);
                             }
                             LAUNCHED();
                             return CHILI_OK;
-                        }, &fused);
+                        });
 }
 
-// Hint tables of the grid set (grid.cuh, find_bin_hinted), rebuilt after
-// every change of the edges.
+// The search tables of the grid set (grid.cuh), rebuilt after every change of
+// the edges.
 int rebuild_hints(chili_ctx *ctx) {
     ctx->hints_stale = false;
-    const int H = kHintPerBin * ctx->bins;
-    CK(ctx->hints.ensure(sizeof(uint32_t) * static_cast<size_t>(ctx->g_nch) * ctx->dims * H));
-    CK(ctx->sorted.ensure(static_cast<size_t>(ctx->g_nch) * ctx->dims));
-    CK(ctx->widths.ensure(sizeof(double) * static_cast<size_t>(ctx->g_nch) * ctx->dims * ctx->bins));
-    k_build_hints<<<dim3(ctx->dims, ctx->g_nch), 128, 0, ctx->stream>>>(ctx->edges.as<double>(), ctx->dims, ctx->bins,
-                                                                        ctx->hints.as<uint32_t>(),
-                                                                        ctx->sorted.as<uint8_t>(),
-                                                                        ctx->widths.as<double>());
+    const size_t rows = static_cast<size_t>(ctx->g_nch) * ctx->dims;
+    CK(ctx->cells.ensure(sizeof(uint32_t) * rows * grid_cells(ctx->bins)));
+    CK(ctx->widths.ensure(sizeof(double) * rows * width_row(ctx->bins)));
+    k_build_cells<<<dim3(ctx->dims, ctx->g_nch), 128, 0, ctx->stream>>>(
+        ctx->edges.as<double>(), ctx->dims, ctx->bins, ctx->cells.as<uint32_t>(), ctx->widths.as<double>());
     LAUNCHED();
     return CHILI_OK;
 }
@@ -354,11 +337,11 @@ int chili_gpu_destroy(chili_ctx *ctx) {
     if (!ctx) return CHILI_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    DevBuf *bufs[] = {&ctx->edges, &ctx->edges_tmp, &ctx->progs, &ctx->point_prog, &ctx->node_soa, &ctx->memo, &ctx->cfail, &ctx->dcv, &ctx->vwv, &ctx->hints, &ctx->sorted, &ctx->widths, &ctx->ich_tile, &ctx->alpha_buf, &ctx->f_dev, &ctx->mom_soa,
+    DevBuf *bufs[] = {&ctx->edges, &ctx->edges_tmp, &ctx->progs, &ctx->point_prog, &ctx->node_soa, &ctx->memo, &ctx->cfail, &ctx->dcv, &ctx->vwv, &ctx->cells, &ctx->widths, &ctx->ich_tile, &ctx->alpha_buf, &ctx->f_dev, &ctx->mom_soa,
                       &ctx->ich, &ctx->flag, &ctx->list, &ctx->block_count, &ctx->block_off, &ctx->part,
                       &ctx->hist, &ctx->round_res, &ctx->acc, &ctx->ctl, &ctx->status, &ctx->v_part,
                       &ctx->v_hist, &ctx->v_train, &ctx->v_out, &ctx->rec, &ctx->ctl3, &ctx->unw, &ctx->iter_ctl,
-                      &ctx->mom_soa_alt, &ctx->ich_alt, &ctx->flag_alt, &ctx->block_count_alt, &ctx->arrivals,
+                      &ctx->mom_soa_alt, &ctx->ich_alt, &ctx->flag_alt, &ctx->block_count_alt,
                       &ctx->v_arrive};
     for (DevBuf *b : bufs) b->release();
     flow_release(ctx);
@@ -443,10 +426,7 @@ int chili_gpu_set_option(chili_ctx *ctx, const char *name, int64_t value) {
         ctx->gen_ppt = value;
         return CHILI_OK;
     }
-    if (std::strcmp(name, "pipeline_fuse") == 0) {
-        ctx->fuse_combine = value != 0;
-        return CHILI_OK;
-    }
+    if (std::strcmp(name, "pipeline_fuse") == 0) return CHILI_OK;  // accepted; the combine step is a launch of its own
     if (std::strcmp(name, "pipeline") == 0) {
         ctx->use_pipeline = value != 0;
         return CHILI_OK;
@@ -599,9 +579,9 @@ int chili_gpu_grid_weight(chili_ctx *ctx, int ch, const double *x, double *w, in
     if (ctx->hints_stale)
         if ((rc = rebuild_hints(ctx))) return rc;
     const double *g = ctx->edges.as<double>() + static_cast<size_t>(ch) * D * (B + 1);
-    const uint32_t *hg = ctx->hints.as<uint32_t>() + static_cast<size_t>(ch) * D * (kHintPerBin * B);
-    const uint8_t *sg = ctx->sorted.as<uint8_t>() + static_cast<size_t>(ch) * D;
-    k_grid_weight<<<grid_for(n, 128), 128, 0, ctx->stream>>>(g, hg, sg, D, B, static_cast<const double *>(ax.dev),
+    const uint32_t *eg = ctx->cells.as<uint32_t>() + static_cast<size_t>(ch) * D * grid_cells(B);
+    const double *sg = ctx->widths.as<double>() + static_cast<size_t>(ch) * D * width_row(B);
+    k_grid_weight<<<grid_for(n, 128), 128, 0, ctx->stream>>>(g, eg, sg, D, B, static_cast<const double *>(ax.dev),
                                                              static_cast<double *>(aw.dev),
                                                              static_cast<int32_t *>(ab.dev), n);
     LAUNCHED();
@@ -1119,7 +1099,7 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
         {
             // keep the per-chunk buffers within ~8 GB
             const PointProgram &P = ctx->pp_host;
-            long long per = 8ll * (4 * NE + nch + 4) + 4ll * D + 8;
+            long long per = 8ll * (4 * NE + nch + 4) + 16ll * bin_rec_vecs(D) + 8;
             if (pipe) per += 8ll * (4 * P.n_nodes + P.n_memo) + P.n_chains;
             m = std::min<long long>(m, std::max<long long>(1 << 16, (8ll << 30) / per));
         }
@@ -1158,7 +1138,7 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
         CK(ctx->block_count.ensure(sizeof(int32_t) * nb_f));
         CK(ctx->block_off.ensure(sizeof(long long) * nb_f));
         CK(ctx->part.ensure(sizeof(double) * (kPartFixed + nch) * nb_w));
-        CK(ctx->rec.ensure(Sa * (2 * sizeof(double) + 1 + sizeof(int32_t) * D + sizeof(double) * nch) + 256));
+        CK(ctx->rec.ensure(Sa * (2 * sizeof(double) + 1 + sizeof(uint4) * bin_rec_vecs(D) + sizeof(double) * nch) + 256));
         CK(ctx->ctl3.ensure(3 * sizeof(RoundCtl)));
         RoundCtl *ctl_pre = ctx->ctl3.as<RoundCtl>(), *ctl_list = ctl_pre + 1;
         if (u_host) {
@@ -1181,12 +1161,12 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
             const long long mm = sb[q + 1] - r0;
             const long long nbf = (mm + kFwdBlock - 1) / kFwdBlock, nbw = (mm + kWgtBlock - 1) / kWgtBlock;
             const long long *gate = u_host ? iter : nullptr;
-            // records with stride mm
-            double *rec_val = ctx->rec.as<double>();
+            // records with stride mm (the bins first: 16-byte rows)
+            uint4 *rec_bins = ctx->rec.as<uint4>();
+            double *rec_val = reinterpret_cast<double *>(rec_bins + static_cast<size_t>(bin_rec_vecs(D)) * mm);
             double *rec_wgt = rec_val + mm;
             double *rec_dens = rec_wgt + mm;
-            int32_t *rec_slot = reinterpret_cast<int32_t *>(rec_dens + static_cast<size_t>(nch) * mm);
-            uint8_t *rec_ok = reinterpret_cast<uint8_t *>(rec_slot + static_cast<size_t>(D) * mm);
+            uint8_t *rec_ok = reinterpret_cast<uint8_t *>(rec_dens + static_cast<size_t>(nch) * mm);
             // host-uniform rounds alternate between two sets of forward
             // buffers, so that the forward pass of round q + 1 (on the
             // forward stream) runs beside the weight pass of round q
@@ -1244,14 +1224,14 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
                     n_pre = ctx->ctl_host->n_acc;
                 }
                 int rc2 = launch_pipeline(ctx, mom, ich, mm, n_pre, B, opt, ctl_pre, rec_val, rec_wgt, rec_ok,
-                                          rec_slot, rec_dens);
+                                          rec_bins, rec_dens);
                 if (rc2) return rc2;
             } else {
                 KTimer kt_(ctx, KT_WEIGHT);
                 k_mc_weight<<<static_cast<unsigned>(nbw), kWgtBlock, 0, ctx->stream>>>(
                     ctx->progs.as<ChannelProgram>(), ctx->edges.as<double>(), alpha_ptr(ctx), nch, D, B, NE,
                     mom, mm, ich, ctx->list.as<int32_t>(), ctl_pre, ctx->f_dev.as<IntegrandDesc>(), opt ? 1 : 0,
-                    rec_val, rec_wgt, rec_ok, rec_slot, rec_dens, pp_ptr(ctx));
+                    rec_val, rec_wgt, rec_ok, rec_bins, rec_dens, pp_ptr(ctx));
                 LAUNCHED();
             }
             // the cut: the needed-th record whose value is not NaN (the
@@ -1270,14 +1250,14 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
             {
                 KTimer kt_(ctx, KT_ACCUM);
                 k_mc_accum<<<static_cast<unsigned>(nbw), kWgtBlock, acc_smem, ctx->stream>>>(
-                    ctx->ctl.as<RoundCtl>(), mm, nch, D, static_cast<int>(hist_n), rec_val, rec_wgt, rec_ok, rec_slot,
+                    ctx->ctl.as<RoundCtl>(), mm, nch, D, B, static_cast<int>(hist_n), rec_val, rec_wgt, rec_ok, rec_bins,
                     rec_dens, opt ? 1 : 0, guard_alpha ? 1 : 0, hist_smem ? nullptr : ctx->hist.as<double>(),
                     ctx->part.as<double>());
                 LAUNCHED();
                 if (hist_smem && opt) {
                     k_mc_hist<<<static_cast<unsigned>(std::min<long long>(nbw, ctx->sms)), 1024,
-                                sizeof(double) * hist_n, ctx->stream>>>(ctx->ctl.as<RoundCtl>(), mm, D,
-                                                                        static_cast<int>(hist_n), rec_val, rec_slot,
+                                sizeof(double) * hist_n, ctx->stream>>>(ctx->ctl.as<RoundCtl>(), mm, D, B,
+                                                                        static_cast<int>(hist_n), rec_val, rec_bins,
                                                                         ctx->hist.as<double>());
                     LAUNCHED();
                 }
@@ -1478,7 +1458,7 @@ int chili_gpu_generate_unweighted(chili_ctx *ctx, int64_t n, uint64_t seed, uint
         {
             // keep the per-chunk buffers within ~8 GB, as an iteration does
             const PointProgram &P = ctx->pp_host;
-            long long per = 8ll * (4 * NE + nch + 4) + 4ll * D + 16;
+            long long per = 8ll * (4 * NE + nch + 4) + 16ll * bin_rec_vecs(D) + 16;
             if (pipe) per += 8ll * (4 * P.n_nodes + P.n_memo) + P.n_chains;
             m = std::min<long long>(m, std::max<long long>(1 << 16, (8ll << 30) / per));
         }
@@ -1490,7 +1470,7 @@ int chili_gpu_generate_unweighted(chili_ctx *ctx, int64_t n, uint64_t seed, uint
         CK(ctx->list.ensure(sizeof(int32_t) * m));
         CK(ctx->block_count.ensure(sizeof(int32_t) * nb_f));
         CK(ctx->block_off.ensure(sizeof(long long) * nb_f));
-        CK(ctx->rec.ensure(m * (2 * sizeof(double) + 1 + sizeof(int32_t) * D + sizeof(double) * nch) + 256));
+        CK(ctx->rec.ensure(m * (2 * sizeof(double) + 1 + sizeof(uint4) * bin_rec_vecs(D) + sizeof(double) * nch) + 256));
         CK(ctx->ctl3.ensure(3 * sizeof(RoundCtl)));
         // keep flags [m] | kept list [m] | partials [nb_f][3] | sums [3] | control
         const size_t off_list = (static_cast<size_t>(m) + 15) & ~static_cast<size_t>(15);
@@ -1505,11 +1485,11 @@ int chili_gpu_generate_unweighted(chili_ctx *ctx, int64_t n, uint64_t seed, uint
         double *outs = reinterpret_cast<double *>(ub + off_out);
         RoundCtl *ctl_keep = reinterpret_cast<RoundCtl *>(ub + off_ctl);
         RoundCtl *ctl_pre = ctx->ctl3.as<RoundCtl>();
-        double *rec_val = ctx->rec.as<double>();
+        uint4 *rec_bins = ctx->rec.as<uint4>();
+        double *rec_val = reinterpret_cast<double *>(rec_bins + static_cast<size_t>(bin_rec_vecs(D)) * m);
         double *rec_wgt = rec_val + m;
         double *rec_dens = rec_wgt + m;
-        int32_t *rec_slot = reinterpret_cast<int32_t *>(rec_dens + static_cast<size_t>(nch) * m);
-        uint8_t *rec_ok = reinterpret_cast<uint8_t *>(rec_slot + static_cast<size_t>(D) * m);
+        uint8_t *rec_ok = reinterpret_cast<uint8_t *>(rec_dens + static_cast<size_t>(nch) * m);
         const uint64_t ctr0 = counter_base + static_cast<uint64_t>(done);
         k_mc_forward<<<static_cast<unsigned>(nb_f), kFwdBlock, 0, ctx->stream>>>(
             ctx->progs.as<ChannelProgram>(), ctx->edges.as<double>(), cp_ptr(ctx), nch, D, B, seed, ctr0, nullptr, m,
@@ -1530,13 +1510,13 @@ int chili_gpu_generate_unweighted(chili_ctx *ctx, int64_t n, uint64_t seed, uint
         n_pre_tot += n_pre;
         if (pipe) {
             if ((rc = launch_pipeline(ctx, ctx->mom_soa.as<double>(), ctx->ich.as<int32_t>(), m, n_pre, B, false,
-                                      ctl_pre, rec_val, rec_wgt, rec_ok, rec_slot, rec_dens)))
+                                      ctl_pre, rec_val, rec_wgt, rec_ok, rec_bins, rec_dens)))
                 return rc;
         } else {
             k_mc_weight<<<static_cast<unsigned>(nb_w), kWgtBlock, 0, ctx->stream>>>(
                 ctx->progs.as<ChannelProgram>(), ctx->edges.as<double>(), alpha_ptr(ctx), nch, D, B, NE,
                 ctx->mom_soa.as<double>(), m, ctx->ich.as<int32_t>(), ctx->list.as<int32_t>(), ctl_pre,
-                ctx->f_dev.as<IntegrandDesc>(), 0, rec_val, rec_wgt, rec_ok, rec_slot, rec_dens, pp_ptr(ctx));
+                ctx->f_dev.as<IntegrandDesc>(), 0, rec_val, rec_wgt, rec_ok, rec_bins, rec_dens, pp_ptr(ctx));
             LAUNCHED();
         }
         k_unw_flag<<<static_cast<unsigned>(nb_f), kFwdBlock, 0, ctx->stream>>>(

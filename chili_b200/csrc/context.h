@@ -16,6 +16,7 @@
 #include "chili_gpu.h"
 #include "channel_program.h"
 #include "mc_device.cuh"
+#include "phase_dev.cuh"
 
 using namespace chili_dev;
 
@@ -63,25 +64,18 @@ void flow_release(chili_ctx *ctx);
 // Frees the batched integrands' state (batch.cu).
 void batch_release(chili_ctx *ctx);
 // Launches the last step of one tile of the phased weight pass (base = first
-// listed point of the tile, T = tile capacity).
-using TileFn = std::function<int(long long base, long long T)>;
+// listed point of the tile, T = tile capacity, dens the channel densities).
+using TileFn = std::function<int(long long base, long long T, Densities dens)>;
 // The phased weight pass (chili_gpu.cu) over listed points of a momenta
 // buffer [slot][component][m]; rec_dens may be null.
-// fused (optional): the standard combine step's outputs; when given (and the
-// "pipeline_fuse" option is on) the combine runs inside the channel kernel
-// and `combine` is not called.
-struct PPFusedOut {
-    double *rec_val, *rec_wgt;
-    uint8_t *rec_ok;
-};
 int pipeline_run(chili_ctx *ctx, const double *mom_soa, long long m, const int32_t *list, const int32_t *ich,
-                 const long long *n_list, long long n_pre, int bins, bool opt, int32_t *rec_slot, double *rec_dens,
-                 const TileFn &combine, const PPFusedOut *fused = nullptr);
+                 const long long *n_list, long long n_pre, int bins, bool opt, uint4 *rec_bins, double *rec_dens,
+                 const TileFn &combine);
 
 // One phased weight pass with explicit buffers and no host round trip (so
 // that a graph can capture it; chili_gpu.cu): T launch points, of which the
 // first *n_list are listed; tile-local buffers with stride T, records with
-// stride mr; hints, sorted and widths may be null (plain bin search).
+// stride mr.
 struct PPPass {
     const PointProgram *pp;       // device
     const PointProgram *pp_host;  // host copy: launch sizes
@@ -91,13 +85,11 @@ struct PPPass {
     const long long *n_list;
     long long T, mr;
     int bins;
-    const double *grids;
-    const uint32_t *hints;
-    const uint8_t *sorted;
-    const double *widths;
-    double *node_soa, *memo, *dcv, *vwv;
+    GridTables tables;
+    double *node_soa, *memo, *vwv;
     uint8_t *cfail;
-    int32_t *ich_tile, *rec_slot;
+    int32_t *ich_tile;
+    uint4 *rec_bins;
     double *rec_dens;
     const double *alpha;
     const IntegrandDesc *f;
@@ -132,10 +124,9 @@ struct chili_ctx {
     bool have_pp = false;      // the set fits the PointProgram limits
     bool use_pp = true;        // option "point_program"
     bool use_pipeline = true;  // option "pipeline": phased weight pass
-    bool fuse_combine = false;  // option "pipeline_fuse": combine step inside the channel kernel (slower: off)
     long long gen_ppt = 2;       // option "vegas_gen_ppt": points per thread of chili_gpu_vegas_generate
     bool vegas_fused = true;     // option "vegas_fused": a whole adapting Vegas iteration in one launch
-    bool hints_stale = false;    // the grids changed since the hint tables were built
+    bool hints_stale = false;    // the grids changed since the search tables were built
     bool defer_train = false;  // option "defer_train": iterations collect training data, Train is the caller's
     bool batch_phased = true;  // option "batch_phased": batched multichannel tasks by the phased weight pass
     bool batch_grouped = true;  // option "batch_grouped": the phased tasks in waves, one launch per step and wave
@@ -153,9 +144,8 @@ struct chili_ctx {
     long long max_rounds = 100000;  // option "max_rounds": chunks an iteration may take before CHILI_ERR_TIMEOUT
     PointProgram pp_host;      // host copy (sizes of the memo buffers)
     DevBuf node_soa, memo, cfail, dcv, vwv;
-    DevBuf arrivals;  // per point block of a tile: the fused combine's arrival counters (zero between launches)
     DevBuf v_arrive;  // the fused Vegas iteration's arrival counter (zero between launches)
-    DevBuf hints, sorted, widths;  // hinted bin search tables and bin widths of the grids
+    DevBuf cells, widths;  // search entries and scaled bin widths of the grids (grid.cuh)
     DevBuf ich_tile;
     // channel weights: alpha[CH], best[CH], cp[CH], min_diff
     DevBuf alpha_buf;

@@ -489,10 +489,10 @@ int flow_points(chili_ctx *ctx, bool train, long long m, uint64_t seed, uint64_t
         c.feat = feat;
         c.logprior = logprior;
         if (int rc = pipeline_run(ctx, S.fmom.as<double>(), m, S.flist.as<int32_t>(), ch, S.fcount.as<long long>(),
-                                  m, ctx->bins, false, nullptr, nullptr, [&](long long base, long long T) -> int {
+                                  m, ctx->bins, false, nullptr, nullptr, [&](long long base, long long T, Densities dens) -> int {
                                       CombineArgs t = c;
                                       t.node_soa = ctx->node_soa.as<double>();
-                                      t.dcv = ctx->dcv.as<double>();
+                                      t.dcv = dens.p;
                                       t.vwv = ctx->vwv.as<double>();
                                       t.ich_tile = ctx->ich_tile.as<int32_t>();
                                       t.base = base;

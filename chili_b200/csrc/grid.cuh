@@ -7,6 +7,7 @@
 // reference's (compiled without FMA contraction) for identical inputs.
 #pragma once
 
+#include "chili_gpu.h"
 #include "common.cuh"
 
 namespace chili_dev {
@@ -112,87 +113,122 @@ __device__ __forceinline__ int train_slot(int d, int bins, int b) {
     return s;  // b == -1 and d == 0 gives -1
 }
 
-// ------------------------------------------------------------ hinted search
-// For a monotone edge table the cells of a uniform H-cell grid over [0, 1)
-// bracket lower_bound: with cell(v) = clamp((int)(v*H), 0, H) (monotone in v),
-// every edge in a cell below x's cell is < x and every edge in a cell above it
-// is > x, so lower_bound(x) lies in [hint[c], hint[c+1]) where hint[j] counts
-// the edges e[k], k < bins, with cell(e[k]) < j.  hint has H+1 entries per
-// (grid, dim); sorted[] marks the tables the shortcut may use (monotone, no
-// NaN); other tables and x outside [0, 1) take the plain search.
-constexpr int kHintPerBin = 2;
+// ------------------------------------------------------------ cell search
+// FindBin through a table of H uniform cells over [0, 1), H a power of two.
+// Every coordinate v in [0, 1) has an integer image g(v) = floor(v H 2^F),
+// exact and monotone: one round-down multiply-add onto 2^52 leaves it in the
+// low word.  Its upper bits are the cell, its lower F bits the place in the
+// cell.  A cell's entry packs the number of edges e[k], k < bins, in lower
+// cells and the places f1 <= f2 of the cell's first two edges, so that one
+// multiply-add counts the edges below x:
+//   entry   = start << (2F+2) | (2^(F+1) - 1 - f1) << (F+1) | (2^F - 1 - f2)
+//   entry + f (2^(F+1) + 1): f > f1 carries into start, f > f2 sets bit F
+// (an absent edge's field is 0).  g(x) > g(e) implies x > e and g(x) < g(e)
+// implies x < e, so the count is FindBin + 1.  A field of ones in the sum is
+// an equal place (2^-F of the points); bit F set in the entry marks a cell
+// with more than two edges; both compare the doubles from the cell's first
+// edge on.  x outside [0, 1) and rows that are not monotone inside [0, 1)
+// (every entry start all ones, bit F) take the plain search.  The bins are
+// those of find_bin in every case.
+//
+// Why: a hint of two cells per bin and a binary search on the edges took 96
+// issued instructions and 16 shared-memory wavefronts per search and bound
+// the channel step by issue; this search is one 4-byte and (for the width)
+// one 8-byte table read.  8 cells per bin: on trained 100-bin grids 1% of a
+// grid's own points fall in a cell with more than two edges (4 per bin: 4%).
+constexpr int kMaxCells = 4096;
 
-__device__ __forceinline__ int edge_cell(double v, int H) {
-    if (!(v > 0.0)) return 0;  // also NaN (excluded by sorted[] anyway)
-    const double p = v * static_cast<double>(H);
-    return p >= static_cast<double>(H) ? H : static_cast<int>(p);
+__host__ __device__ inline int grid_cells(int bins) {
+    int h = 64;
+    while (h < 8 * bins && h < kMaxCells) h <<= 1;
+    return h;
 }
 
-template <bool NC = true>
-__device__ __forceinline__ int find_bin_hinted(const double *__restrict__ e, const uint32_t *__restrict__ hint,
-                                               bool sorted, int bins, int H, double x) {
-    if (!sorted || !(x >= 0.0 && x < 1.0)) return find_bin<NC>(e, bins, x);
-    const int c = static_cast<int>(x * static_cast<double>(H));  // < H for x < 1
-    const uint32_t hp = tab_ld<NC>(hint + c);  // hint[c] | hint[c+1] << 16
-    int first = static_cast<int>(hp & 0xffffu);
-    int len = static_cast<int>(hp >> 16) - first;
-    while (len > 0) {  // lower_bound inside the bracket
-        const int half = len >> 1;
-        const int mid = first + half;
-        if (tab_ld<NC>(e + mid) < x) {
-            first = mid + 1;
-            len = len - half - 1;
-        } else {
-            len = half;
-        }
+// Place bits: 11 where the count and the marker fit the remaining 8 bits, else
+// 9 (12 bits; rows of more than 4094 bins are always marked).
+__host__ __device__ constexpr int cell_fbits(int bins) { return bins <= 254 ? 11 : 9; }
+
+// FindBin + 1 of x from the row's entries (TABLE_NC: in global memory, else
+// staged in shared memory), cells = grid_cells(bins), scale = cells 2^F;
+// slow: the entry does not decide, and the count is find_bin's.
+template <bool TABLE_NC, int F>
+__device__ __forceinline__ int cell_count(const uint32_t *__restrict__ entries, int cells, double scale, double x,
+                                          bool &slow) {
+    const double t = __fma_rd(x, scale, 0x1p52);
+    const uint32_t lo = static_cast<uint32_t>(__double2loint(t));
+    const uint32_t q = tab_ld<TABLE_NC>(entries + ((lo >> F) & (cells - 1)));
+    const uint32_t s = q + (lo & ((1u << F) - 1u)) * ((2u << F) + 1u);
+    const uint32_t inv = ~s;
+    slow = __double2hiint(t) != 0x43300000 || lo >= (static_cast<uint32_t>(cells) << F) || (q & (1u << F)) != 0 ||
+           (inv & ((1u << F) - 1u)) == 0 || (inv & (((2u << F) - 1u) << (F + 1))) == 0;
+    return static_cast<int>(s >> (2 * F + 2)) + static_cast<int>((s >> F) & 1u);
+}
+
+// FindBin + 1 where the entry does not decide, on the row of edges e (global
+// memory): from the cell's first edge, four independent loads at a time.
+template <bool TABLE_NC, int F>
+__device__ __forceinline__ int cell_count_slow(const double *__restrict__ e, const uint32_t *__restrict__ entries,
+                                               int bins, int cells, double scale, double x) {
+    if (!(x >= 0.0 && x < 1.0)) return find_bin<true>(e, bins, x) + 1;
+    const uint32_t lo = static_cast<uint32_t>(__double2loint(__fma_rd(x, scale, 0x1p52)));
+    int k = static_cast<int>(tab_ld<TABLE_NC>(entries + ((lo >> F) & (cells - 1))) >> (2 * F + 2));
+    if (k == static_cast<int>(0xffffffffu >> (2 * F + 2))) return find_bin<true>(e, bins, x) + 1;
+    for (;;) {
+        int n = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) n += (k + j < bins && __ldg(e + min(k + j, bins)) < x) ? 1 : 0;
+        k += n;
+        if (n < 4) return k;
     }
-    return first - 1;
 }
 
-// The hint table of one (grid, dimension) row of edges e[0..bins], its
-// widths w[k] = e[k+1] - e[k] and its monotone flag, built by one block
-// (every thread of the block calls this).  hint[j] = first k in [0, bins)
-// with cell(e[k]) >= j, packed with hint[j+1] in the upper 16 bits.
-__device__ __forceinline__ void build_hint_row(const double *__restrict__ e, int bins, uint32_t *__restrict__ h,
-                                               uint8_t *__restrict__ sorted, double *__restrict__ w) {
-    const int H = kHintPerBin * bins;
-    int bad = 0;
+// Doubles of a row of scaled widths: bins + 1, rounded to 16 bytes.
+__host__ __device__ inline int width_row(int bins) { return (bins + 2) & ~1; }
+
+// The entries of row (dimension) dim of the grid g (dims x (bins+1) edges)
+// and its scaled widths: ws[0] the reference's reading of bin == SIZE_MAX,
+// ws[1 + k] = (e[k+1] - e[k]) * bins (the factors of
+// AdaptiveMap::GenerateWeight, rounded as there).  Built by one block.
+__device__ __forceinline__ void build_cell_row(const double *__restrict__ g, int dims, int bins, int dim,
+                                               uint32_t *__restrict__ entries, double *__restrict__ ws) {
+    __shared__ uint32_t g_s[CHILI_MAX_BINS];
+    const double *e = g + static_cast<size_t>(dim) * (bins + 1);
+    const int F = cell_fbits(bins), cells = grid_cells(bins);
+    const double scale = static_cast<double>(cells) * static_cast<double>(1 << F), fb = static_cast<double>(bins);
+    const uint32_t mask = (1u << F) - 1u;
+    int bad = bins > 4094;
     for (int k = threadIdx.x; k < bins; k += blockDim.x) {
         const double a = e[k];
-        if (a != a) bad = 1;
-        if (k + 1 < bins && !(a <= e[k + 1])) bad = 1;
-        w[k] = __dsub_rn(e[k + 1], a);
+        if (!(a >= 0.0 && a < 1.0) || (k + 1 < bins && !(a <= e[k + 1]))) bad = 1;
+        g_s[k] = static_cast<uint32_t>(__double2loint(__fma_rd(a, scale, 0x1p52)));
+        ws[1 + k] = __dmul_rn(__dsub_rn(e[k + 1], a), fb);
     }
+    if (threadIdx.x == 0) ws[0] = __dmul_rn(bin_width<false>(g, bins, dim, -1, edge_before_table(dims, bins)), fb);
     bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) *sorted = bad ? 0 : 1;
-    if (bad) return;
-    for (int j = threadIdx.x; j < H; j += blockDim.x) {
-        int lo[2];
-        for (int q = 0; q < 2; ++q) {
-            int first = 0, len = bins;
-            while (len > 0) {
-                const int half = len >> 1, mid = first + half;
-                if (edge_cell(e[mid], H) < j + q) {
-                    first = mid + 1;
-                    len = len - half - 1;
-                } else {
-                    len = half;
-                }
-            }
-            lo[q] = first;
+    for (int j = threadIdx.x; j < cells; j += blockDim.x) {
+        if (bad) {
+            entries[j] = (0xffffffffu << (2 * F + 2)) | 1u << F;
+            continue;
         }
-        h[j] = static_cast<uint32_t>(lo[0]) | (static_cast<uint32_t>(lo[1]) << 16);
+        int first = 0, len = bins;  // edges in lower cells
+        while (len > 0) {
+            const int half = len >> 1, mid = first + half;
+            if (static_cast<int>(g_s[mid] >> F) < j) {
+                first = mid + 1;
+                len = len - half - 1;
+            } else {
+                len = half;
+            }
+        }
+        int in = 0;
+        while (in < 3 && first + in < bins && static_cast<int>(g_s[first + in] >> F) == j) ++in;
+        uint32_t q = static_cast<uint32_t>(first) << (2 * F + 2);
+        if (in > 0) q |= (2u * mask + 1u - (g_s[first] & mask)) << (F + 1);
+        if (in > 1) q |= mask - (g_s[first + 1] & mask);
+        if (in > 2) q = (static_cast<uint32_t>(first) << (2 * F + 2)) | 1u << F;
+        entries[j] = q;
     }
-}
-
-// width(dim, bin) from the precomputed table wt[dim*bins + bin] (the same
-// subtraction as bin_width, done once per grid), the reference's reading of
-// bin == SIZE_MAX from the edges.
-template <bool NC = true>
-__device__ __forceinline__ double bin_width_t(const double *__restrict__ g, const double *__restrict__ wt, int bins,
-                                              int dim, int bin, double before) {
-    if (bin >= 0) return tab_ld<NC>(wt + dim * bins + bin);
-    return bin_width<NC>(g, bins, dim, bin, before);
+    __syncthreads();  // g_s is free for another row
 }
 
 }  // namespace chili_dev

@@ -32,15 +32,14 @@
 namespace chili_dev {
 
 // ------------------------------------------------------------- grid kernels
-// One block per (dim = blockIdx.x, grid = blockIdx.y): the hint table (as
-// pairs hint[j] | hint[j+1] << 16, j < H), the monotone flag and the bin
-// widths of that edge table.
-__global__ void k_build_hints(const double *__restrict__ grids, int dims, int bins, uint32_t *__restrict__ hints,
-                              uint8_t *__restrict__ sorted, double *__restrict__ widths) {
+// One block per (dim = blockIdx.x, grid = blockIdx.y): the cell entries and
+// scaled bin widths of that edge table.
+__global__ void k_build_cells(const double *__restrict__ grids, int dims, int bins, uint32_t *__restrict__ entries,
+                              double *__restrict__ ws) {
     const int d = blockIdx.x, c = blockIdx.y;
     const size_t row = static_cast<size_t>(c) * dims + d;
-    build_hint_row(grids + row * (bins + 1), bins, hints + row * (kHintPerBin * bins), sorted + row,
-                   widths + row * bins);
+    build_cell_row(grids + static_cast<size_t>(c) * dims * (bins + 1), dims, bins, d,
+                   entries + row * grid_cells(bins), ws + row * width_row(bins));
 }
 
 __global__ void k_grid_map(const double *__restrict__ g, int dims, int bins, const double *__restrict__ u,
@@ -58,21 +57,27 @@ __global__ void k_grid_map(const double *__restrict__ g, int dims, int bins, con
     jac[i] = j;
 }
 
-// AdaptiveMap::FindBin / GenerateWeight through the hinted search that the
-// iteration uses (grid.cuh, find_bin_hinted).
-__global__ void k_grid_weight(const double *__restrict__ g, const uint32_t *__restrict__ hints,
-                              const uint8_t *__restrict__ sorted, int dims, int bins, const double *__restrict__ x,
+// AdaptiveMap::FindBin / GenerateWeight through the cell search that the
+// iteration uses (grid.cuh).
+__global__ void k_grid_weight(const double *__restrict__ g, const uint32_t *__restrict__ entries,
+                              const double *__restrict__ ws, int dims, int bins, const double *__restrict__ x,
                               double *__restrict__ w, int32_t *__restrict__ bin, long long n) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
     double jac = 1.0;
-    const double fb = static_cast<double>(bins);
-    const int H = kHintPerBin * bins;
+    const int cells = grid_cells(bins);
     for (int d = 0; d < dims; ++d) {
-        const int b = find_bin_hinted(g + d * (bins + 1), hints + d * H, sorted[d] != 0, bins, H,
-                                      x[i * dims + d]);
-        if (bin) bin[i * dims + d] = b;
-        jac = __dmul_rn(jac, __dmul_rn(bin_width(g, bins, d, b, edge_before_table(dims, bins)), fb));
+        const double *e = g + d * (bins + 1);
+        const uint32_t *en = entries + static_cast<size_t>(d) * cells;
+        const double v = x[i * dims + d];
+        bool slow;
+        int k = cell_fbits(bins) == 11 ? cell_count<true, 11>(en, cells, cells * 2048.0, v, slow)
+                                       : cell_count<true, 9>(en, cells, cells * 512.0, v, slow);
+        if (slow)
+            k = cell_fbits(bins) == 11 ? cell_count_slow<true, 11>(e, en, bins, cells, cells * 2048.0, v)
+                                       : cell_count_slow<true, 9>(e, en, bins, cells, cells * 512.0, v);
+        if (bin) bin[i * dims + d] = k - 1;
+        jac = __dmul_rn(jac, __ldg(ws + d * width_row(bins) + k));
     }
     if (w) w[i] = jac;
 }
@@ -533,16 +538,15 @@ __global__ void __launch_bounds__(kFwdBlock) k_mc_compact(const uint8_t *__restr
 // counter order) can be taken afterwards and only that prefix accumulated:
 //   rec_val, rec_wgt   value f*w and weight (both 0 for a NaN retry)
 //   rec_ok             0 for a NaN retry (MultiChannel.hh:230-236), else 1
-//   rec_slot[j*n+i]    histogram slot of dimension j in the chosen channel's
-//                      histogram (Integrand.hh:91-95), -1 when it would lie
-//                      before the histogram
+//   rec_bins           the bins in the chosen channel's grid (mc_device.cuh,
+//                      for_each_train_slot)
 //   rec_dens[c*n+i]    channel c's density, for the alpha-training terms
 __global__ void __launch_bounds__(kWgtBlock) k_mc_weight(
     const ChannelProgram *__restrict__ progs, const double *__restrict__ grids, const double *__restrict__ alpha,
     int nch, int dims, int bins, int n_ext, const double *__restrict__ mom_soa, long long m,
     const int32_t *__restrict__ ich_arr, const int32_t *__restrict__ list, const RoundCtl *__restrict__ ctl,
     const IntegrandDesc *__restrict__ f, int should_opt, double *__restrict__ rec_val, double *__restrict__ rec_wgt,
-    uint8_t *__restrict__ rec_ok, int32_t *__restrict__ rec_slot, double *__restrict__ rec_dens,
+    uint8_t *__restrict__ rec_ok, uint4 *__restrict__ rec_bins, double *__restrict__ rec_dens,
     const PointProgram *__restrict__ pp) {
     // records are laid out with stride m (the chunk size, known on the host);
     // only the first ctl->n_acc entries are written
@@ -572,12 +576,9 @@ __global__ void __launch_bounds__(kWgtBlock) k_mc_weight(
     rec_ok[i] = ok;
     if (should_opt) {
         const double *g = grids + static_cast<size_t>(c_sel) * dims * (bins + 1);
-        const int base = c_sel * dims * bins;
-        for (int j = 0; j < dims; ++j) {
-            const int b = find_bin(g + j * (bins + 1), bins, xs[j]);
-            const int s = j * bins + b;
-            rec_slot[j * m + i] = s >= 0 ? base + s : -1;
-        }
+        uint16_t *o = reinterpret_cast<uint16_t *>(rec_bins + i * bin_rec_vecs(dims));
+        for (int j = 0; j < dims; ++j) o[j] = static_cast<uint16_t>(8 * (find_bin(g + j * (bins + 1), bins, xs[j]) + 1));
+        o[dims] = static_cast<uint16_t>(c_sel);
     }
 }
 
@@ -640,9 +641,9 @@ __global__ void k_iter_init(long long *__restrict__ iter, long long needed) {
 // val^2 w / dens_j (MultiChannel.hh:167-180).  Dynamic shared memory:
 // (kWgtBlock/32) * nch.
 __global__ void __launch_bounds__(kWgtBlock) k_mc_accum(
-    const RoundCtl *__restrict__ ctl, long long n_rec, int nch, int dims, int hist_size,
+    const RoundCtl *__restrict__ ctl, long long n_rec, int nch, int dims, int bins, int hist_size,
     const double *__restrict__ rec_val,
-    const double *__restrict__ rec_wgt, const uint8_t *__restrict__ rec_ok, const int32_t *__restrict__ rec_slot,
+    const double *__restrict__ rec_wgt, const uint8_t *__restrict__ rec_ok, const uint4 *__restrict__ rec_bins,
     const double *__restrict__ rec_dens, int should_opt, int guard, double *__restrict__ hist,
     double *__restrict__ part) {
     extern __shared__ double atr_s[];  // (kWgtBlock/32) * nch
@@ -656,14 +657,13 @@ __global__ void __launch_bounds__(kWgtBlock) k_mc_accum(
     double dropped = 0;
     const double val2 = val * val;
     if (active && should_opt) {
-        for (int j = 0; j < dims; ++j) {
-            const int s = rec_slot[j * n_rec + i];
+        for_each_train_slot(rec_bins, i, dims, bins, [&](int s) {
             if (s >= 0 && s < hist_size) {
                 if (hist) atomicAdd(hist + s, val2);
             } else {
                 dropped += 1;
             }
-        }
+        });
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double nonfin = 0;
@@ -723,8 +723,8 @@ __global__ void __launch_bounds__(kWgtBlock) k_mc_accum(
 // The bins' sums agree with k_mc_accum's direct adds up to the order of
 // addition.
 __global__ void __launch_bounds__(1024) k_mc_hist(const RoundCtl *__restrict__ ctl, long long n_rec, int dims,
-                                                  int hist_size, const double *__restrict__ rec_val,
-                                                  const int32_t *__restrict__ rec_slot, double *__restrict__ hist) {
+                                                  int bins, int hist_size, const double *__restrict__ rec_val,
+                                                  const uint4 *__restrict__ rec_bins, double *__restrict__ hist) {
     extern __shared__ double sh[];
     for (int k = threadIdx.x; k < hist_size; k += blockDim.x) sh[k] = 0.0;
     __syncthreads();
@@ -733,10 +733,9 @@ __global__ void __launch_bounds__(1024) k_mc_hist(const RoundCtl *__restrict__ c
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n; i += stride) {
         const double v = rec_val[i];
         const double v2 = v * v;
-        for (int j = 0; j < dims; ++j) {
-            const int s = rec_slot[j * n_rec + i];
+        for_each_train_slot(rec_bins, i, dims, bins, [&](int s) {
             if (s >= 0 && s < hist_size) atomicAdd(sh + s, v2);
-        }
+        });
     }
     __syncthreads();
     for (int k = threadIdx.x; k < hist_size; k += blockDim.x) {

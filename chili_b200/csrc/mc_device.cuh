@@ -41,6 +41,37 @@ struct RoundCtl {
 
 constexpr int kPartFixed = 10;  // n, min, max, sum, sum2, nfin, nan, nonfin, wmax, dropped
 
+// A record's histogram bins: dims halfwords 8 (FindBin + 1) in the record's
+// channel (the byte offsets the channel step reads its widths at), then the
+// channel, in bin_rec_vecs(dims) 16-byte words (one row per
+// record, so that the channel step writes a point's bins in two or three
+// stores and the accumulation reads them in as many).
+__host__ __device__ inline int bin_rec_vecs(int dims) { return (dims + 8) / 8; }
+
+// fn(s) for every dimension of record r: the flat histogram slot s of the
+// record's channel the way Integrand::AddTrainData indexes it
+// (Integrand.hh:91-95; a FindBin of SIZE_MAX wraps to the previous
+// dimension's last bin), -1 where it lies before the histogram.
+template <class Fn>
+__device__ __forceinline__ void for_each_train_slot(const uint4 *__restrict__ rec_bins, long long r, int dims, int bins,
+                                                    Fn fn) {
+    const int nv = bin_rec_vecs(dims);
+    const uint4 *p = rec_bins + r * nv;
+    const int base = static_cast<int>(reinterpret_cast<const uint16_t *>(p)[dims]) * dims * bins;
+    for (int j = 0; j < nv; ++j) {
+        const uint4 v = p[j];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+            const int d = 8 * j + h;
+            if (d < dims) {
+                const int s = d * bins + static_cast<int>(((w[h >> 1] >> (16 * (h & 1))) & 0xffffu) >> 3) - 1;
+                fn(s >= 0 ? base + s : -1);
+            }
+        }
+    }
+}
+
 // libstdc++ lower_bound over cp[0..n) (probe order of bits/stl_algobase.h).
 __device__ __forceinline__ int lower_bound_d(const double *__restrict__ a, int n, double v) {
     int first = 0, len = n;

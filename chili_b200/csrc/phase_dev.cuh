@@ -96,7 +96,7 @@ __device__ __forceinline__ void pp_items_block(const PointProgram *__restrict__ 
                                    : massive_prop_weight(pp->dw_mass[k], pp->dw_width[k], smin, pp->dw_smax[k], s, u);
         }
         double *o = memo + static_cast<long long>(pp->memo_dw + 2 * k) * m + i;
-        o[0] = w;
+        o[0] = w / kTwoPi;  // WgtDecays divides by 2 pi per decay (Channel.cc:111)
         o[m] = u;
         return;
     }
@@ -187,20 +187,36 @@ __device__ __forceinline__ double eval_momenta_soa(const IntegrandDesc *__restri
     return (top2 ? big1 * big2 : sum) * tprod;
 }
 
+// Every channel's densities: channel c's at tile point i is
+// p[c * stride + i] (the per-record array of an iteration from the tile's
+// first record on, or a tile's own buffer).
+struct Densities {
+    double *p;
+    long long stride;
+};
+
 __device__ __forceinline__ void pp_combine_point(const PointProgram *__restrict__ pp, const double *__restrict__ alpha,
-                                                 const double *dcv, const double *vwv,
+                                                 Densities dens, const double *__restrict__ vwv,
                                                  const double *__restrict__ node_soa, long long m, long long i,
                                                  long long r, const IntegrandDesc *__restrict__ f,
                                                  double *__restrict__ rec_val, double *__restrict__ rec_wgt,
-                                                 uint8_t *__restrict__ rec_ok, bool coherent) {
+                                                 uint8_t *__restrict__ rec_ok) {
     double acc = 0.0;
     const int nch = pp->nch;
-    for (int c = 0; c < nch; ++c) {
-        const long long q = static_cast<long long>(c) * m + i;
-        // written by other blocks of this launch: read from L2, past L1
-        const double d = coherent ? __ldcg(dcv + q) : dcv[q];
-        const double v = coherent ? __ldcg(vwv + q) : vwv[q];
-        acc += __ldg(alpha + c) / d / v;
+    // eight channels' values in flight before the first division: one at a
+    // time, the divisions' slow-path branches kept the next loads back
+    const double *dp = dens.p + i, *vp = vwv + i;
+    for (int c0 = 0; c0 < nch; c0 += 8) {
+        double d[8], v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int c = min(c0 + k, nch - 1);
+            d[k] = __ldg(dp + c * dens.stride);
+            v[k] = __ldg(vp + c * m);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (c0 + k < nch) acc += __ldg(alpha + c0 + k) / d[k] / v[k];
     }
     double wgt = 1.0 / acc;
     const double fv = eval_momenta_soa(f, node_soa, m, i, pp->n_ext);
@@ -215,75 +231,167 @@ __device__ __forceinline__ void pp_combine_point(const PointProgram *__restrict_
     rec_ok[r] = ok;
 }
 
-// Channel c's density and VEGAS weight at tile point i (record r).
-// TAB: grids / hints / sorted / widths are channel c's own tables staged in
-// shared memory (plain loads), instead of the tables of every channel in
-// global memory.
-template <int DIMS, bool HINTS, bool TAB = false>
-__device__ __forceinline__ void pp_channel_point(
-    const PointProgram *__restrict__ pp, const double *__restrict__ grids, const uint32_t *__restrict__ hints,
-    const uint8_t *__restrict__ sorted, const double *__restrict__ widths, int bins, const double *__restrict__ memo,
-    const uint8_t *__restrict__ cfail, const int32_t *__restrict__ ich_tile, long long m, long long mr,
-    int should_opt, double *__restrict__ dcv, double *__restrict__ vwv, int32_t *__restrict__ rec_slot,
-    double *__restrict__ rec_dens, long long i, long long r, int c) {
+// The grid set's search tables (grid.cuh), every channel's rows back to back.
+struct GridTables {
+    const double *edges;      // [nch][dims][bins + 1]
+    const uint32_t *entries;  // [nch][dims][grid_cells(bins)]
+    const double *ws;         // [nch][dims][width_row(bins)]
+};
+
+// Shared-memory bytes of the channel step: the position and factor rows, and
+// one channel's tables where they are staged.
+constexpr int kMaxFactors = 2 * CHILI_MAX_DECAYS + 1;
+__host__ __device__ inline size_t channel_smem_bytes(int dims, int bins, bool tables) {
+    const size_t rows = 16 * ((sizeof(int32_t) * (2 * static_cast<size_t>(dims) + kMaxFactors) + 15) / 16);
+    return rows + (tables ? static_cast<size_t>(dims) * (4 * static_cast<size_t>(grid_cells(bins)) + 8 * width_row(bins)) : 0);
+}
+
+// 16 bytes from global to shared memory (both 16-byte aligned), and the wait
+// for this thread's copies.
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+// The channel step of one block: channel c's density (the product of its
+// items in the reference's order, Channel.cc:40-61) and its VEGAS weight at
+// the tile points [i0, i1) on the uniforms that the position map selects, the
+// density record and, for the point's own channel, its bins record.  When c's
+// chain fails, its last uniform is the one the shared buffer still holds: the
+// last uniform of the latest earlier channel whose chain did not fail (zero
+// if none).  TAB: channel c's entries and widths are staged in shared memory
+// first; the edges, which only undecided searches read, stay in global
+// memory.  Three passes over the dimensions: the uniforms are loaded, then
+// counted without a branch (the undecided ones noted in a mask and searched
+// afterwards: 0.7% of them on trained 200-bin grids, but some lane of a warp
+// in every fifth search), then the widths multiplied in the reference's
+// order.  smem: channel_smem_bytes.
+template <int DIMS, bool TAB, int F>
+__device__ __forceinline__ void pp_channel_block(const PointProgram *__restrict__ pp, const GridTables &T, int bins,
+                                                 const double *__restrict__ memo, const uint8_t *__restrict__ cfail,
+                                                 const int32_t *__restrict__ ich_tile, long long m, int should_opt,
+                                                 Densities dens, double *__restrict__ vwv,
+                                                 uint4 *__restrict__ rec_bins, long long base, long long i0,
+                                                 long long i1, int c, void *smem) {
+    const int cells = grid_cells(bins);
+    const double scale = static_cast<double>(cells) * static_cast<double>(1 << F);
+    int32_t *pos_s = static_cast<int32_t *>(smem);  // [2][DIMS]: chain found, chain failed
+    uint32_t *en_s = reinterpret_cast<uint32_t *>(static_cast<char *>(smem) + channel_smem_bytes(DIMS, bins, false));
+    double *ws_s = reinterpret_cast<double *>(en_s + static_cast<size_t>(DIMS) * cells);
     const PPChannel &C = pp->ch[c];
-    const bool fail = cfail[C.chain * m + i] != 0;
-    double wdec = 1;
-    for (int k = 0; k < C.n_dec; ++k) {
-        wdec *= memo[static_cast<long long>(pp->memo_dw + 2 * C.dw[k]) * m + i];
-        wdec /= kTwoPi;
+    const double *g = T.edges + static_cast<size_t>(c) * DIMS * (bins + 1);
+    const uint32_t *en = T.entries + static_cast<size_t>(c) * DIMS * cells;
+    const int wn = width_row(bins);
+    const double *ws = T.ws + static_cast<size_t>(c) * DIMS * wn;
+    for (int p = threadIdx.x; p < 2 * DIMS; p += blockDim.x)
+        pos_s[p] = p < DIMS ? pp->pos_src[c][p] : pp->pos_src_fail[c][p - DIMS];
+    // the density's factors: decay propagators, two-body decays, the chain
+    const int n_dec = C.n_dec, n_fac = n_dec + C.n_sd, chain = C.chain;
+    int32_t *fac_s = pos_s + 2 * DIMS;
+    for (int k = threadIdx.x; k <= n_fac; k += blockDim.x)
+        fac_s[k] = k < n_dec ? pp->memo_dw + 2 * C.dw[k]
+                             : (k < n_fac ? pp->memo_sw + 3 * C.sw[k - n_dec] : pp->memo_chain + 2 * chain);
+    if constexpr (TAB) {
+        // all copies in flight at once (rows are multiples of 16 bytes): a
+        // loop of loads and stores took one memory latency per pass of the block
+        const char *src = reinterpret_cast<const char *>(en), *srcw = reinterpret_cast<const char *>(ws);
+        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(en_s));
+        const uint32_t dstw = static_cast<uint32_t>(__cvta_generic_to_shared(ws_s));
+        for (int k = threadIdx.x; k < DIMS * (cells >> 2); k += blockDim.x) copy16_async(dst + 16 * k, src + 16 * k);
+        for (int k = threadIdx.x; k < DIMS * (wn >> 1); k += blockDim.x) copy16_async(dstw + 16 * k, srcw + 16 * k);
+        copy_async_wait();
+        en = en_s;
+        ws = ws_s;
     }
-    const double wt = memo[static_cast<long long>(pp->memo_chain + 2 * C.chain) * m + i];
-    double ws = 1;
-    for (int k = 0; k < C.n_sd; ++k) ws *= memo[static_cast<long long>(pp->memo_sw + 3 * C.sw[k]) * m + i];
-    const double dc = wdec * wt * ws;
-    double x[DIMS];
-    if (!fail) {
-        const int16_t *pos = pp->pos_src[c];
+    __syncthreads();
+    const long long ms = m;
+    double *dens_c = dens.p + c * dens.stride, *vw_c = vwv + c * ms;
+    const uint8_t *fail_c = cfail + chain * ms;
+    const unsigned row_bytes = static_cast<unsigned>(m) * 8u;  // tiles stay below 2^28 points
+    constexpr int NW = 4 * ((DIMS + 8) / 8);                   // words of a bins record
+    constexpr int kFacAhead = 2;
+    uint8_t fail_next = i0 + threadIdx.x < i1 ? fail_c[i0 + threadIdx.x] : 0;
+#pragma unroll 1
+    for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        const char *mi = reinterpret_cast<const char *>(memo + i);
+        auto at = [&](int slot) {  // memo slot of point i
+            return *reinterpret_cast<const double *>(mi + static_cast<unsigned long long>(row_bytes) *
+                                                              static_cast<unsigned>(slot));
+        };
+        const bool fail = fail_next != 0;
+        if (i + blockDim.x < i1) fail_next = fail_c[i + blockDim.x];
+        const int32_t *pos = pos_s + (fail ? DIMS : 0);
+        double x[DIMS];
 #pragma unroll
-        for (int p = 0; p < DIMS; ++p) x[p] = memo[static_cast<long long>(pos[p]) * m + i];
-    } else {
-        const int16_t *pos = pp->pos_src_fail[c];
-#pragma unroll
-        for (int p = 0; p < DIMS - 1; ++p) x[p] = memo[static_cast<long long>(pos[p]) * m + i];
-        double stale = 0.0;
-        for (int q = c - 1; q >= 0; --q) {
-            if (!cfail[pp->ch[q].chain * m + i]) {
-                stale = memo[static_cast<long long>(pp->pos_src[q][DIMS - 1]) * m + i];
-                break;
-            }
-        }
-        x[DIMS - 1] = stale;
-    }
-    const int H = kHintPerBin * bins;
-    const double fb = static_cast<double>(bins);
-    const double before = edge_before_table(DIMS, bins);
-    const double *g = TAB ? grids : grids + static_cast<size_t>(c) * DIMS * (bins + 1);
-    const uint32_t *hc = HINTS ? (TAB ? hints : hints + static_cast<size_t>(c) * DIMS * H) : nullptr;
-    const double *wc = HINTS ? (TAB ? widths : widths + static_cast<size_t>(c) * DIMS * bins) : nullptr;
-    const uint8_t *sc = HINTS ? (TAB ? sorted : sorted + c * DIMS) : nullptr;
-    const bool chosen = should_opt && c == ich_tile[i];
-    double vw = 1.0;
-#pragma unroll
-    for (int p = 0; p < DIMS; ++p) {
-        int b;
-        double wdt;
-        if constexpr (HINTS) {
-            b = find_bin_hinted<!TAB>(g + p * (bins + 1), hc + p * H, tab_ld<!TAB>(sc + p) != 0, bins, H, x[p]);
-            wdt = bin_width_t<!TAB>(g, wc, bins, p, b, before);
+        for (int p = 0; p < DIMS - 1; ++p) x[p] = at(pos[p]);
+        if (!fail) {
+            x[DIMS - 1] = at(pos[DIMS - 1]);
         } else {
-            b = find_bin<!TAB>(g + p * (bins + 1), bins, x[p]);
-            wdt = bin_width<!TAB>(g, bins, p, b, before);
+            double stale = 0.0;
+            for (int k = c - 1; k >= 0; --k) {
+                if (!cfail[pp->ch[k].chain * ms + i]) {
+                    stale = at(pp->pos_src[k][DIMS - 1]);
+                    break;
+                }
+            }
+            x[DIMS - 1] = stale;
         }
-        vw = __dmul_rn(vw, __dmul_rn(wdt, fb));
-        if (chosen) {
-            const int s = p * bins + b;
-            rec_slot[p * mr + r] = s >= 0 ? c * DIMS * bins + s : -1;
+        // the first factors loaded together, before the first product waits
+        const double wt = at(fac_s[n_fac]);
+        double fv[kFacAhead], wdec = 1, sw = 1;
+#pragma unroll
+        for (int k = 0; k < kFacAhead; ++k) fv[k] = at(fac_s[min(k, n_fac)]);
+        const int own = should_opt ? ich_tile[i] : -1;
+#pragma unroll
+        for (int k = 0; k < kFacAhead; ++k) {
+            if (k < n_dec) wdec *= fv[k];
+            else if (k < n_fac) sw *= fv[k];
+        }
+        for (int k = kFacAhead; k < n_fac; ++k) {
+            if (k < n_dec) wdec *= at(fac_s[k]);
+            else sw *= at(fac_s[k]);
+        }
+        const double dc = wdec * wt * sw;
+        uint32_t rec[NW], todo = 0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) rec[k] = 0;
+#pragma unroll
+        for (int p = 0; p < DIMS; ++p) {
+            bool slow;
+            const int n = cell_count<!TAB, F>(en + p * cells, cells, scale, x[p], slow);
+            if (slow) todo |= 1u << p;
+            else rec[p >> 1] |= static_cast<uint32_t>(n) << (16 * (p & 1) + 3);
+        }
+        while (todo) {
+            const int p = __ffs(todo) - 1;
+            todo &= todo - 1;
+            double v = x[DIMS - 1];
+            if (p < DIMS - 1) v = at(pos[p]);
+            const uint32_t n = static_cast<uint32_t>(cell_count_slow<!TAB, F>(g + p * (bins + 1), en + p * cells, bins,
+                                                                              cells, scale, v))
+                               << (16 * (p & 1) + 3);
+#pragma unroll
+            for (int k = 0; k < (DIMS + 1) / 2; ++k)  // masks, not an index: rec stays in registers
+                rec[k] |= n & (0u - static_cast<uint32_t>(k == (p >> 1)));
+        }
+        double vw = 1.0;
+#pragma unroll
+        for (int p = 0; p < DIMS; ++p) {
+            const uint32_t off = (rec[p >> 1] >> (16 * (p & 1))) & 0xffffu;
+            vw = __dmul_rn(vw, tab_ld<!TAB>(reinterpret_cast<const double *>(
+                                   reinterpret_cast<const char *>(ws + p * wn) + off)));
+        }
+        dens_c[i] = dc;
+        vw_c[i] = vw;
+        if (c == own) {
+            rec[DIMS >> 1] |= static_cast<uint32_t>(c) << (16 * (DIMS & 1));
+            uint4 *o = rec_bins + (base + i) * (NW / 4);
+#pragma unroll
+            for (int k = 0; k < NW / 4; ++k) o[k] = make_uint4(rec[4 * k], rec[4 * k + 1], rec[4 * k + 2], rec[4 * k + 3]);
         }
     }
-    dcv[static_cast<long long>(c) * m + i] = dc;
-    vwv[static_cast<long long>(c) * m + i] = vw;
-    if (rec_dens) rec_dens[static_cast<long long>(c) * mr + r] = dc;
 }
 
 // (The body as a device function, so that a grouped launch can run it for
