@@ -567,10 +567,10 @@ __global__ void __launch_bounds__(256) k_g_channel(WaveDev W, int lo, int hi, lo
     if (i0 >= end) return;
     const long long i1 = i0 + W.ch_pts < end ? i0 + W.ch_pts : end;
     if (cell_fbits(P.bins) == 11)
-        pp_channel_block<DIMS, TAB, 11>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms, 1,
+        pp_channel_block<DIMS, TAB, 11, true>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms,
                                         Densities{P.dens, P.ms}, P.vwv, P.bin_rec, 0, i0, i1, c, smem);
     else
-        pp_channel_block<DIMS, TAB, 9>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms, 1,
+        pp_channel_block<DIMS, TAB, 9, true>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms,
                                         Densities{P.dens, P.ms}, P.vwv, P.bin_rec, 0, i0, i1, c, smem);
 }
 

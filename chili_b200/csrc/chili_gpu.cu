@@ -14,6 +14,8 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "chili_gpu.h"
@@ -48,7 +50,7 @@ GridTables grid_tables(const chili_ctx *ctx) {
 template <int D>
 int launch_channel(chili_ctx *ctx, const PointProgram *pp, const GridTables &G, int bins, const double *memo,
                    const uint8_t *cfail, const int32_t *ich_tile, const long long *n_list, long long base, long long T,
-                   int opt, Densities dens, double *vwv, uint4 *rec_bins, int nch, long long n) {
+                   Densities dens, double *vwv, uint4 *rec_bins, double *x_own, int nch, long long n) {
     const bool tab = ctx->channel_tables && channel_smem_bytes(D, bins, true) <= kMaxChannelTab;
     const size_t smem = channel_smem_bytes(D, bins, tab);
     // as many threads per block as keep 32 warps on an SM beside the tables
@@ -60,12 +62,16 @@ int launch_channel(chili_ctx *ctx, const PointProgram *pp, const GridTables &G, 
     points = std::max(points, (T / 65535 / threads + 1) * threads);  // gridDim.y stays below 65536
     const dim3 grid(static_cast<unsigned>(nch), static_cast<unsigned>((T + points - 1) / points));
     const bool f11 = cell_fbits(bins) == 11;
-    auto kern = tab ? (f11 ? k_pp_channel<D, true, 11> : k_pp_channel<D, true, 9>)
-                    : (f11 ? k_pp_channel<D, false, 11> : k_pp_channel<D, false, 9>);
+    auto pick = [&](auto rec) {
+        constexpr bool R = decltype(rec)::value;
+        return tab ? (f11 ? k_pp_channel<D, true, 11, R> : k_pp_channel<D, true, 9, R>)
+                   : (f11 ? k_pp_channel<D, false, 11, R> : k_pp_channel<D, false, 9, R>);
+    };
+    auto kern = rec_bins ? pick(std::true_type{}) : pick(std::false_type{});
     if (smem > 48 * 1024)
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    kern<<<grid, threads, smem, ctx->stream>>>(pp, G, bins, memo, cfail, ich_tile, n_list, base, T, opt, dens, vwv,
-                                               rec_bins, static_cast<int>(points));
+    kern<<<grid, threads, smem, ctx->stream>>>(pp, G, bins, memo, cfail, ich_tile, n_list, base, T, dens, vwv,
+                                               rec_bins ? static_cast<void *>(rec_bins) : x_own, static_cast<int>(points));
     LAUNCHED();
     return CHILI_OK;
 }
@@ -88,6 +94,99 @@ int launch_channel_dims(chili_ctx *ctx, int dims, A... a) {
 
 }  // namespace
 
+namespace {
+
+// The tile buffers of the phased pass for T points, for a whole number of
+// 2^16 points: the accepted count of a chunk varies from call to call, and a
+// buffer that grew by a few points each time would be reallocated (a device
+// synchronisation) each time.
+cudaError_t pipeline_buffers(chili_ctx *ctx, long long T, bool own_dens) {
+    const PointProgram &P = ctx->pp_host;
+    const long long Ta = (T + 65535) / 65536 * 65536;
+    const std::pair<DevView *, size_t> want[] = {
+        {&ctx->node_soa, sizeof(double) * 4 * P.n_nodes * Ta},
+        {&ctx->memo, sizeof(double) * std::max(1, P.n_memo) * Ta},
+        {&ctx->vwv, sizeof(double) * ctx->nch * Ta},
+        {&ctx->dcv, own_dens ? sizeof(double) * ctx->nch * Ta : 0},
+        {&ctx->ich_tile, sizeof(int32_t) * Ta},
+        {&ctx->cfail, static_cast<size_t>(std::max(1, P.n_chains)) * Ta}};
+    size_t total = 0;
+    for (const auto &w : want) total += w.second;  // Ta keeps every part a multiple of 2^16 bytes
+    const cudaError_t e = ctx->tile.ensure(total);
+    if (e != cudaSuccess) return e;
+    char *at = ctx->tile.as<char>();
+    for (const auto &w : want) {
+        w.first->p = w.second ? at : nullptr;
+        at += w.second;
+    }
+    return cudaSuccess;
+}
+
+// The steps from the items to the channels over a tile of T points (n of
+// them listed, as far as the host knows) whose nodes and channels are in
+// place: densities, VEGAS weights and, where asked for, bins records or own
+// uniforms (pp_channel_block).
+int pipeline_tile(chili_ctx *ctx, const long long *n_list, long long base, long long T, long long n, int bins,
+                  Densities dens, uint4 *rec_bins, double *x_own) {
+    if (ctx->hints_stale)
+        if (int rc = rebuild_hints(ctx)) return rc;
+    const PointProgram &P = ctx->pp_host;
+    const PointProgram *pp = ctx->point_prog.as<PointProgram>();
+    const double *node = ctx->node_soa.as<double>();
+    double *memo = ctx->memo.as<double>();
+    const unsigned gx = static_cast<unsigned>((T + 255) / 256);
+    if (P.n_tents + P.n_dws + P.n_sws > 0) {
+        KTimer kt_(ctx, KT_ITEMS);
+        if (P.n_tents > 0) {
+            k_pp_items<0><<<dim3(P.n_tents, gx), 256, 0, ctx->stream>>>(pp, node, n_list, base, T, memo);
+            LAUNCHED();
+        }
+        if (P.n_dws > 0) {
+            k_pp_items<1><<<dim3(P.n_dws, gx), 256, 0, ctx->stream>>>(pp, node, n_list, base, T, memo);
+            LAUNCHED();
+        }
+        if (P.n_sws > 0) {
+            k_pp_items<2><<<dim3(P.n_sws, gx), 256, 0, ctx->stream>>>(pp, node, n_list, base, T, memo);
+            LAUNCHED();
+        }
+    }
+    {
+        KTimer kt_(ctx, KT_CHAINS);
+        k_pp_chains<<<dim3(P.n_chains, gx), 256, 0, ctx->stream>>>(pp, node, n_list, base, T, memo,
+                                                                   ctx->cfail.as<uint8_t>());
+    }
+    LAUNCHED();
+    KTimer kt_(ctx, KT_CHANNEL);
+    return launch_channel_dims(ctx, P.ndims, pp, grid_tables(ctx), bins, static_cast<const double *>(memo),
+                               static_cast<const uint8_t *>(ctx->cfail.as<uint8_t>()),
+                               static_cast<const int32_t *>(ctx->ich_tile.as<int32_t>()), n_list, base, T, dens,
+                               ctx->vwv.as<double>(), rec_bins, x_own, ctx->nch, n);
+}
+
+// Tiles of entry points that weight every one of n points (k_pp_given,
+// k_pp_drawn): points per tile, or 0 where the per-thread kernels take the
+// call -- a set without shared program or phased kernels, the option
+// "pipeline" 0, a stream that is being captured (the tile buffers may move
+// later, and the per-thread kernels need none), or no memory for the tile.
+// 2^18 points: 0.4 GB of buffers for the 2->4 set; larger tiles are no
+// faster, smaller ones lose to launch tails.
+long long every_point_tile(chili_ctx *ctx, long long n) {
+    if (!(pipeline_dims_ok(ctx->ndims) && ctx->have_pp && ctx->use_pp && ctx->use_pipeline)) return 0;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return 0;
+    }
+    const long long tiles = (n + (1ll << 18) - 1) >> 18, T = (n + tiles - 1) / tiles;  // tiles of one size
+    if (ctx->every_count.ensure(sizeof(long long)) != cudaSuccess || pipeline_buffers(ctx, T, true) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return T;
+}
+
+}  // namespace
+
 // The phased weight pass (pipeline.cuh) over the n_pre listed points of a
 // momenta buffer of m points (list: their indices, ich: their channels,
 // n_list: the device-side count), in tiles of at most ctx->pipe_tile points
@@ -100,63 +199,21 @@ int launch_channel_dims(chili_ctx *ctx, int dims, A... a) {
 int pipeline_run(chili_ctx *ctx, const double *mom_soa, long long m, const int32_t *list, const int32_t *ich,
                  const long long *n_list, long long n_pre, int bins, bool opt, uint4 *rec_bins, double *rec_dens,
                  const TileFn &combine) {
-    if (ctx->hints_stale)
-        if (int rc = rebuild_hints(ctx)) return rc;
-    const PointProgram &P = ctx->pp_host;
-    const PointProgram *pp = ctx->point_prog.as<PointProgram>();
     // gridDim.y (point blocks of 128) stays below 65536
     const long long T = std::min<long long>(std::min<long long>(ctx->pipe_tile, 65535ll * 128),
                                             std::max<long long>(n_pre, 1));
-    // buffers for a whole number of 2^16 points: the accepted count of a
-    // chunk varies from call to call, and a buffer that grew by a few points
-    // each time would be reallocated (a device synchronisation) each time
-    const long long Ta = (T + 65535) / 65536 * 65536;
-    CK(ctx->node_soa.ensure(sizeof(double) * 4 * P.n_nodes * Ta));
-    CK(ctx->memo.ensure(sizeof(double) * std::max(1, P.n_memo) * Ta));
-    CK(ctx->cfail.ensure(static_cast<size_t>(std::max(1, P.n_chains)) * Ta));
-    if (!rec_dens) CK(ctx->dcv.ensure(sizeof(double) * ctx->nch * Ta));
-    CK(ctx->ich_tile.ensure(sizeof(int32_t) * Ta));
-    CK(ctx->vwv.ensure(sizeof(double) * ctx->nch * Ta));
+    CK(pipeline_buffers(ctx, T, !rec_dens));
     const unsigned gx = static_cast<unsigned>((T + 255) / 256);
-    const int n_items = P.n_tents + P.n_dws + P.n_sws;
-    const int o = opt ? 1 : 0;
     for (long long base = 0; base < n_pre; base += T) {
         // the densities go straight to the records, or to a tile buffer
         const Densities dens = rec_dens ? Densities{rec_dens + base, m} : Densities{ctx->dcv.as<double>(), T};
         { KTimer kt_(ctx, KT_NODES);
-        k_pp_nodes<<<gx, 256, 0, ctx->stream>>>(pp, mom_soa, m, list, ich, n_list, base, ctx->node_soa.as<double>(),
-                                                 ctx->ich_tile.as<int32_t>(), T); }
+        k_pp_nodes<<<gx, 256, 0, ctx->stream>>>(ctx->point_prog.as<PointProgram>(), mom_soa, m, list, ich, n_list, base,
+                                                ctx->node_soa.as<double>(), ctx->ich_tile.as<int32_t>(), T); }
         LAUNCHED();
-        if (n_items > 0) {
-            KTimer kt_(ctx, KT_ITEMS);
-            if (P.n_tents > 0) {
-                k_pp_items<0><<<dim3(P.n_tents, gx), 256, 0, ctx->stream>>>(pp, ctx->node_soa.as<double>(), n_list,
-                                                                             base, T, ctx->memo.as<double>());
-                LAUNCHED();
-            }
-            if (P.n_dws > 0) {
-                k_pp_items<1><<<dim3(P.n_dws, gx), 256, 0, ctx->stream>>>(pp, ctx->node_soa.as<double>(), n_list,
-                                                                           base, T, ctx->memo.as<double>());
-                LAUNCHED();
-            }
-            if (P.n_sws > 0) {
-                k_pp_items<2><<<dim3(P.n_sws, gx), 256, 0, ctx->stream>>>(pp, ctx->node_soa.as<double>(), n_list,
-                                                                           base, T, ctx->memo.as<double>());
-                LAUNCHED();
-            }
-        }
-        { KTimer kt_(ctx, KT_CHAINS);
-        k_pp_chains<<<dim3(P.n_chains, gx), 256, 0, ctx->stream>>>(pp, ctx->node_soa.as<double>(), n_list, base, T,
-                                                                    ctx->memo.as<double>(), ctx->cfail.as<uint8_t>()); }
-        LAUNCHED();
-        {
-            KTimer kt_(ctx, KT_CHANNEL);
-            if (int rc = launch_channel_dims(ctx, P.ndims, pp, grid_tables(ctx), bins, ctx->memo.as<double>(),
-                                             ctx->cfail.as<uint8_t>(), ctx->ich_tile.as<int32_t>(), n_list, base, T, o,
-                                             dens, ctx->vwv.as<double>(), rec_bins, ctx->nch,
-                                             std::min(T, n_pre - base)))
-                return rc;
-        }
+        if (int rc = pipeline_tile(ctx, n_list, base, T, std::min(T, n_pre - base), bins, dens,
+                                   opt ? rec_bins : nullptr, nullptr))
+            return rc;
         if (int rc = combine(base, T, dens)) return rc;
     }
     return CHILI_OK;
@@ -187,7 +244,8 @@ int pp_pass_launch(chili_ctx *ctx, const PPPass &a) {
         LAUNCHED();
     }
     if (int rc = launch_channel_dims(ctx, P.ndims, a.pp, a.tables, a.bins, a.memo, a.cfail, a.ich_tile, a.n_list, 0ll, T,
-                                     1, Densities{a.rec_dens, a.mr}, a.vwv, a.rec_bins, static_cast<int>(P.nch), T))
+                                     Densities{a.rec_dens, a.mr}, a.vwv, a.rec_bins, static_cast<double *>(nullptr),
+                                     static_cast<int>(P.nch), T))
         return rc;
     k_pp_combine<<<gx, 256, 0, ctx->stream>>>(a.pp, a.alpha, Densities{a.rec_dens, a.mr}, a.vwv, a.node_soa, a.n_list, 0, T, a.f,
                                                a.rec_val, a.rec_wgt, a.rec_ok);
@@ -337,10 +395,10 @@ int chili_gpu_destroy(chili_ctx *ctx) {
     if (!ctx) return CHILI_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    DevBuf *bufs[] = {&ctx->edges, &ctx->edges_tmp, &ctx->progs, &ctx->point_prog, &ctx->node_soa, &ctx->memo, &ctx->cfail, &ctx->dcv, &ctx->vwv, &ctx->cells, &ctx->widths, &ctx->ich_tile, &ctx->alpha_buf, &ctx->f_dev, &ctx->mom_soa,
+    DevBuf *bufs[] = {&ctx->edges, &ctx->edges_tmp, &ctx->progs, &ctx->point_prog, &ctx->tile, &ctx->cells, &ctx->widths, &ctx->alpha_buf, &ctx->f_dev, &ctx->mom_soa,
                       &ctx->ich, &ctx->flag, &ctx->list, &ctx->block_count, &ctx->block_off, &ctx->part,
                       &ctx->hist, &ctx->round_res, &ctx->acc, &ctx->ctl, &ctx->status, &ctx->v_part,
-                      &ctx->v_hist, &ctx->v_train, &ctx->v_out, &ctx->rec, &ctx->ctl3, &ctx->unw, &ctx->iter_ctl,
+                      &ctx->v_hist, &ctx->v_train, &ctx->v_out, &ctx->rec, &ctx->ctl3, &ctx->unw, &ctx->iter_ctl, &ctx->every_count,
                       &ctx->mom_soa_alt, &ctx->ich_alt, &ctx->flag_alt, &ctx->block_count_alt,
                       &ctx->v_arrive};
     for (DevBuf *b : bufs) b->release();
@@ -1040,11 +1098,34 @@ int chili_gpu_multichannel_weight(chili_ctx *ctx, const double *mom, const int32
     if ((rc = resolve(ctx, wgt, sizeof(double) * n, 2, false, aw))) return rc;
     if ((rc = resolve(ctx, dens, sizeof(double) * n * ctx->nch, 3, false, ad))) return rc;
     if ((rc = resolve(ctx, x_ich, sizeof(double) * n * ctx->ndims, 4, false, ax))) return rc;
-    k_mc_weight_batch<<<grid_for(n, 128), 128, 0, ctx->stream>>>(
-        ctx->progs.as<ChannelProgram>(), ctx->edges.as<double>(), alpha_ptr(ctx), ctx->nch, ctx->ndims, ctx->bins,
-        ctx->n_ext, static_cast<const double *>(am.dev), static_cast<const int32_t *>(ai.dev),
-        static_cast<double *>(aw.dev), static_cast<double *>(ad.dev), static_cast<double *>(ax.dev), n, pp_ptr(ctx));
-    LAUNCHED();
+    const long long T = every_point_tile(ctx, n);
+    for (long long base = 0; T > 0 && base < n; base += T) {
+        const unsigned gx = static_cast<unsigned>((T + 255) / 256);
+        const Densities dd{ctx->dcv.as<double>(), T};
+        {
+            KTimer kt_(ctx, KT_NODES);
+            k_pp_given<<<gx, 256, 0, ctx->stream>>>(pp_ptr(ctx), static_cast<const double *>(am.dev),
+                                                    static_cast<const int32_t *>(ai.dev), base, n, T,
+                                                    ctx->node_soa.as<double>(), ctx->ich_tile.as<int32_t>(),
+                                                    static_cast<double *>(ax.dev), ctx->every_count.as<long long>());
+            LAUNCHED();
+        }
+        if ((rc = pipeline_tile(ctx, ctx->every_count.as<long long>(), base, T, std::min<long long>(T, n - base), ctx->bins,
+                                dd, nullptr, static_cast<double *>(ax.dev))))
+            return rc;
+        KTimer kt_(ctx, KT_COMBINE);
+        k_pp_weights<<<gx, 256, 0, ctx->stream>>>(pp_ptr(ctx), alpha_ptr(ctx), dd, ctx->vwv.as<double>(),
+                                                  ctx->node_soa.as<double>(), base, n, T, nullptr,
+                                                  static_cast<double *>(ad.dev), static_cast<double *>(aw.dev));
+        LAUNCHED();
+    }
+    if (T == 0) {
+        k_mc_weight_batch<<<grid_for(n, 128), 128, 0, ctx->stream>>>(
+            ctx->progs.as<ChannelProgram>(), ctx->edges.as<double>(), alpha_ptr(ctx), ctx->nch, ctx->ndims, ctx->bins,
+            ctx->n_ext, static_cast<const double *>(am.dev), static_cast<const int32_t *>(ai.dev),
+            static_cast<double *>(aw.dev), static_cast<double *>(ad.dev), static_cast<double *>(ax.dev), n, pp_ptr(ctx));
+        LAUNCHED();
+    }
     if ((rc = finish_out(ctx, aw)) || (rc = finish_out(ctx, ad)) || (rc = finish_out(ctx, ax))) return rc;
     return sync_if_host(ctx, {&am, &ai, &aw, &ad, &ax});
 }
@@ -1426,11 +1507,35 @@ int chili_gpu_generate(chili_ctx *ctx, int64_t n, uint64_t seed, uint64_t counte
     if ((rc = resolve(ctx, mom, sizeof(double) * n * ctx->n_ext * 4, 0, false, am))) return rc;
     if ((rc = resolve(ctx, wgt, sizeof(double) * n, 1, false, aw))) return rc;
     if ((rc = resolve(ctx, ch, sizeof(int32_t) * n, 2, false, ac))) return rc;
-    k_generate<<<grid_for(n, 128), 128, 0, ctx->stream>>>(
-        ctx->progs.as<ChannelProgram>(), ctx->edges.as<double>(), alpha_ptr(ctx), cp_ptr(ctx), ctx->nch, ctx->ndims,
-        ctx->bins, ctx->n_ext, seed, counter_base, n, ctx->f_dev.as<IntegrandDesc>(), static_cast<double *>(am.dev),
-        static_cast<double *>(aw.dev), static_cast<int32_t *>(ac.dev), pp_ptr(ctx));
-    LAUNCHED();
+    const long long T = every_point_tile(ctx, n);
+    for (long long base = 0; T > 0 && base < n; base += T) {
+        const Densities dd{ctx->dcv.as<double>(), T};
+        {
+            KTimer kt_(ctx, KT_FORWARD);
+            k_pp_drawn<<<static_cast<unsigned>((T + kFwdBlock - 1) / kFwdBlock), kFwdBlock, 0, ctx->stream>>>(
+                pp_ptr(ctx), ctx->progs.as<ChannelProgram>(), ctx->edges.as<double>(), cp_ptr(ctx), ctx->ndims,
+                ctx->bins, seed, counter_base, base, n, T, wgt ? ctx->node_soa.as<double>() : nullptr,
+                ctx->ich_tile.as<int32_t>(), static_cast<double *>(am.dev), static_cast<int32_t *>(ac.dev),
+                ctx->every_count.as<long long>());
+            LAUNCHED();
+        }
+        if (!wgt) continue;
+        if ((rc = pipeline_tile(ctx, ctx->every_count.as<long long>(), base, T, std::min<long long>(T, n - base), ctx->bins,
+                                dd, nullptr, nullptr)))
+            return rc;
+        KTimer kt_(ctx, KT_COMBINE);
+        k_pp_weights<<<static_cast<unsigned>((T + 255) / 256), 256, 0, ctx->stream>>>(
+            pp_ptr(ctx), alpha_ptr(ctx), dd, ctx->vwv.as<double>(), ctx->node_soa.as<double>(), base, n, T,
+            ctx->f_dev.as<IntegrandDesc>(), nullptr, static_cast<double *>(aw.dev));
+        LAUNCHED();
+    }
+    if (T == 0) {
+        k_generate<<<grid_for(n, 128), 128, 0, ctx->stream>>>(
+            ctx->progs.as<ChannelProgram>(), ctx->edges.as<double>(), alpha_ptr(ctx), cp_ptr(ctx), ctx->nch, ctx->ndims,
+            ctx->bins, ctx->n_ext, seed, counter_base, n, ctx->f_dev.as<IntegrandDesc>(), static_cast<double *>(am.dev),
+            static_cast<double *>(aw.dev), static_cast<int32_t *>(ac.dev), pp_ptr(ctx));
+        LAUNCHED();
+    }
     if ((rc = finish_out(ctx, am)) || (rc = finish_out(ctx, aw)) || (rc = finish_out(ctx, ac))) return rc;
     return sync_if_host(ctx, {&am, &aw, &ac});
 }

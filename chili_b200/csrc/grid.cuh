@@ -169,10 +169,13 @@ __device__ __forceinline__ int cell_count(const uint32_t *__restrict__ entries, 
 template <bool TABLE_NC, int F>
 __device__ __forceinline__ int cell_count_slow(const double *__restrict__ e, const uint32_t *__restrict__ entries,
                                                int bins, int cells, double scale, double x) {
-    if (!(x >= 0.0 && x < 1.0)) return find_bin<true>(e, bins, x) + 1;
-    const uint32_t lo = static_cast<uint32_t>(__double2loint(__fma_rd(x, scale, 0x1p52)));
+    // outside [0, 1) (points outside a channel's region, uncut events): any
+    // cell tells whether the row is monotone inside it
+    const bool in = x >= 0.0 && x < 1.0;
+    const uint32_t lo = in ? static_cast<uint32_t>(__double2loint(__fma_rd(x, scale, 0x1p52))) : 0u;
     int k = static_cast<int>(tab_ld<TABLE_NC>(entries + ((lo >> F) & (cells - 1))) >> (2 * F + 2));
     if (k == static_cast<int>(0xffffffffu >> (2 * F + 2))) return find_bin<true>(e, bins, x) + 1;
+    if (!in) return x >= 1.0 ? bins : 0;
     for (;;) {
         int n = 0;
 #pragma unroll

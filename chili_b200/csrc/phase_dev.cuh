@@ -25,8 +25,17 @@ __device__ __forceinline__ void store_v4(double *__restrict__ soa, int node, lon
     soa[(4 * node + 3) * m + i] = v.z;
 }
 
+// The compound nodes of tile point i, summed as the reference's tmp_mom, its
+// external nodes being stored.
+__device__ __forceinline__ void pp_compounds(const PointProgram *__restrict__ pp, double *__restrict__ node_soa,
+                                             long long m, long long i) {
+    const int ne = pp->n_ext, nn = pp->n_nodes;
+    for (int s = ne; s < nn; ++s)
+        store_v4(node_soa, s, m, i, load_v4(node_soa, pp->node_a[s], m, i) + load_v4(node_soa, pp->node_b[s], m, i));
+}
+
 // Nodes of point i = list[i]: externals copied from the chunk's momenta
-// (mom_soa, stride mc), compounds summed as the reference's tmp_mom.
+// (mom_soa, stride mc), then the compounds.
 __device__ __forceinline__ void pp_nodes_block(const PointProgram *__restrict__ pp, const double *__restrict__ mom_soa,
                                                long long mc, const int32_t *__restrict__ list,
                                                const int32_t *__restrict__ ich_arr,
@@ -37,10 +46,8 @@ __device__ __forceinline__ void pp_nodes_block(const PointProgram *__restrict__ 
     if (i >= m || base + i >= *n_list) return;
     const long long k = list[base + i];
     ich_tile[i] = ich_arr[k];
-    const int ne = pp->n_ext, nn = pp->n_nodes;
-    for (int s = 0; s < ne; ++s) store_v4(node_soa, s, m, i, load_v4(mom_soa, s, mc, k));
-    for (int s = ne; s < nn; ++s)
-        store_v4(node_soa, s, m, i, load_v4(node_soa, pp->node_a[s], m, i) + load_v4(node_soa, pp->node_b[s], m, i));
+    for (int s = 0; s < pp->n_ext; ++s) store_v4(node_soa, s, m, i, load_v4(mom_soa, s, mc, k));
+    pp_compounds(pp, node_soa, m, i);
 }
 
 // One thread per (point, item): items 0..n_tents-1 are t-channel entries
@@ -195,17 +202,16 @@ struct Densities {
     long long stride;
 };
 
-__device__ __forceinline__ void pp_combine_point(const PointProgram *__restrict__ pp, const double *__restrict__ alpha,
-                                                 Densities dens, const double *__restrict__ vwv,
-                                                 const double *__restrict__ node_soa, long long m, long long i,
-                                                 long long r, const IntegrandDesc *__restrict__ f,
-                                                 double *__restrict__ rec_val, double *__restrict__ rec_wgt,
-                                                 uint8_t *__restrict__ rec_ok) {
-    double acc = 0.0;
-    const int nch = pp->nch;
-    // eight channels' values in flight before the first division: one at a
-    // time, the divisions' slow-path branches kept the next loads back
+// 1 / sum_c alpha_c / dens_c / vw_c at tile point i in channel order
+// (Integrand.hh:118-122).  Eight channels' values are in flight before the
+// first division: one at a time, the divisions' slow-path branches kept the
+// next loads back (0.151 against 0.097 ms per 1e6 points of 15 channels).
+// dens_row: the point's densities in channel order, where asked for.
+__device__ __forceinline__ double pp_weight_sum(int nch, const double *__restrict__ alpha, Densities dens,
+                                                const double *__restrict__ vwv, long long m, long long i,
+                                                double *__restrict__ dens_row = nullptr) {
     const double *dp = dens.p + i, *vp = vwv + i;
+    double acc = 0.0;
     for (int c0 = 0; c0 < nch; c0 += 8) {
         double d[8], v[8];
 #pragma unroll
@@ -216,9 +222,21 @@ __device__ __forceinline__ void pp_combine_point(const PointProgram *__restrict_
         }
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            if (c0 + k < nch) acc += __ldg(alpha + c0 + k) / d[k] / v[k];
+            if (c0 + k < nch) {
+                acc += __ldg(alpha + c0 + k) / d[k] / v[k];
+                if (dens_row) dens_row[c0 + k] = d[k];
+            }
     }
-    double wgt = 1.0 / acc;
+    return 1.0 / acc;
+}
+
+__device__ __forceinline__ void pp_combine_point(const PointProgram *__restrict__ pp, const double *__restrict__ alpha,
+                                                 Densities dens, const double *__restrict__ vwv,
+                                                 const double *__restrict__ node_soa, long long m, long long i,
+                                                 long long r, const IntegrandDesc *__restrict__ f,
+                                                 double *__restrict__ rec_val, double *__restrict__ rec_wgt,
+                                                 uint8_t *__restrict__ rec_ok) {
+    double wgt = pp_weight_sum(pp->nch, alpha, dens, vwv, m, i);
     const double fv = eval_momenta_soa(f, node_soa, m, i, pp->n_ext);
     double val = wgt == 0 ? 0 : fv * wgt;
     uint8_t ok = 1;
@@ -258,7 +276,9 @@ __device__ __forceinline__ void copy_async_wait() {
 // The channel step of one block: channel c's density (the product of its
 // items in the reference's order, Channel.cc:40-61) and its VEGAS weight at
 // the tile points [i0, i1) on the uniforms that the position map selects, the
-// density record and, for the point's own channel, its bins record.  When c's
+// density and, for the point's own channel, its bins record (REC: own_out is
+// uint4 rows, mc_device.cuh) or its uniforms (own_out, [point][DIMS], may be
+// null).  When c's
 // chain fails, its last uniform is the one the shared buffer still holds: the
 // last uniform of the latest earlier channel whose chain did not fail (zero
 // if none).  TAB: channel c's entries and widths are staged in shared memory
@@ -268,13 +288,12 @@ __device__ __forceinline__ void copy_async_wait() {
 // afterwards: 0.7% of them on trained 200-bin grids, but some lane of a warp
 // in every fifth search), then the widths multiplied in the reference's
 // order.  smem: channel_smem_bytes.
-template <int DIMS, bool TAB, int F>
+template <int DIMS, bool TAB, int F, bool REC>
 __device__ __forceinline__ void pp_channel_block(const PointProgram *__restrict__ pp, const GridTables &T, int bins,
                                                  const double *__restrict__ memo, const uint8_t *__restrict__ cfail,
-                                                 const int32_t *__restrict__ ich_tile, long long m, int should_opt,
-                                                 Densities dens, double *__restrict__ vwv,
-                                                 uint4 *__restrict__ rec_bins, long long base, long long i0,
-                                                 long long i1, int c, void *smem) {
+                                                 const int32_t *__restrict__ ich_tile, long long m, Densities dens,
+                                                 double *__restrict__ vwv, void *__restrict__ own_out, long long base,
+                                                 long long i0, long long i1, int c, void *smem) {
     const int cells = grid_cells(bins);
     const double scale = static_cast<double>(cells) * static_cast<double>(1 << F);
     int32_t *pos_s = static_cast<int32_t *>(smem);  // [2][DIMS]: chain found, chain failed
@@ -343,7 +362,7 @@ __device__ __forceinline__ void pp_channel_block(const PointProgram *__restrict_
         double fv[kFacAhead], wdec = 1, sw = 1;
 #pragma unroll
         for (int k = 0; k < kFacAhead; ++k) fv[k] = at(fac_s[min(k, n_fac)]);
-        const int own = should_opt ? ich_tile[i] : -1;
+        const bool own = (REC || own_out) && ich_tile[i] == c;
 #pragma unroll
         for (int k = 0; k < kFacAhead; ++k) {
             if (k < n_dec) wdec *= fv[k];
@@ -354,6 +373,11 @@ __device__ __forceinline__ void pp_channel_block(const PointProgram *__restrict_
             else sw *= at(fac_s[k]);
         }
         const double dc = wdec * wt * sw;
+        if (!REC && own) {
+            double *o = static_cast<double *>(own_out) + (base + i) * DIMS;
+#pragma unroll
+            for (int p = 0; p < DIMS; ++p) o[p] = x[p];
+        }
         uint32_t rec[NW], todo = 0;
 #pragma unroll
         for (int k = 0; k < NW; ++k) rec[k] = 0;
@@ -385,9 +409,9 @@ __device__ __forceinline__ void pp_channel_block(const PointProgram *__restrict_
         }
         dens_c[i] = dc;
         vw_c[i] = vw;
-        if (c == own) {
+        if (REC && own) {
             rec[DIMS >> 1] |= static_cast<uint32_t>(c) << (16 * (DIMS & 1));
-            uint4 *o = rec_bins + (base + i) * (NW / 4);
+            uint4 *o = static_cast<uint4 *>(own_out) + (base + i) * (NW / 4);
 #pragma unroll
             for (int k = 0; k < NW / 4; ++k) o[k] = make_uint4(rec[4 * k], rec[4 * k + 1], rec[4 * k + 2], rec[4 * k + 3]);
         }

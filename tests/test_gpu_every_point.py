@@ -1,0 +1,67 @@
+"""Entry points that weight every point of a call (Integrand::GenerateWeight,
+Integrand.hh:112-123; MultiChannel::GeneratePoint/GenerateWeight,
+MultiChannel.hh:141-165): the tiled phased pass against the kernel that runs
+one point per thread, at sizes around a block and around a tile."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from chili_b200 import abi, channels, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def _context(make, n_out, pipeline):
+    cs = workloads.channel_set(n_out)
+    ctx = make()
+    ctx.set_channels(cs)
+    ctx.set_option("pipeline", pipeline)
+    rng = np.random.default_rng(5)
+    e = np.sort(rng.random((cs.nch, ctx.ndims, 19)) ** 1.5, axis=2)
+    ctx.set_grids(np.concatenate([np.zeros(e.shape[:2] + (1,)), e, np.ones(e.shape[:2] + (1,))], 2))
+    ctx.set_integrand(abi.CHILI_FUNC_PROPAGATOR, channels.propagator_params())
+    a = rng.random(cs.nch) + 0.1
+    ctx.set_alpha(a / a.sum())
+    return ctx
+
+
+def _close(got, want):
+    """The same operations on the same inputs, except that a channel of two
+    decays divides by 2 pi in another order: one rounding per factor, amplified
+    where the channels' signed densities cancel (a median bar and equal
+    non-finite patterns)."""
+    assert np.array_equal(np.isfinite(got), np.isfinite(want))
+    ok = np.isfinite(want)
+    err = np.abs(got[ok] - want[ok]) / np.maximum(np.abs(want[ok]), 1e-300)
+    assert np.percentile(err, 99) <= 1e-14 if err.size else True
+
+
+@pytest.mark.parametrize("n_out,n", [(2, 1), (4, 255), (4, 257), (6, 1001), (4, 262145)])
+def test_tiled_weights_and_events_match_per_thread(ctx_factory, n_out, n):
+    ctxs = [_context(ctx_factory, n_out, p) for p in (0, 1)]
+    events = [c.generate(n, seed=11, counter=3) for c in ctxs]
+    assert np.array_equal(events[0][0], events[1][0], equal_nan=True)
+    assert np.array_equal(events[0][2], events[1][2])
+    _close(events[1][1], events[0][1])
+    mom, _, ich = events[0]
+    ich = ich.copy()
+    ich[n // 2] = -1  # no channel's uniforms: zeros
+    got = [c.multichannel_weight(mom, ich) for c in ctxs]
+    _close(got[1][0], got[0][0])
+    _close(got[1][1], got[0][1])
+    assert np.array_equal(got[1][2], got[0][2], equal_nan=True)
+    assert not got[1][2][n // 2].any()
+
+
+def test_outputs_are_optional(ctx_factory):
+    ctx = _context(ctx_factory, 4, 1)
+    mom, w, ch = ctx.generate(300, seed=2)
+    only = np.empty_like(mom)
+    ctx.call("chili_gpu_generate", 300, 2, 0, C.c_void_p(only.ctypes.data), None, None)
+    assert np.array_equal(only, mom, equal_nan=True)
+    full, _, _ = ctx.multichannel_weight(mom, ch)
+    alone = np.empty(300)
+    ctx.call("chili_gpu_multichannel_weight", C.c_void_p(mom.ctypes.data), C.c_void_p(ch.ctypes.data),
+             C.c_void_p(alone.ctypes.data), None, None, 300)
+    assert np.array_equal(alone, full, equal_nan=True)
