@@ -366,14 +366,19 @@ __device__ __forceinline__ void bt_accum_block(const BatchDev &B, int ti, long l
     }
     const unsigned any = __ballot_sync(0xffffffffu, vw != 0);
     if (any) {
-        for (int c = 0; c < T.nch; ++c) {
-            double term = 0.0;
-            if (vw != 0) {  // only the records' own lanes read their densities
-                term = vw / rec_dens[c * mr + r];
-                if (!isfinite(term)) term = 0.0;  // non-finite terms dropped
+        for (int c0 = 0; c0 < T.nch; c0 += 8) {
+            double term[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)  // only the records' own lanes read their densities
+                term[q] = vw != 0 ? rec_dens[min(c0 + q, T.nch - 1) * mr + r] : 1.0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                term[q] = vw != 0 ? vw / term[q] : 0.0;
+                if (!isfinite(term[q])) term[q] = 0.0;  // non-finite terms dropped
             }
-            term = warp_sum(term);
-            if (lane == 0 && term != 0) atomicAdd(s_atr + c, term);
+            int q;
+            const double sum8 = warp_sum8(term, q);
+            if ((lane & 3) == 0 && c0 + q < T.nch && sum8 != 0) atomicAdd(s_atr + c0 + q, sum8);
         }
     }
     // StatsData over the unit's active points: the records, and value-0
@@ -634,10 +639,10 @@ __global__ void __launch_bounds__(kFoldThreads) k_batch_finalize(BatchDev B, int
         double *o = B.stats + (slot * B.ntasks + ti) * 6;
         // retry tasks: the StatsData that k_rt_end folded round by round
         for (int k = 0; k < 6; ++k) o[k] = T.retry ? B.retry[ti].acc[k] : sh[k][0];
-        if (adapt && T.kind == CHILI_TASK_MULTICHANNEL)
-            alpha_update(B.alpha + T.ch_off, B.best + T.ch_off, B.mindiff + ti, B.cp + T.ch_off,
-                         B.atrain + T.ch_off, T.nch, T.beta, T.min_alpha, 1);
     }
+    if (adapt && T.kind == CHILI_TASK_MULTICHANNEL)
+        alpha_update(B.alpha + T.ch_off, B.best + T.ch_off, B.mindiff + ti, B.cp + T.ch_off, B.atrain + T.ch_off, T.nch,
+                     T.beta, T.min_alpha, 1);
 }
 
 // Retry loop: the state of every retry task at the start of an iteration
@@ -1193,7 +1198,10 @@ int enqueue_final(chili_ctx *ctx, bool adapt) {
     k_batch_finalize<<<static_cast<unsigned>(S.tasks.size()), kFoldThreads, 0, ctx->stream>>>(B, adapt ? 1 : 0);
     LAUNCHED();
     if (adapt && !S.jobs.empty()) {
-        k_batch_adapt<<<static_cast<unsigned>(S.jobs.size()), 32, sizeof(double) * S.max_bins, ctx->stream>>>(
+        const size_t scratch = adapt_scratch_bytes(S.max_bins);
+        if (scratch > 48 * 1024)
+            CK(cudaFuncSetAttribute(k_batch_adapt, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scratch)));
+        k_batch_adapt<<<static_cast<unsigned>(S.jobs.size()), 64, scratch, ctx->stream>>>(
             B, S.d_jobs.as<AdaptJob>(), static_cast<int>(S.jobs.size()), S.d_status.as<int>());
         LAUNCHED();
         k_batch_commit<<<static_cast<unsigned>(S.jobs.size()), 128, 0, ctx->stream>>>(

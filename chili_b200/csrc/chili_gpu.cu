@@ -274,6 +274,10 @@ namespace {
 // of this one.
 constexpr long long kFirstSlice = 1ll << 16;   // rows, a multiple of kFwdBlock
 
+// Rounds of more points than this size their weight pass by the accepted
+// count, read back from the device.
+constexpr long long kReadBack = 1ll << 16;
+
 // Slice boundaries of a chunk of m rows: slices that double from kFirstSlice
 // rows up to `top` rows (option "upload_slice", default kUploadSlice).
 std::vector<long long> slice_bounds(long long m, long long top) {
@@ -341,8 +345,9 @@ int rebuild_hints(chili_ctx *ctx) {
     const size_t rows = static_cast<size_t>(ctx->g_nch) * ctx->dims;
     CK(ctx->cells.ensure(sizeof(uint32_t) * rows * grid_cells(ctx->bins)));
     CK(ctx->widths.ensure(sizeof(double) * rows * width_row(ctx->bins)));
-    k_build_cells<<<dim3(ctx->dims, ctx->g_nch), 128, 0, ctx->stream>>>(
-        ctx->edges.as<double>(), ctx->dims, ctx->bins, ctx->cells.as<uint32_t>(), ctx->widths.as<double>());
+    k_build_cells<<<dim3(ctx->dims, ctx->g_nch), 256, 0, ctx->stream>>>(
+        ctx->edges.as<double>(), ctx->dims, ctx->bins, ctx->cells.as<uint32_t>(), ctx->widths.as<double>(),
+        TrainGate{});
     LAUNCHED();
     return CHILI_OK;
 }
@@ -374,8 +379,10 @@ int chili_gpu_create(int device, chili_ctx **out) {
     }
     ctx->own_stream = true;
     if (cudaMallocHost(reinterpret_cast<void **>(&ctx->ctl_host), 2 * sizeof(RoundCtl)) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void **>(&ctx->iter_host), sizeof(long long) * kIterCtl) != cudaSuccess) {
+        cudaMallocHost(reinterpret_cast<void **>(&ctx->iter_host), sizeof(long long) * kIterCtl) != cudaSuccess ||
+        cudaMallocHost(reinterpret_cast<void **>(&ctx->acc_host), sizeof(IterAcc)) != cudaSuccess) {
         if (ctx->ctl_host) cudaFreeHost(ctx->ctl_host);
+        if (ctx->iter_host) cudaFreeHost(ctx->iter_host);
         cudaStreamDestroy(ctx->stream);
         delete ctx;
         return fail(nullptr, CHILI_ERR_CUDA, "cudaMallocHost failed");
@@ -407,6 +414,7 @@ int chili_gpu_destroy(chili_ctx *ctx) {
     for (auto &b : ctx->stage) b.release();
     if (ctx->ctl_host) cudaFreeHost(ctx->ctl_host);
     if (ctx->iter_host) cudaFreeHost(ctx->iter_host);
+    if (ctx->acc_host) cudaFreeHost(ctx->acc_host);
     collect_times(ctx);
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->copy_events) cudaEventDestroy(e);
@@ -657,12 +665,32 @@ static int adapt_grids(chili_ctx *ctx, int first, int count, double alpha, const
         CK(cudaMemcpyAsync(ctx->edges_tmp.p, ctx->edges.p, sizeof(double) * gsz * ctx->g_nch,
                            cudaMemcpyDeviceToDevice, ctx->stream));
     dim3 grid(D, count);
-    k_grid_adapt<<<grid, 32, sizeof(double) * B, ctx->stream>>>(
+    k_grid_adapt<<<grid, 128, adapt_scratch_bytes(B), ctx->stream>>>(
         ctx->edges.as<double>() + first * gsz, ctx->edges_tmp.as<double>() + first * gsz, D, B, alpha, train_dev,
-        skip_zero, ctx->status.as<int>());
+        skip_zero, ctx->status.as<int>(), TrainGate{});
     LAUNCHED();
     std::swap(ctx->edges, ctx->edges_tmp);
     return rebuild_hints(ctx);
+}
+
+// MultiChannel::Train (MultiChannel.hh:182-194) of an iteration, queued
+// behind its round: channel weights, every grid into edges_tmp and the search
+// tables of the new edges, all skipped on the device when the gate is closed.
+// The caller swaps the edge buffers once it knows that the gate was open.
+static int queue_training(chili_ctx *ctx, const chili_multichannel_params *params, TrainGate gate) {
+    const int D = ctx->dims, B = ctx->bins;
+    KTimer kt_(ctx, KT_ITER_END);
+    k_alpha_update<<<1, 256, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx),
+                                               acc_train_ptr(ctx), ctx->nch, params->beta, params->min_alpha, 1, gate);
+    LAUNCHED();
+    k_grid_adapt<<<dim3(D, ctx->g_nch), 128, adapt_scratch_bytes(B), ctx->stream>>>(
+        ctx->edges.as<double>(), ctx->edges_tmp.as<double>(), D, B, params->grid_alpha, ctx->hist.as<double>(), 1,
+        ctx->status.as<int>(), gate);
+    LAUNCHED();
+    k_build_cells<<<dim3(D, ctx->g_nch), 256, 0, ctx->stream>>>(ctx->edges_tmp.as<double>(), D, B,
+                                                                ctx->cells.as<uint32_t>(), ctx->widths.as<double>(), gate);
+    LAUNCHED();
+    return CHILI_OK;
 }
 
 int chili_gpu_grid_adapt(chili_ctx *ctx, int ch, double alpha, const double *train) {
@@ -773,6 +801,7 @@ int chili_gpu_vegas_iterate(chili_ctx *ctx, uint64_t ncalls, uint64_t seed, uint
     const bool smem = hist_bytes <= 48 * 1024;
     if (smem && adapt && ctx->vegas_fused && ctx->g_nch == 1 &&
         sizeof(double) * B * (kVegasBlock / 32) <= 48 * 1024) {
+        const size_t step_smem = std::max(hist_bytes, adapt_scratch_bytes(B) * (kVegasBlock / 32));
         // the whole iteration in one launch (k_vegas_step): points, a
         // two-level ordered fold and the adaptation
         const long long nb = std::min<long long>(grid_for(n, kVegasBlock), static_cast<long long>(sms) * 4);
@@ -804,8 +833,9 @@ int chili_gpu_vegas_iterate(chili_ctx *ctx, uint64_t ncalls, uint64_t seed, uint
         double *out_dev = stats_out ? static_cast<double *>(ast.dev) : ctx->v_out.as<double>();
         {
             KTimer kt_(ctx, KT_VEGAS_STEP);
-            kern<<<static_cast<unsigned>(nb), kVegasBlock,
-                   std::max(hist_bytes, sizeof(double) * B * (kVegasBlock / 32)), ctx->stream>>>(
+            if (step_smem > 48 * 1024)
+                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(step_smem)));
+            kern<<<static_cast<unsigned>(nb), kVegasBlock, step_smem, ctx->stream>>>(
                 ctx->edges.as<double>(), ctx->edges_tmp.as<double>(), D, B, seed, counter_base,
                 static_cast<const double *>(au.dev), n, ctx->f_dev.as<IntegrandDesc>(), ctx->v_part.as<double>(),
                 ctx->v_hist.as<double>(), ctx->v_part.as<double>() + 6 * nb, ctx->v_hist.as<double>() + nh * nb,
@@ -953,8 +983,8 @@ int chili_gpu_set_channels(chili_ctx *ctx, const chili_channel_desc *descs, int 
     a[3 * CHILI_MAX_CHANNELS] = INFINITY;
     CK(ctx->alpha_buf.ensure(sizeof(double) * a.size()));
     CK(cudaMemcpyAsync(ctx->alpha_buf.p, a.data(), sizeof(double) * a.size(), cudaMemcpyHostToDevice, ctx->stream));
-    k_alpha_update<<<1, 32, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx), nullptr,
-                                              nch, 0.0, 0.0, 0);
+    k_alpha_update<<<1, 256, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx), nullptr,
+                                              nch, 0.0, 0.0, 0, TrainGate{});
     LAUNCHED();
     ctx->alpha_set = true;
     // best_weights start empty in the reference; they read back as NaN until
@@ -1039,8 +1069,8 @@ int chili_gpu_set_alpha(chili_ctx *ctx, const double *alpha, int nch) {
     Arg a;
     if ((rc = resolve(ctx, alpha, sizeof(double) * nch, 0, true, a))) return rc;
     CK(cudaMemcpyAsync(alpha_ptr(ctx), a.dev, sizeof(double) * nch, cudaMemcpyDeviceToDevice, ctx->stream));
-    k_alpha_update<<<1, 32, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx), nullptr,
-                                              nch, 0.0, 0.0, 0);
+    k_alpha_update<<<1, 256, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx), nullptr,
+                                              nch, 0.0, 0.0, 0, TrainGate{});
     LAUNCHED();
     CK(cudaStreamSynchronize(ctx->stream));
     return CHILI_OK;
@@ -1154,13 +1184,10 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
     CK(ctx->acc.ensure(sizeof(IterAcc)));
     CK(ctx->ctl.ensure(sizeof(RoundCtl)));
     CK(ctx->round_res.ensure(sizeof(double) * (kPartFixed + nch)));
-    CK(cudaMemsetAsync(ctx->hist.p, 0, sizeof(double) * hist_n, ctx->stream));
-    {
-        IterAcc a0{};
-        a0.st[1] = 1.7976931348623157e308;  // StatsData min = lim::max()
-        a0.st[2] = 2.2250738585072014e-308; // StatsData max = lim::min()
-        CK(cudaMemcpyAsync(ctx->acc.p, &a0, sizeof(IterAcc), cudaMemcpyHostToDevice, ctx->stream));
-    }
+    CK(ctx->status.ensure(sizeof(int)));
+    k_mc_begin<<<static_cast<unsigned>(std::min<size_t>(ctx->sms, (hist_n + 255) / 256)), 256, 0, ctx->stream>>>(
+        ctx->hist.as<double>(), static_cast<long long>(hist_n), ctx->acc.as<IterAcc>(), ctx->status.as<int>());
+    LAUNCHED();
     const size_t acc_smem = sizeof(double) * (kWgtBlock / 32) * nch;
     // the histogram adds staged in shared memory when one block can hold the
     // whole histogram (option "hist_shared")
@@ -1294,11 +1321,13 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
             if (pipe) {
                 // the launches are sized by the accepted count, read back here;
                 // a queued host-uniform round (or any round with the option
-                // "pipeline_sync" 0) does not wait for it: its launches cover
+                // "pipeline_sync" 0, or of few points, where the read back
+                // takes longer than the empty blocks that it saves) does not
+                // wait for it: its launches cover
                 // all mm points and the threads past the device-side count
                 // return at once
                 long long n_pre = mm;
-                if ((!u_host && ctx->pipe_sync) || mm > ctx->pipe_tile) {
+                if ((!u_host && ctx->pipe_sync && mm > kReadBack) || mm > ctx->pipe_tile) {
                     CK(cudaMemcpyAsync(ctx->ctl_host, ctl_pre, sizeof(RoundCtl), cudaMemcpyDeviceToHost,
                                        ctx->stream));
                     CK(cudaStreamSynchronize(ctx->stream));
@@ -1321,11 +1350,9 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
                 KTimer kt_(ctx, KT_ROUND_OTHER);
                 k_block_count<<<static_cast<unsigned>(nbf), kFwdBlock, 0, ctx->stream>>>(rec_ok, ctl_pre, bcount);
                 LAUNCHED();
-                k_mc_scan<<<1, 1024, 0, ctx->stream>>>(bcount, static_cast<int>(nbf), rec_ok, mm, needed, gate, 1,
-                                                       ctx->block_off.as<long long>(), ctl_list);
-                LAUNCHED();
-                k_cut_finalize<<<1, 1, 0, ctx->stream>>>(ctl_list, ctl_pre, ctx->list.as<int32_t>(), mm, needed,
-                                                         u_host ? iter : nullptr, ctx->ctl.as<RoundCtl>());
+                k_mc_cut<<<1, 1024, 0, ctx->stream>>>(bcount, static_cast<int>(nbf), rec_ok, mm, needed,
+                                                      u_host ? iter : nullptr, ctx->block_off.as<long long>(), ctl_list,
+                                                      ctl_pre, ctx->list.as<int32_t>(), ctx->ctl.as<RoundCtl>());
                 LAUNCHED();
             }
             {
@@ -1357,11 +1384,24 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
                 CK(cudaEventRecord(ctx->round_done[par], ctx->stream));
                 continue;
             }
+            // the training of the iteration runs on behind the round, before
+            // the host knows whether the round completed the iteration
+            const bool train = opt && !ctx->defer_train &&
+                               rounds + static_cast<unsigned long long>(n_rounds) <=
+                                   static_cast<unsigned long long>(ctx->max_rounds);
+            if (train)
+                if ((rc = queue_training(ctx, params, TrainGate{ctx->ctl.as<RoundCtl>(), needed}))) return rc;
             CK(cudaMemcpyAsync(ctx->ctl_host, ctx->ctl.p, sizeof(RoundCtl), cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaMemcpyAsync(ctx->ctl_host + 1, ctl_pre, sizeof(RoundCtl), cudaMemcpyDeviceToHost, ctx->stream));
+            CK(cudaMemcpyAsync(ctx->acc_host, ctx->acc.p, sizeof(IterAcc), cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
             if (ctx->timing) collect_times(ctx);
             const RoundCtl r = ctx->ctl_host[0];
+            const bool trained = train && r.n_acc - r.nan_round >= needed;
+            if (trained) {
+                std::swap(ctx->edges, ctx->edges_tmp);
+                ctx->hints_stale = false;  // queue_training built the new grids' tables
+            }
             if (r.cut <= 0 || r.cut > mm || r.n_acc < 0 || r.nan_round < 0 || r.nan_round > r.n_acc)
                 return fail(ctx, CHILI_ERR_CUDA, "inconsistent round record");
             tried += r.cut;
@@ -1390,17 +1430,16 @@ int chili_gpu_multichannel_iterate(chili_ctx *ctx, const chili_multichannel_para
         if (rounds > static_cast<unsigned long long>(ctx->max_rounds))
             return fail(ctx, CHILI_ERR_TIMEOUT, "ncalls not reached after max_rounds rounds (every point rejected or NaN?)");
     }
-    IterAcc acc_h;
-    if (opt && !ctx->defer_train) {
-        KTimer kt_(ctx, KT_ITER_END);
-        k_alpha_update<<<1, 32, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx),
-                                                  acc_train_ptr(ctx), nch, params->beta,
-                                                  params->min_alpha, 1);
-        LAUNCHED();
-        if ((rc = adapt_grids(ctx, 0, nch, params->grid_alpha, ctx->hist.as<double>(), 1))) return rc;
+    if (u_host) {  // host uniforms: the queued rounds' host read came before the training
+        if (opt && !ctx->defer_train) {
+            if ((rc = queue_training(ctx, params, TrainGate{}))) return rc;
+            std::swap(ctx->edges, ctx->edges_tmp);
+            ctx->hints_stale = false;
+        }
+        CK(cudaMemcpyAsync(ctx->acc_host, ctx->acc.p, sizeof(IterAcc), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
     }
-    CK(cudaMemcpyAsync(&acc_h, ctx->acc.p, sizeof(IterAcc), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    const IterAcc &acc_h = *ctx->acc_host;
     if (stats_out) std::memcpy(stats_out, acc_h.st, sizeof(chili_stats));
     if (info) {
         info->points_tried = static_cast<uint64_t>(tried);
@@ -1431,8 +1470,8 @@ int chili_gpu_multichannel_train(chili_ctx *ctx, const chili_multichannel_params
     if ((rc = resolve(ctx, alpha_train, sizeof(double) * nch, 1, true, aa))) return rc;
     CK(cudaMemcpyAsync(ctx->hist.p, ah.dev, sizeof(double) * hist_n, cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaMemcpyAsync(acc_train_ptr(ctx), aa.dev, sizeof(double) * nch, cudaMemcpyDeviceToDevice, ctx->stream));
-    k_alpha_update<<<1, 32, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx),
-                                              acc_train_ptr(ctx), nch, params->beta, params->min_alpha, 1);
+    k_alpha_update<<<1, 256, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx),
+                                              acc_train_ptr(ctx), nch, params->beta, params->min_alpha, 1, TrainGate{});
     LAUNCHED();
     if ((rc = adapt_grids(ctx, 0, nch, params->grid_alpha, ctx->hist.as<double>(), 1))) return rc;
     // host inputs were staged: their buffers are free once the copies ran

@@ -170,6 +170,7 @@ struct chili_ctx {
     cudaEvent_t fwd_done[2] = {nullptr, nullptr}, round_done[2] = {nullptr, nullptr};
     RoundCtl *ctl_host = nullptr;  // pinned, two records: the round, the PreProcess count
     long long *iter_host = nullptr;  // pinned, the queued rounds' state (k_iter_init)
+    IterAcc *acc_host = nullptr;     // pinned, the iteration's accumulator
     DevBuf iter_ctl;                 // device copy of that state
     double accept_rate = 0.5, nan_rate = 0.0;
     DevBuf rec, ctl3;

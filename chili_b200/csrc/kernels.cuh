@@ -14,7 +14,7 @@
 //   k_mc_compact   ordered list of the PreProcess-accepted points
 //   k_mc_weight    every channel's inverse map + grid weight -> combined
 //                  weight and integrand, as per-point records
-//   k_block_count, k_mc_scan, k_cut_finalize
+//   k_block_count, k_mc_cut
 //                  the cut: the `needed`-th point whose value is not NaN
 //                  (NaN values are retried, MultiChannel.hh:230-236)
 //   k_mc_accum     StatsData, channel histograms and alpha training over the
@@ -31,11 +31,36 @@
 
 namespace chili_dev {
 
+// Training steps queued behind a round whose outcome the host has not read:
+// they do nothing when the round left the iteration short of its points.
+struct TrainGate {
+    const RoundCtl *ctl = nullptr;  // null: always open
+    long long needed = 0;
+    __device__ __forceinline__ bool closed() const { return ctl && ctl->n_acc - ctl->nan_round < needed; }
+};
+
+// Start of an iteration: zero histograms, an empty accumulator
+// (StatsData: min = lim::max(), max = lim::min()) and status.
+__global__ void k_mc_begin(double *__restrict__ hist, long long hist_n, IterAcc *__restrict__ acc,
+                           int *__restrict__ status) {
+    const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    for (long long k = t; k < hist_n; k += static_cast<long long>(gridDim.x) * blockDim.x) hist[k] = 0.0;
+    if (t < CHILI_MAX_CHANNELS) acc->atrain[t] = 0.0;
+    if (t == 0) {
+        for (int q = 0; q < 6; ++q) acc->st[q] = 0.0;
+        acc->st[1] = 1.7976931348623157e308;
+        acc->st[2] = 2.2250738585072014e-308;
+        acc->nan_count = acc->nonfinite = acc->wmax = acc->dropped = acc->rejected_pre = acc->pad = 0.0;
+        *status = 0;
+    }
+}
+
 // ------------------------------------------------------------- grid kernels
 // One block per (dim = blockIdx.x, grid = blockIdx.y): the cell entries and
 // scaled bin widths of that edge table.
 __global__ void k_build_cells(const double *__restrict__ grids, int dims, int bins, uint32_t *__restrict__ entries,
-                              double *__restrict__ ws) {
+                              double *__restrict__ ws, TrainGate gate) {
+    if (gate.closed()) return;
     const int d = blockIdx.x, c = blockIdx.y;
     const size_t row = static_cast<size_t>(c) * dims + d;
     build_cell_row(grids + static_cast<size_t>(c) * dims * (bins + 1), dims, bins, d,
@@ -90,8 +115,9 @@ __global__ void k_grid_weight(const double *__restrict__ g, const uint32_t *__re
 // status bit 1: the rebinning ran past the last bin or before the first.
 __global__ void k_grid_adapt(const double *__restrict__ g_old, double *__restrict__ g_new, int dims, int bins,
                              double alpha, const double *__restrict__ train, int skip_zero,
-                             int *__restrict__ status) {
-    extern __shared__ double tmp[];  // bins
+                             int *__restrict__ status, TrainGate gate) {
+    if (gate.closed()) return;
+    extern __shared__ double tmp[];  // adapt_scratch_bytes(bins)
     grid_adapt_block(g_old, g_new, dims, bins, alpha, train, skip_zero, status, blockIdx.x, blockIdx.y, tmp);
 }
 
@@ -384,13 +410,13 @@ __global__ void k_vegas_step(const double *__restrict__ g, double *__restrict__ 
     vegas_fold_range(gpart, ghist, 0, ngrp, nh, train, out6);
     __syncthreads();  // train complete (and the points' shared histogram no longer needed)
     if (adapt) {
-        // one warp per dimension (each with its own bins doubles of shared
+        // one warp per dimension (each with its own scratch in shared
         // memory), the dimensions in rounds of the block's warps
         if (threadIdx.x == 0) *status = 0;
         __syncthreads();
         const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
         for (int d = w; d < dims; d += nw) grid_adapt_impl<true>(g, g_new, dims, bins, alpha, train, 0, status, d, 0,
-                                                                 sh + static_cast<size_t>(w) * bins);
+                                                                 sh + w * (adapt_scratch_bytes(bins) / sizeof(double)));
     }
     if (threadIdx.x == 0) *arrive = 0u;
 }
@@ -592,15 +618,21 @@ __global__ void __launch_bounds__(kFwdBlock) k_block_count(const uint8_t *__rest
     if (threadIdx.x == 0) block_count[blockIdx.x] = cnt;
 }
 
-// Turns the cut over the record list (ctl_list: cut = records included,
-// n_acc = non-NaN among them) into the round record: counters consumed,
-// PreProcess-accepted points among them, NaN retries among those.
-// iter (queued rounds, may be NULL; k_iter_init): the count still needed
-// replaces `needed` and is brought down by this round, which also adds to
-// the chunk's totals; a round queued after the count reached 0 is empty.
-__global__ void k_cut_finalize(const RoundCtl *__restrict__ ctl_list, const RoundCtl *__restrict__ ctl_pre,
-                               const int32_t *__restrict__ list, long long m, long long needed,
-                               long long *__restrict__ iter, RoundCtl *__restrict__ ctl) {
+// The cut over the record list in one launch: k_mc_scan's work on rec_ok
+// (ctl_list: cut = records included, n_acc = non-NaN among them), then the
+// round record: counters consumed, PreProcess-accepted points among them, NaN
+// retries among those.  iter (queued rounds, may be NULL; k_iter_init): the
+// count still needed replaces `needed` and is brought down by this round,
+// which also adds to the chunk's totals; a round queued after the count
+// reached 0 is empty.
+__global__ void __launch_bounds__(1024) k_mc_cut(const int32_t *__restrict__ block_count, int nb,
+                                                 const uint8_t *__restrict__ rec_ok, long long m, long long needed,
+                                                 long long *__restrict__ iter, long long *__restrict__ block_off,
+                                                 RoundCtl *__restrict__ ctl_list, const RoundCtl *__restrict__ ctl_pre,
+                                                 const int32_t *__restrict__ list, RoundCtl *__restrict__ ctl) {
+    mc_scan_body(block_count, nb, rec_ok, m, needed, iter, 1, block_off, ctl_list);
+    __syncthreads();  // the thread that met the cut has written ctl_list
+    if (threadIdx.x != 0) return;
     if (iter) {
         needed = iter[0];
         if (needed <= 0) {
@@ -640,7 +672,7 @@ __global__ void k_iter_init(long long *__restrict__ iter, long long needed) {
 // out-of-range slots are counted here either way), alpha-training terms
 // val^2 w / dens_j (MultiChannel.hh:167-180).  Dynamic shared memory:
 // (kWgtBlock/32) * nch.
-__global__ void __launch_bounds__(kWgtBlock) k_mc_accum(
+__global__ void __launch_bounds__(kWgtBlock, 8) k_mc_accum(
     const RoundCtl *__restrict__ ctl, long long n_rec, int nch, int dims, int bins, int hist_size,
     const double *__restrict__ rec_val,
     const double *__restrict__ rec_wgt, const uint8_t *__restrict__ rec_ok, const uint4 *__restrict__ rec_bins,
@@ -648,6 +680,9 @@ __global__ void __launch_bounds__(kWgtBlock) k_mc_accum(
     double *__restrict__ part) {
     extern __shared__ double atr_s[];  // (kWgtBlock/32) * nch
     const long long n_list = ctl->n_acc;
+    // blocks past the cut hold no record (the launch covers every drawn point
+    // of the chunk); k_mc_reduce reads the partials of the others only
+    if (blockIdx.x * static_cast<long long>(kWgtBlock) >= n_list) return;
     const long long i = blockIdx.x * static_cast<long long>(kWgtBlock) + threadIdx.x;
     const bool active = i < n_list && i < n_rec;
     const double val = active ? rec_val[i] : 0.0;
@@ -657,25 +692,39 @@ __global__ void __launch_bounds__(kWgtBlock) k_mc_accum(
     double dropped = 0;
     const double val2 = val * val;
     if (active && should_opt) {
-        for_each_train_slot(rec_bins, i, dims, bins, [&](int s) {
-            if (s >= 0 && s < hist_size) {
-                if (hist) atomicAdd(hist + s, val2);
-            } else {
-                dropped += 1;
-            }
-        });
+        if (hist) {
+            for_each_train_slot(rec_bins, i, dims, bins, [&](int s) {
+                if (s >= 0 && s < hist_size) atomicAdd(hist + s, val2);
+                else dropped += 1;
+            });
+        } else if (reinterpret_cast<const uint16_t *>(rec_bins + i * bin_rec_vecs(dims))[0] == 0) {
+            dropped = 1;  // only dimension 0 can lie before the histogram
+        }
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double nonfin = 0;
     if (should_opt) {
-        for (int j = 0; j < nch; ++j) {
-            double term = active ? val2 * wgt / rec_dens[j * n_rec + i] : 0.0;
-            if (guard && !isfinite(term)) {
-                nonfin += 1;
-                term = 0.0;
+        // eight channels at a time: their densities in flight together, their
+        // folds interleaved
+        const double v2w = val2 * wgt;
+        for (int j0 = 0; j0 < nch; j0 += 8) {
+            double term[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int j = min(j0 + q, nch - 1);
+                term[q] = active ? rec_dens[j * n_rec + i] : 1.0;
             }
-            term = warp_sum(term);
-            if (lane == 0) atr_s[w * nch + j] = term;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                term[q] = active ? v2w / term[q] : 0.0;
+                if (guard && j0 + q < nch && !isfinite(term[q])) {
+                    nonfin += 1;
+                    term[q] = 0.0;
+                }
+            }
+            int q;
+            const double r = warp_sum8(term, q);
+            if ((lane & 3) == 0 && j0 + q < nch) atr_s[w * nch + j0 + q] = r;
         }
     }
     double sum = warp_sum(val), sum2 = warp_sum(val * val);
@@ -807,8 +856,8 @@ __global__ void k_mc_accumulate(const double *__restrict__ round_res, int nch, R
 // mode 0: only rebuild cp from alpha.
 __global__ void k_alpha_update(double *__restrict__ alpha, double *__restrict__ best, double *__restrict__ min_diff,
                                double *__restrict__ cp, const double *__restrict__ train, int nch, double beta,
-                               double min_alpha, int mode) {
-    if (threadIdx.x != 0) return;
+                               double min_alpha, int mode, TrainGate gate) {
+    if (gate.closed()) return;
     alpha_update(alpha, best, min_diff, cp, train, nch, beta, min_alpha, mode);
 }
 
