@@ -207,6 +207,7 @@ bool build_point_program(const std::vector<ChannelProgram> &progs, PointProgram 
     pp.sqrts = p0.sqrts;
     pp.ptmax = p0.ptmax;
     pp.inv16pi3 = p0.inv16pi3;
+    pp.rsqrts = 1.0 / p0.sqrts;
     std::map<std::pair<int, int>, int> node_of_pair;
     std::map<std::tuple<int, double, double>, int> tent_of;
     std::map<std::pair<std::vector<int>, int>, int> chain_of;
@@ -254,6 +255,7 @@ bool build_point_program(const std::vector<ChannelProgram> &progs, PointProgram 
                 pp.dw_smin2[id] = P.dec_smin2[k];
                 pp.dw_cut[id] = P.dec_cut_smin[k];
                 pp.dw_smax[id] = P.dec_smax[k];
+                pp.dw_rmw[id] = 1.0 / (P.dec_mass[k] * P.dec_width[k]);
                 // smin when smin1 < max(smin2, cut): evaluated with std::max
                 // semantics in the same order as the device (Channel.cc:151)
                 {
@@ -278,6 +280,8 @@ bool build_point_program(const std::vector<ChannelProgram> &progs, PointProgram 
                 pp.tent_node[id] = static_cast<int8_t>(node[P.info_slot[i]]);
                 pp.tent_ptmin[id] = P.info_ptmin[i];
                 pp.tent_etacut[id] = P.info_etamax[i];
+                pp.tent_rptmin[id] = 1.0 / P.info_ptmin[i];
+                pp.tent_rsum[id] = 1.0 / (2 * P.info_ptmin[i] + P.ptmax);
                 tent_of[key] = id;
             } else {
                 id = it->second;
@@ -322,6 +326,15 @@ bool build_point_program(const std::vector<ChannelProgram> &progs, PointProgram 
     pp.memo_sw = pp.memo_dw + 2 * pp.n_dws;
     pp.memo_chain = pp.memo_sw + 3 * pp.n_sws;
     pp.n_memo = pp.memo_chain + 2 * pp.n_chains;
+    for (int t = 0; t < pp.n_tents; ++t) pp.tent_y[t] = -1;
+    for (int c = 0; c < pp.n_chains; ++c) {
+        pp.chain_y[c] = -1;
+        for (int t = 0; t < pp.n_tents && pp.chain_y[c] < 0; ++t) {
+            if (pp.tent_node[t] != pp.chain_last[c]) continue;
+            if (pp.tent_y[t] < 0) pp.tent_y[t] = static_cast<int16_t>(pp.n_memo++);
+            pp.chain_y[c] = pp.tent_y[t];
+        }
+    }
     for (int c = 0; c < pp.nch; ++c) {
         const PPChannel &C = pp.ch[c];
         for (int fail = 0; fail < 2; ++fail) {

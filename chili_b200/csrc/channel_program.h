@@ -83,6 +83,12 @@ struct PointProgram {
     // massless: pow(smin, 0.01), pow(smax, 0.01); massive: atan((smin-m2)/mw),
     // atan((smax-m2)/mw).
     double dw_smin_c[PP_MAX_DWS], dw_t1[PP_MAX_DWS], dw_t2[PP_MAX_DWS];
+    // and, of these, (t2 - t1) / ce (massless) and 1 over the span that the
+    // uniform is divided by (also filled by k_pp_prepare)
+    double dw_wce[PP_MAX_DWS], dw_rspan[PP_MAX_DWS];
+    // correctly rounded reciprocals of the set's constant divisors:
+    // 1 / ptmin, 1 / (2 ptmin + ptmax), 1 / (m g), 1 / sqrts
+    double tent_rptmin[PP_MAX_TENTS], tent_rsum[PP_MAX_TENTS], dw_rmw[PP_MAX_DWS], rsqrts;
     int8_t sw_a[PP_MAX_SWS], sw_b[PP_MAX_SWS];
     PPChannel ch[CHILI_MAX_CHANNELS];
     // Phased evaluation: every item's outputs live in a memo buffer of
@@ -93,6 +99,9 @@ struct PointProgram {
     // s-channel uniforms move down by one and the last position keeps the
     // value the previous channels left there (-1).
     int32_t memo_tent, memo_dw, memo_sw, memo_chain, n_memo;
+    // memo slot of the rapidity of a t-channel entry whose node is some
+    // chain's last (-1: none), and of a chain's last node
+    int16_t tent_y[PP_MAX_TENTS], chain_y[PP_MAX_CHAINS];
     int16_t pos_src[CHILI_MAX_CHANNELS][CHILI_MAX_DIMS];
     int16_t pos_src_fail[CHILI_MAX_CHANNELS][CHILI_MAX_DIMS];
 };

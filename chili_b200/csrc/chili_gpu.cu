@@ -378,15 +378,19 @@ int chili_gpu_create(int device, chili_ctx **out) {
         return fail(nullptr, CHILI_ERR_CUDA, "cudaStreamCreate failed");
     }
     ctx->own_stream = true;
-    if (cudaMallocHost(reinterpret_cast<void **>(&ctx->ctl_host), 2 * sizeof(RoundCtl)) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void **>(&ctx->iter_host), sizeof(long long) * kIterCtl) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void **>(&ctx->acc_host), sizeof(IterAcc)) != cudaSuccess) {
-        if (ctx->ctl_host) cudaFreeHost(ctx->ctl_host);
-        if (ctx->iter_host) cudaFreeHost(ctx->iter_host);
+    // one pinned block: the round records, the queued rounds' state, the
+    // accumulator (a pinned allocation takes about half a millisecond)
+    constexpr size_t kCtl = 2 * sizeof(RoundCtl), kIter = sizeof(long long) * kIterCtl;
+    static_assert(kCtl % 8 == 0 && kIter % 8 == 0, "8-byte aligned parts");
+    char *pinned = nullptr;
+    if (cudaMallocHost(reinterpret_cast<void **>(&pinned), kCtl + kIter + sizeof(IterAcc)) != cudaSuccess) {
         cudaStreamDestroy(ctx->stream);
         delete ctx;
         return fail(nullptr, CHILI_ERR_CUDA, "cudaMallocHost failed");
     }
+    ctx->ctl_host = reinterpret_cast<RoundCtl *>(pinned);
+    ctx->iter_host = reinterpret_cast<long long *>(pinned + kCtl);
+    ctx->acc_host = reinterpret_cast<IterAcc *>(pinned + kCtl + kIter);
     cudaDeviceGetAttribute(&ctx->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device);
     cudaFuncSetAttribute(k_mc_accum, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin);
@@ -412,9 +416,7 @@ int chili_gpu_destroy(chili_ctx *ctx) {
     flow_release(ctx);
     batch_release(ctx);
     for (auto &b : ctx->stage) b.release();
-    if (ctx->ctl_host) cudaFreeHost(ctx->ctl_host);
-    if (ctx->iter_host) cudaFreeHost(ctx->iter_host);
-    if (ctx->acc_host) cudaFreeHost(ctx->acc_host);
+    if (ctx->ctl_host) cudaFreeHost(ctx->ctl_host);  // the block that holds iter_host and acc_host too
     collect_times(ctx);
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->copy_events) cudaEventDestroy(e);

@@ -40,6 +40,21 @@ __device__ __forceinline__ double mass2(V4 a) { return dot4(a, a); }
 __device__ __forceinline__ double pt2(V4 a) { return dadd(dmul(a.x, a.x), dmul(a.y, a.y)); }
 __device__ __forceinline__ double p2(V4 a) { return dadd(pt2(a), dmul(a.z, a.z)); }
 __device__ __forceinline__ double dot3(V4 a, V4 b) { return dadd(dadd(dmul(a.x, b.x), dmul(a.y, b.y)), dmul(a.z, b.z)); }
+// a / b for a denominator whose correctly rounded reciprocal rb is at hand (a
+// constant of the channel set, or a divisor shared by several quotients):
+// Markstein's correction q + (a - q b) rb of q = a rb ("Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34 (1990)) is the correctly rounded quotient (but for about one pair
+// in 2^50, half an ulp by a hair).  Three FP64 operations instead of about
+// ten; quotients outside 2^-962 .. 2^957 (zeros, infinities, NaN among them)
+// take the division.
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+    const double q = __dmul_rn(a, rb);
+    if ((static_cast<uint32_t>(__double2hiint(q)) & 0x7fffffffu) - 0x03d00000u >= 0x77c00000u) return __ddiv_rn(a, b);
+    return __fma_rn(__fma_rn(-q, b, a), rb, q);
+}
+constexpr double kRcpPi = 1.0 / kPi, kRcpTwoPi = 1.0 / kTwoPi, kEightPi = 8. * kPi, kRcpEightPi = 1.0 / kEightPi;
+
 __device__ __forceinline__ double rapidity(V4 a) {
     if (a.e == 0) return 99;
     return log((a.e + a.z) / (a.e - a.z)) / 2;

@@ -45,24 +45,22 @@ __device__ __forceinline__ double massless_prop_weight(double cn, double cxm, do
     return w / pow(s, -cn);
 }
 
-// The same weights with the (smin, smax)-only terms supplied: t1, t2 are
-// pow(cxm, ce), pow(cxp, ce) (massless) or atan((smin-m2)/mw),
-// atan((smax-m2)/mw) (massive), evaluated by the same functions, so the
-// results are identical to the functions above.
-__device__ __forceinline__ double massless_prop_weight_c(double cn, double t_min, double t_max, double s,
-                                                         double &ran) {
+// The same weights with the (smin, smax)-only terms supplied (evaluated by
+// the same functions, so the results are identical): t_min, t_max are
+// pow(cxm, ce), pow(cxp, ce), w_ce (t_max - t_min) / ce; ymax, ymin are
+// atan((smin-m2)/mw), atan((smax-m2)/mw); r_span 1 over the difference that
+// the uniform is divided by, r_mw 1 / (m g).
+__device__ __forceinline__ double massless_prop_weight_c(double cn, double t_min, double t_max, double w_ce,
+                                                         double r_span, double s, double &ran) {
     const double ce = 1. - cn;
-    const double amin = t_min;
-    double w = t_max - amin;
-    ran = (pow(s, ce) - amin) / w;
-    w /= ce;
-    return w / pow(s, -cn);
+    ran = div_by(pow(s, ce) - t_min, t_max - t_min, r_span);
+    return w_ce / pow(s, -cn);
 }
-__device__ __forceinline__ double massive_prop_weight_c(double m, double g, double ymax, double ymin, double s,
-                                                        double &ran) {
+__device__ __forceinline__ double massive_prop_weight_c(double m, double g, double ymax, double ymin, double r_span,
+                                                        double r_mw, double s, double &ran) {
     const double m2 = m * m, mw = m * g;
-    const double y = atan((s - m2) / mw);
-    ran = (y - ymin) / (ymax - ymin);
+    const double y = atan(div_by(s - m2, mw, r_mw));
+    ran = div_by(y - ymin, ymax - ymin, r_span);
     double w = mw / ((s - m2) * (s - m2) + mw * mw);
     w = (ymin - ymax) / w;
     return w;
@@ -86,37 +84,43 @@ __device__ __forceinline__ double massive_prop_weight(double m, double g, double
     return w;
 }
 
-// LT: the 4-d cross product (ChannelElements.cc:9-19).
-__device__ __forceinline__ V4 lorentz_cross(V4 a, V4 b, V4 c) {
-    const double t = a.x * b.y * c.z + a.y * b.z * c.x + a.z * b.x * c.y - a.x * b.z * c.y -
-                     a.z * b.y * c.x - a.y * b.x * c.z;
-    const double x = -a.e * b.y * c.z - a.y * b.z * c.e - a.z * b.e * c.y + a.e * b.z * c.y +
-                     a.z * b.y * c.e + a.y * b.e * c.z;
-    const double y = -a.x * b.e * c.z - a.e * b.z * c.x - a.z * b.x * c.e + a.x * b.z * c.e +
-                     a.z * b.e * c.x + a.e * b.x * c.z;
-    const double z = -a.x * b.y * c.e - a.y * b.e * c.x - a.e * b.x * c.y + a.x * b.e * c.y +
-                     a.e * b.y * c.x + a.y * b.x * c.e;
-    return V4{t, -x, -y, -z};
-}
-
-// The transverse axis m_t of the rotation Poincare(v1, v2) (Poincare.cc:10-34).
-__device__ __forceinline__ V4 rotation_axis(V4 v1, V4 v2) {
-    const double pv2 = sqrt(p2(v2));
-    const V4 b{0., v2.x / pv2, v2.y / pv2, v2.z / pv2};
-    const double pv1 = sqrt(p2(v1));
-    const V4 l{0., v1.x / pv1, v1.y / pv1, v1.z / pv1};
-    V4 t = b + scale(l, dot4(l, b));
-    const double mt = p2(t);
-    if (mt != 0.) t = scale(t, 1. / sqrt(mt));
-    int i0 = 1, i1 = 2, i2 = 3;
-    const double ml[4] = {0., fabs(l.x), fabs(l.y), fabs(l.z)};
-    if (ml[i2] > ml[i1]) { const int s = i1; i1 = i2; i2 = s; }
-    if (ml[i1] > ml[i0]) { const int s = i0; i0 = i1; i1 = s; }
-    if (ml[i2] > ml[i1]) { const int s = i1; i1 = i2; i2 = s; }
-    const double tdp = comp(t, i1) * comp(l, i1) + comp(t, i2) * comp(l, i2);
-    if (tdp != 0.) set_comp(t, i0, -tdp / comp(l, i0));
-    if (p2(t) == 0.) set_comp(t, i1, 1.);
-    return t;
+// The two transverse axes of a decay of p (SChannelMomenta/SChannelWeight,
+// ChannelElements.cc:87-135) with the reference axis x = (1,1,0,0): n_perp the
+// axis m_t of the rotation Poincare(p, x) (Poincare.cc:10-34), l_perp the
+// normalised LT(p, x, n_perp) (ChannelElements.cc:9-19).  pl is p, or
+// (1,0,0,1) for a vanishing 3-momentum.  The reference's operations in its
+// order, those on the zeros and ones of the reference axis left out (exact:
+// x 1 and + 0 change nothing).
+__device__ __forceinline__ void decay_axes(V4 pl, V4 &l_perp, V4 &n_perp) {
+    const double pv = sqrt(p2(pl)), rpv = 1. / pv;
+    const double l[3] = {div_by(pl.x, pv, rpv), div_by(pl.y, pv, rpv), div_by(pl.z, pv, rpv)};
+    double t[3] = {1. + l[0] * -l[0], l[1] * -l[0], l[2] * -l[0]};
+    const double mt = dadd(dadd(dmul(t[0], t[0]), dmul(t[1], t[1])), dmul(t[2], t[2]));
+    if (mt != 0.) {
+        const double k = 1. / sqrt(mt);
+        t[0] *= k;
+        t[1] *= k;
+        t[2] *= k;
+    }
+    // components by falling |l|: i0 is replaced so that t and l are orthogonal
+    auto pick = [](const double *v, int i) { return i == 0 ? v[0] : (i == 1 ? v[1] : v[2]); };
+    int i0 = 0, i1 = 1, i2 = 2;
+    const double ml[3] = {fabs(l[0]), fabs(l[1]), fabs(l[2])};
+    if (ml[2] > ml[1]) { i1 = 2; i2 = 1; }
+    if (pick(ml, i1) > pick(ml, i0)) { const int s = i1; i1 = i0; i0 = s; }
+    if (pick(ml, i2) > pick(ml, i1)) { const int s = i1; i1 = i2; i2 = s; }
+    const double tdp = pick(t, i1) * pick(l, i1) + pick(t, i2) * pick(l, i2);
+    auto put = [&](int i, double v) {
+        if (i == 0) t[0] = v;
+        else if (i == 1) t[1] = v;
+        else t[2] = v;
+    };
+    if (tdp != 0.) put(i0, -tdp / pick(l, i0));
+    if (mt == 0. && t[0] * t[0] + t[1] * t[1] + t[2] * t[2] == 0.) put(i1, 1.);
+    n_perp = V4{0., t[0], t[1], t[2]};
+    const double e = pl.z * t[1] - pl.y * t[2];
+    l_perp = V4{e, e, -((-pl.x * t[2] + pl.z * t[0]) + pl.e * t[2]), -((-pl.y * t[0] - pl.e * t[1]) + pl.x * t[1])};
+    l_perp = scale(l_perp, 1.0 / sqrt(fabs(mass2(l_perp))));
 }
 
 // Poincare boost with m_l = l, m_rsq = rsq (Poincare.cc:36-50).
@@ -153,15 +157,13 @@ __device__ __forceinline__ void schannel_momenta(V4 p, double s1, double s2, V4 
     const double e1 = (s + s1 - s2) / rs / 2., m1 = sqrt(e1 * e1 - s1);
     const double ct = -1. + 2. * ran1, st = sqrt(1. - ct * ct);
     const double ph = kTwoPi * ran2;
-    const V4 xref{1., 1., 0., 0.};
     const V4 pl = p2(p) != 0. ? p : V4{1., 0., 0., 1.};
-    const double rsq = sqrt(mass2(p));  // Poincare(p): m_rsq = p.Mass()
-    const V4 n_perp = rotation_axis(pl, xref);
-    V4 l_perp = lorentz_cross(pl, xref, n_perp);
-    l_perp = scale(l_perp, 1.0 / sqrt(fabs(mass2(l_perp))));
-    const double plp = sqrt(p2(pl));
+    const double rsq = sqrt(s);  // Poincare(p): m_rsq = p.Mass()
+    V4 n_perp, l_perp;
+    decay_axes(pl, l_perp, n_perp);
+    const double plp = sqrt(p2(pl)), rplp = 1. / plp;
     const double mc = m1 * ct;
-    V4 q{e1, pl.x * mc / plp, pl.y * mc / plp, pl.z * mc / plp};
+    V4 q{e1, div_by(pl.x * mc, plp, rplp), div_by(pl.y * mc, plp, rplp), div_by(pl.z * mc, plp, rplp)};
     const double cph = cos(ph), sph = sin(ph);
     q = q + scale(scale(l_perp, cph) + scale(n_perp, sph), m1 * st);
     q = boost_back(p, rsq, q);
@@ -169,31 +171,43 @@ __device__ __forceinline__ void schannel_momenta(V4 p, double s1, double s2, V4 
     p2o = p - q;
 }
 
+// SqLam of a decay into two legs whose squared masses both vanish, with
+// s = E1 E2 SmallOMCT (ChannelElements.cc:127-131): the general evaluation.
+__device__ __noinline__ inline double massless_pair_lambda(V4 p1, V4 p2v) {
+    return sq_lambda(p1.e * p2v.e * small_omct(p1, p2v), 0., 0.);
+}
+
 // SChannelWeight (ChannelElements.cc:113-135): returns the weight, writes the
 // two uniforms.
 __device__ __forceinline__ double schannel_weight(V4 p1, V4 p2v, double &ran1, double &ran2) {
     const V4 p = p1 + p2v;
     const V4 pl = p2(p) != 0. ? p : V4{1., 0., 0., 1.};
-    const V4 xref{1., 1., 0., 0.};
-    const double rsq = sqrt(mass2(p));
-    const V4 n_perp = rotation_axis(pl, xref);
-    V4 l_perp = lorentz_cross(pl, xref, n_perp);
-    l_perp = scale(l_perp, 1.0 / sqrt(fabs(mass2(l_perp))));
+    const double m2 = mass2(p), rsq = sqrt(m2);
+    V4 n_perp, l_perp;
+    decay_axes(pl, l_perp, n_perp);
     const V4 p1h = boost(p, rsq, p1);
     const double ct = dot3(p1h, pl) / sqrt(p2(p1h) * p2(pl));
-    double cp = -dot4(l_perp, p1), sp = -dot4(n_perp, p1);
-    const double norm = sqrt(cp * cp + sp * sp);
-    cp /= norm;
-    sp /= norm;
-    ran1 = (ct + 1.) / 2.;
-    ran2 = atan2(sp, cp) / kTwoPi;
+    double cp = -dot4(l_perp, p1), sp = -(0. - dot3(n_perp, p1));
+    const double norm = sqrt(cp * cp + sp * sp), rnorm = 1. / norm;
+    cp = div_by(cp, norm, rnorm);
+    sp = div_by(sp, norm, rnorm);
+    ran1 = (ct + 1.) * 0.5;
+    ran2 = div_by(atan2(sp, cp), kTwoPi, kRcpTwoPi);
     if (ran2 < 0.) ran2 += 1.;
-    double w = 1.;  // (ctmax - ctmin)/2
     const double s1 = std_max(mass2(p1), 0.), s2 = std_max(mass2(p2v), 0.);
-    double s = mass2(p);
-    if (s1 == 0. && s2 == 0.) s = p1.e * p2v.e * small_omct(p1, p2v);
-    w *= sq_lambda(s, s1, s2) / (8. * kPi);
-    return w;
+    double lam;
+    if (s1 == 0. && s2 == 0.) {
+        // sqrt(s s) / s is exactly the sign of s, and s = E1 E2 SmallOMCT
+        // has the sign of E1 E2 unless the legs are parallel
+        const double cx = p1.y * p2v.z - p1.z * p2v.y, cy = p1.z * p2v.x - p1.x * p2v.z,
+                     cz = p1.x * p2v.y - p1.y * p2v.x;
+        const double c2 = cx * cx + cy * cy + cz * cz, ee = p1.e * p2v.e, n2 = p2(p1) * p2(p2v);
+        const bool sane = fabs(ee) > 1e-60 && fabs(ee) < 1e60 && n2 > 1e-60 && n2 < 1e60;
+        lam = sane && (c2 > 1e-60 * n2) ? (ee > 0. ? 1. : -1.) : massless_pair_lambda(p1, p2v);
+    } else {
+        lam = sq_lambda(m2, s1, s2);
+    }
+    return div_by(lam, kEightPi, kRcpEightPi);
 }
 
 // ------------------------------------------------- FSMapper forward
@@ -364,12 +378,19 @@ __device__ __forceinline__ void pp_prepare_entry(PointProgram *__restrict__ pp, 
     const double smin = pp->dw_smin_c[k], smax = pp->dw_smax[k];
     if (pp->dw_massless[k]) {
         const double ce = 1. - 0.99;
-        pp->dw_t1[k] = pow(smin, ce);
-        pp->dw_t2[k] = pow(smax, ce);
+        const double t1 = pow(smin, ce), t2 = pow(smax, ce);
+        pp->dw_t1[k] = t1;
+        pp->dw_t2[k] = t2;
+        pp->dw_wce[k] = (t2 - t1) / ce;
+        pp->dw_rspan[k] = 1. / (t2 - t1);
     } else {
         const double m2 = pp->dw_mass[k] * pp->dw_mass[k], mw = pp->dw_mass[k] * pp->dw_width[k];
-        pp->dw_t1[k] = atan((smin - m2) / mw);  // "ymax" of ChannelElements.cc:94
-        pp->dw_t2[k] = atan((smax - m2) / mw);  // "ymin"
+        const double ymax = atan((smin - m2) / mw);  // "ymax" of ChannelElements.cc:94
+        const double ymin = atan((smax - m2) / mw);
+        pp->dw_t1[k] = ymax;
+        pp->dw_t2[k] = ymin;
+        pp->dw_wce[k] = 0.;
+        pp->dw_rspan[k] = 1. / (ymax - ymin);
     }
 }
 

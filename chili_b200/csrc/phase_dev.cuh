@@ -5,6 +5,8 @@
 // covers the pieces of many tasks.
 #pragma once
 
+#include <type_traits>
+
 #include "channel_program.h"
 #include "common.cuh"
 #include "fsmapper.cuh"
@@ -14,15 +16,27 @@
 
 namespace chili_dev {
 
+// Rows of a tile's SoA buffers: element i of row r of stride m.  The row's
+// offset is one 32 x 32 -> 64 bit multiply-add on the element's address (rows
+// stay below 2^32 bytes: a tile or chunk has at most 2^24 points); with 64-bit
+// strides the addresses took a tenth of the item kernels' instructions.
+template <class T>
+__device__ __forceinline__ T *soa_at(T *p, int r, long long m, long long i) {
+    using Byte = std::conditional_t<std::is_const_v<T>, const char, char>;
+    return reinterpret_cast<T *>(reinterpret_cast<Byte *>(p + i) +
+                                 static_cast<unsigned long long>(static_cast<unsigned>(m) * 8u) *
+                                     static_cast<unsigned>(r));
+}
 __device__ __forceinline__ V4 load_v4(const double *__restrict__ soa, int node, long long m, long long i) {
-    return V4{soa[(4 * node + 0) * m + i], soa[(4 * node + 1) * m + i], soa[(4 * node + 2) * m + i],
-              soa[(4 * node + 3) * m + i]};
+    const double *p = soa_at(soa, 4 * node, m, i);
+    return V4{*p, *soa_at(p, 1, m, 0), *soa_at(p, 2, m, 0), *soa_at(p, 3, m, 0)};
 }
 __device__ __forceinline__ void store_v4(double *__restrict__ soa, int node, long long m, long long i, V4 v) {
-    soa[(4 * node + 0) * m + i] = v.e;
-    soa[(4 * node + 1) * m + i] = v.x;
-    soa[(4 * node + 2) * m + i] = v.y;
-    soa[(4 * node + 3) * m + i] = v.z;
+    double *p = soa_at(soa, 4 * node, m, i);
+    *p = v.e;
+    *soa_at(p, 1, m, 0) = v.x;
+    *soa_at(p, 2, m, 0) = v.y;
+    *soa_at(p, 3, m, 0) = v.z;
 }
 
 // The compound nodes of tile point i, summed as the reference's tmp_mom, its
@@ -74,37 +88,44 @@ __device__ __forceinline__ void pp_items_block(const PointProgram *__restrict__ 
         const V4 q = load_v4(node_soa, pp->tent_node[t], m, i);
         const double pt = sqrt(pt2(q));
         const double f2 = 2 * ptmin + pt;
-        double *o = memo + static_cast<long long>(pp->memo_tent + 5 * t) * m + i;
-        o[0] = pt * ptmax / 2 / ptmin / (2 * ptmin + ptmax) * (f2 * f2);
-        o[2 * m] = pt * (ptmax + 2 * ptmin) / (ptmax * (pt + 2 * ptmin));
-        double etamax = sqrts / 2 / pt;
+        double *o = soa_at(memo, pp->memo_tent + 5 * t, m, i);
+        *o = div_by(div_by(pt * ptmax * 0.5, ptmin, pp->tent_rptmin[t]), 2 * ptmin + ptmax, pp->tent_rsum[t]) * (f2 * f2);
+        *soa_at(o, 2, m, 0) = pt * (ptmax + 2 * ptmin) / (ptmax * (pt + 2 * ptmin));
+        double etamax = sqrts * 0.5 / pt;
         etamax = log(etamax + sqrt(etamax * etamax - 1));
         etamax = isnan(etamax) ? 99 : etamax;
         etamax = std_min(etamax, pp->tent_etacut[t]);
-        o[m] = 2 * etamax * 2 * kPi;
-        o[3 * m] = (rapidity(q) / etamax + 1) / 2;
-        o[4 * m] = phi_0_2pi(q) / 2 / kPi;
+        *soa_at(o, 1, m, 0) = 2 * etamax * 2 * kPi;
+        const double y = rapidity(q);
+        if (pp->tent_y[t] >= 0) *soa_at(memo, pp->tent_y[t], m, i) = y;  // some chain's last node
+        *soa_at(o, 3, m, 0) = (y / etamax + 1) * 0.5;
+        *soa_at(o, 4, m, 0) = div_by(phi_0_2pi(q) * 0.5, kPi, kRcpPi);
         return;
     }
     item -= pp->n_tents;
     if (KIND == 1 && item < pp->n_dws) {
         const int k = item;
-        const V4 a = load_v4(node_soa, pp->dw_c1[k], m, i), b = load_v4(node_soa, pp->dw_c2[k], m, i);
-        const double r = sqrt(fabs(mass2(a))) + sqrt(fabs(mass2(b)));
-        const double smin = std_max(std_max(r * r, pp->dw_smin2[k]), pp->dw_cut[k]);
+        const double ma = fabs(mass2(load_v4(node_soa, pp->dw_c1[k], m, i)));
+        const double mb = fabs(mass2(load_v4(node_soa, pp->dw_c2[k], m, i)));
         const double s = mass2(load_v4(node_soa, pp->dw_node[k], m, i));
-        double u, w;
+        double u, w, smin = pp->dw_smin_c[k];
+        // (sqrt ma + sqrt mb)^2 <= 2 (ma + mb): below the cut without the roots
+        if (!(2.0000001 * (ma + mb) < smin)) {
+            const double r = sqrt(ma) + sqrt(mb);
+            smin = std_max(std_max(r * r, pp->dw_smin2[k]), pp->dw_cut[k]);
+        }
         if (smin == pp->dw_smin_c[k]) {  // the usual case: smin-only terms precomputed
-            w = pp->dw_massless[k] ? massless_prop_weight_c(0.99, pp->dw_t1[k], pp->dw_t2[k], s, u)
+            w = pp->dw_massless[k] ? massless_prop_weight_c(0.99, pp->dw_t1[k], pp->dw_t2[k], pp->dw_wce[k],
+                                                            pp->dw_rspan[k], s, u)
                                    : massive_prop_weight_c(pp->dw_mass[k], pp->dw_width[k], pp->dw_t1[k],
-                                                           pp->dw_t2[k], s, u);
+                                                           pp->dw_t2[k], pp->dw_rspan[k], pp->dw_rmw[k], s, u);
         } else {
             w = pp->dw_massless[k] ? massless_prop_weight(0.99, smin, pp->dw_smax[k], s, u)
                                    : massive_prop_weight(pp->dw_mass[k], pp->dw_width[k], smin, pp->dw_smax[k], s, u);
         }
-        double *o = memo + static_cast<long long>(pp->memo_dw + 2 * k) * m + i;
-        o[0] = w / kTwoPi;  // WgtDecays divides by 2 pi per decay (Channel.cc:111)
-        o[m] = u;
+        double *o = soa_at(memo, pp->memo_dw + 2 * k, m, i);
+        *o = div_by(w, kTwoPi, kRcpTwoPi);  // WgtDecays divides by 2 pi per decay (Channel.cc:111)
+        *soa_at(o, 1, m, 0) = u;
         return;
     }
     item -= pp->n_dws;
@@ -113,10 +134,10 @@ __device__ __forceinline__ void pp_items_block(const PointProgram *__restrict__ 
         double r1, r2;
         const double w = schannel_weight(load_v4(node_soa, pp->sw_a[k], m, i), load_v4(node_soa, pp->sw_b[k], m, i),
                                          r1, r2);
-        double *o = memo + static_cast<long long>(pp->memo_sw + 3 * k) * m + i;
-        o[0] = w;
-        o[m] = r1;
-        o[2 * m] = r2;
+        double *o = soa_at(memo, pp->memo_sw + 3 * k, m, i);
+        *o = w;
+        *soa_at(o, 1, m, 0) = r1;
+        *soa_at(o, 2, m, 0) = r2;
     }
 }
 
@@ -136,10 +157,10 @@ __device__ __forceinline__ void pp_chains_block(const PointProgram *__restrict__
     const int len = pp->chain_len[c];
     for (int e = 0; e < len; ++e) {
         const int t = pp->chain_tent[c][e];
-        const double *tm = memo + static_cast<long long>(pp->memo_tent + 5 * t) * m + i;
+        const double *tm = soa_at(static_cast<const double *>(memo), pp->memo_tent + 5 * t, m, i);
         wt *= pp->inv16pi3;
-        wt *= tm[0];
-        wt *= tm[m];
+        wt *= *tm;
+        wt *= *soa_at(tm, 1, m, 0);
         psum = psum + load_v4(node_soa, pp->tent_node[t], m, i);
     }
     const V4 q = load_v4(node_soa, pp->chain_last[c], m, i);
@@ -148,20 +169,18 @@ __device__ __forceinline__ void pp_chains_block(const PointProgram *__restrict__
     const double ptj2 = pt2(psum);
     const double qt = sqrt(mass2(q) + ptj2);
     const double mt = sqrt(mjets2 + ptj2);
-    const double yv = rapidity(q);
-    const double ymin = -log(sqrts / qt * (1 - mt / sqrts * exp(-yjets)));
-    const double ymax = log(sqrts / qt * (1 - mt / sqrts * exp(yjets)));
+    // the last node's rapidity, where a t-channel entry has computed it
+    const int ys = pp->chain_y[c];
+    const double yv = ys >= 0 ? *soa_at(static_cast<const double *>(memo), ys, m, i) : rapidity(q);
+    const double sq = sqrts / qt, ms = div_by(mt, sqrts, pp->rsqrts);
+    const double ymin = -log(sq * (1 - ms * exp(-yjets)));
+    const double ymax = log(sq * (1 - ms * exp(yjets)));
     const double dely = ymax - ymin;
-    double *o = memo + static_cast<long long>(pp->memo_chain + 2 * c) * m + i;
-    if (isnan(ymax) || isnan(ymin)) {
-        o[0] = 0;
-        o[m] = 0;
-        cfail[c * m + i] = 1;
-    } else {
-        o[0] = wt * (dely / sqrts / sqrts);
-        o[m] = (yv - ymin) / dely;
-        cfail[c * m + i] = 0;
-    }
+    double *o = soa_at(memo, pp->memo_chain + 2 * c, m, i);
+    const bool fail = isnan(ymax) || isnan(ymin);
+    *o = fail ? 0 : wt * div_by(div_by(dely, sqrts, pp->rsqrts), sqrts, pp->rsqrts);
+    *soa_at(o, 1, m, 0) = fail ? 0 : (yv - ymin) / dely;
+    cfail[c * m + i] = fail;
 }
 
 // Pair Breit-Wigner / t-channel integrand reading the externals from the
