@@ -272,25 +272,14 @@ __device__ __forceinline__ void bt_forward_block(const BatchDev &B, int ti, long
     if (k < mm) {
         const int D = T.dims, bins = T.bins;
         const uint64_t ctr = (*B.iter << 32) + static_cast<uint64_t>(ctr_off + p0 + k);
-        double r[CHILI_MAX_DIMS + 1];
-        load_uniforms(T.key, ctr, nullptr, D + 1, r);
-        const int c = select_channel(B.cp + T.ch_off, T.nch, r[D]);
-        const double *g = B.grids + T.grid_off + static_cast<size_t>(c) * D * (bins + 1);
-        double jac;
-        if (grid_map_checked(g, D, bins, r, jac)) {
-            V4 mom[CHILI_MAX_SLOTS];
-            double m2[CHILI_MAX_SLOTS];
-            const ChannelProgram *prog = B.progs + T.ch_off + c;
-            fs_generate(prog, r, mom, m2);
-            if (preprocess(B.descs + T.desc, mom)) {
-                acc = 1;
-                for (int s = 0; s < prog->n_ext; ++s) {
-                    mom_soa[(4 * s + 0) * ms + k] = mom[s].e;
-                    mom_soa[(4 * s + 1) * ms + k] = mom[s].x;
-                    mom_soa[(4 * s + 2) * ms + k] = mom[s].y;
-                    mom_soa[(4 * s + 3) * ms + k] = mom[s].z;
-                }
-            }
+        V4 mom[CHILI_MAX_SLOTS];
+        const ChannelProgram *progs = B.progs + T.ch_off;
+        const int ne = progs->n_ext;
+        const int c = draw_point(progs, B.grids + T.grid_off, B.cp + T.ch_off, T.nch, D, bins, T.key, ctr, nullptr, ne,
+                                 mom);
+        if (preprocess(B.descs + T.desc, mom)) {
+            acc = 1;
+            for (int s = 0; s < ne; ++s) store_v4(mom_soa, s, ms, k, mom[s]);
         }
         ich_out[k] = c;
         flag[k] = static_cast<uint8_t>(acc);
@@ -493,7 +482,7 @@ __device__ __forceinline__ long long round_points(const RetryState &R, const Pie
     return m <= 0 ? 0 : (m < P.mm ? m : P.mm);
 }
 
-__global__ void __launch_bounds__(kFwdBlock) k_g_forward(BatchDev B, WaveDev W, int lo, int hi, long long blk0) {
+__global__ void __launch_bounds__(kFwdBlock, 3) k_g_forward(BatchDev B, WaveDev W, int lo, int hi, long long blk0) {
     CHILI_PIECE(GS_FWD)
     if (B.tasks[P.ti].retry) {
         const RetryState &R = B.retry[P.ti];
@@ -1627,6 +1616,7 @@ int chili_gpu_batch_set(chili_ctx *ctx, const chili_task *tasks, int ntasks) {
             d.pre = t.pre;
             d.n_ext = t.n_ext;
             for (int i = 0; i < 4; ++i) d.cut[i] = t.pre == CHILI_PRE_CUTS ? t.pre_cuts[i] : 0.0;
+            set_cut_bounds(d);
         } else {
             batch_release(ctx);
             return fail(ctx, CHILI_ERR_INVALID_ARG, "task " + std::to_string(k) + ": unknown kind");

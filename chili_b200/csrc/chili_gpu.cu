@@ -774,6 +774,7 @@ int chili_gpu_set_preprocess_cuts(chili_ctx *ctx, double sqrts, double ptmin, do
     ctx->f_host.cut[1] = ptmin;
     ctx->f_host.cut[2] = etamax;
     ctx->f_host.cut[3] = delta_r;
+    set_cut_bounds(ctx->f_host);
     CK(ctx->f_dev.ensure(sizeof(IntegrandDesc)));
     CK(cudaMemcpyAsync(ctx->f_dev.p, &ctx->f_host, sizeof(IntegrandDesc), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));

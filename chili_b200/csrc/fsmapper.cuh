@@ -164,7 +164,8 @@ __device__ __forceinline__ void schannel_momenta(V4 p, double s1, double s2, V4 
     const double plp = sqrt(p2(pl)), rplp = 1. / plp;
     const double mc = m1 * ct;
     V4 q{e1, div_by(pl.x * mc, plp, rplp), div_by(pl.y * mc, plp, rplp), div_by(pl.z * mc, plp, rplp)};
-    const double cph = cos(ph), sph = sin(ph);
+    double cph, sph;
+    sincos(ph, &sph, &cph);
     q = q + scale(scale(l_perp, cph) + scale(n_perp, sph), m1 * st);
     q = boost_back(p, rsq, q);
     p1 = q;
@@ -213,11 +214,9 @@ __device__ __forceinline__ double schannel_weight(V4 p1, V4 p2v, double &ran1, d
 // ------------------------------------------------- FSMapper forward
 // FSMapper::GeneratePoint (Channel.cc:22-38): x[ndims] -> mom[slot] for all
 // slots; mom[0..n_ext) are the external legs (incoming with negative energy).
-__device__ __forceinline__ void fs_generate(const ChannelProgram *__restrict__ P, const double *x,
-                                            V4 *mom, double *m2) {
-    const int n_ext = P->n_ext;
-    for (int s = 0; s < P->n_slots; ++s) m2[s] = P->slot_m2[s];
+__device__ __forceinline__ void fs_generate(const ChannelProgram *__restrict__ P, const double *x, V4 *mom, double *m2) {
     int ir = 0;
+    for (int s = 0; s < P->n_slots; ++s) m2[s] = P->slot_m2[s];
     // GenDecays (Channel.cc:63-81)
     const int nd = P->n_decay;
     for (int k = 0; k < nd; ++k) {
@@ -248,8 +247,11 @@ __device__ __forceinline__ void fs_generate(const ChannelProgram *__restrict__ P
         const double ph = kTwoPi * x[ir++];
         const int sl = P->info_slot[i];
         const double mt = sqrt(pt * pt + m2[sl]);
-        mom[sl] = V4{mt * coshy, pt * cos(ph), pt * sin(ph), mt * sinhy};
-        psum = psum + mom[sl];
+        double sph, cph;
+        sincos(ph, &sph, &cph);
+        const V4 q{mt * coshy, pt * cph, pt * sph, mt * sinhy};
+        mom[sl] = q;
+        psum = psum + q;
     }
     {
         const int sl = P->info_slot[ni - 1];
@@ -264,8 +266,9 @@ __device__ __forceinline__ void fs_generate(const ChannelProgram *__restrict__ P
         const double yv = ymin + x[ir++] * dely;
         const double sinhy = sinh(yv);
         const double coshy = sqrt(1 + sinhy * sinhy);
-        mom[sl] = V4{qt * coshy, -psum.x, -psum.y, qt * sinhy};
-        const V4 tot = mom[sl] + psum;
+        const V4 q{qt * coshy, -psum.x, -psum.y, qt * sinhy};
+        mom[sl] = q;
+        const V4 tot = q + psum;
         const double pp = tot.e + tot.z, pm = tot.e - tot.z;
         mom[0] = V4{-pp / 2, 0, 0, -pp / 2};
         mom[1] = V4{-pm / 2, 0, 0, pm / 2};
@@ -278,7 +281,6 @@ __device__ __forceinline__ void fs_generate(const ChannelProgram *__restrict__ P
         const double r2 = x[ir++];
         schannel_momenta(mom[P->sdec_ab[k]], m2[a], m2[b], mom[a], mom[b], r1, r2);
     }
-    (void)n_ext;
 }
 
 // ------------------------------------------------- FSMapper inverse

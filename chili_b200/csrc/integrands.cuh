@@ -5,6 +5,8 @@
 // integrands are compiled in and chosen by chili_integrand_kind.
 #pragma once
 
+#include <cmath>
+
 #include "chili_gpu.h"
 #include "common.cuh"
 
@@ -17,7 +19,21 @@ struct IntegrandDesc {
     int32_t n_ext;  // external legs (CHILI_PRE_CUTS)
     double p[CHILI_MAX_INTEGRAND_PARAMS];
     double cut[4];  // CHILI_PRE_CUTS: sqrts, ptmin, etamax, delta_r
+    double sure[3];  // set_cut_bounds
 };
+
+// Bounds that decide most cuts of CHILI_PRE_CUTS without the transverse
+// angles: |z| / pT below which |eta| <= etamax surely holds, and
+// cosh(deta) - cos(dphi) above which a pair's Delta R surely reaches delta_r
+// (at most cosh(R) - 1 on the circle of radius R) and below which it surely
+// does not (at least 1 - cos(R), R <= pi).  The margins are far above the
+// rounding of both sides; what they leave open takes the angles themselves.
+inline void set_cut_bounds(IntegrandDesc &f) {
+    const double eta = f.cut[2], r = f.cut[3];
+    f.sure[0] = eta > 700.0 ? 1e300 : std::sinh(eta) * (1.0 - 1e-9) - 1e-9;
+    f.sure[1] = r > 3.0 ? 1e300 : (std::cosh(r) - 1.0) * (1.0 + 1e-6) + 1e-9;
+    f.sure[2] = r > 3.0 ? -1.0 : (1.0 - std::cos(r)) * (1.0 - 1e-6) - 1e-9;
+}
 
 // f(x) = N [exp(-|x-a|^2/s^2) + exp(-|x-b|^2/s^2)]; params {s, N, a[D], b[D]}.
 __device__ __forceinline__ double camel(const IntegrandDesc *__restrict__ f, const double *x, int dims) {
@@ -66,20 +82,16 @@ __device__ __forceinline__ double eval_momenta(const IntegrandDesc *__restrict__
     }
 }
 
-// The physical region and the cuts of CHILI_PRE_CUTS (include/chili_gpu.h).
-// NaN momenta fail every comparison.
-__device__ __forceinline__ bool pass_cuts(const IntegrandDesc *__restrict__ f, const V4 *mom) {
-    const double half = 0.5 * f->cut[0] * (1.0 + 1e-12);
-    if (!(-mom[0].e <= half) || !(-mom[1].e <= half)) return false;
-    const double pt2min = f->cut[1] * f->cut[1], etamax = f->cut[2], dr2 = f->cut[3] * f->cut[3];
+// The eta and Delta R cuts of CHILI_PRE_CUTS on legs whose pT passed.
+__device__ __noinline__ inline bool pass_angles(const IntegrandDesc *__restrict__ f, const V4 *mom) {
+    const double etamax = f->cut[2], dr2 = f->cut[3] * f->cut[3];
     const int ne = f->n_ext;
     double eta[CHILI_MAX_EXT], phi[CHILI_MAX_EXT];
     for (int i = 2; i < ne; ++i) {
-        const double pt2 = mom[i].x * mom[i].x + mom[i].y * mom[i].y;
-        if (!(pt2 >= pt2min) || !(pt2 > 0)) return false;
-        eta[i] = asinh(mom[i].z / sqrt(pt2));
+        const V4 q = mom[i];
+        eta[i] = asinh(q.z / sqrt(q.x * q.x + q.y * q.y));
         if (!(fabs(eta[i]) <= etamax)) return false;
-        phi[i] = atan2(mom[i].y, mom[i].x);
+        phi[i] = atan2(q.y, q.x);
     }
     for (int i = 2; i < ne; ++i)
         for (int j = i + 1; j < ne; ++j) {
@@ -89,6 +101,41 @@ __device__ __forceinline__ bool pass_cuts(const IntegrandDesc *__restrict__ f, c
             if (!(deta * deta + dphi * dphi >= dr2)) return false;
         }
     return true;
+}
+
+// The physical region and the cuts of CHILI_PRE_CUTS (include/chili_gpu.h).
+// NaN momenta fail every comparison.  The bounds replace an asinh and an
+// atan2 per leg by two roots: the forward pass of 1.7e6 2->4 points 0.59 ->
+// 0.54 ms (with sincos; the angles inside the pair loop instead of behind it:
+// 0.63 ms, some lane of a warp always took them).
+__device__ __forceinline__ bool pass_cuts(const IntegrandDesc *__restrict__ f, const V4 *mom) {
+    const double half = 0.5 * f->cut[0] * (1.0 + 1e-12);
+    if (!(-mom[0].e <= half) || !(-mom[1].e <= half)) return false;
+    const double pt2min = f->cut[1] * f->cut[1];
+    const int ne = f->n_ext;
+    double pabs[CHILI_MAX_EXT], ptr[CHILI_MAX_EXT];  // |p|, pT
+    bool open = false;  // a cut that the bounds do not decide
+    for (int i = 2; i < ne; ++i) {
+        const V4 q = mom[i];
+        const double t2 = q.x * q.x + q.y * q.y;
+        if (!(t2 >= pt2min) || !(t2 > 0)) return false;
+        ptr[i] = sqrt(t2);
+        pabs[i] = sqrt(p2(q));
+        open = open || !(fabs(q.z) < f->sure[0] * ptr[i]);
+    }
+    for (int i = 2; i < ne; ++i) {
+        const V4 q = mom[i];
+        for (int j = i + 1; j < ne; ++j) {
+            // (|p_i| |p_j| - p_i p_j) / (pT_i pT_j) = cosh(deta) - cos(dphi);
+            // its rounding error is a few ulps of |p_i| |p_j|
+            const double pp = pabs[i] * pabs[j], tt = ptr[i] * ptr[j];
+            const double v = pp - dot3(q, mom[j]);
+            const bool sound = pp < 1e5 * tt;
+            if (sound && v < f->sure[2] * tt) return false;
+            open = open || !(sound && v > f->sure[1] * tt);
+        }
+    }
+    return !open || pass_angles(f, mom);
 }
 
 // PreProcess (MultiChannel.hh:219-223); CHILI_PRE_FINITE follows the first

@@ -492,7 +492,7 @@ __global__ void k_mc_weight_batch(const ChannelProgram *__restrict__ progs, cons
 }
 
 // ------------------------------------------------------------- multichannel
-__global__ void __launch_bounds__(kFwdBlock) k_mc_forward(
+__global__ void __launch_bounds__(kFwdBlock, 3) k_mc_forward(
     const ChannelProgram *__restrict__ progs, const double *__restrict__ grids, const double *__restrict__ cp,
     int nch, int dims, int bins, uint64_t seed, uint64_t ctr0, const double *__restrict__ u_in, long long m,
     const IntegrandDesc *__restrict__ f, int n_ext, double *__restrict__ mom_soa, int32_t *__restrict__ ich_out,
@@ -505,30 +505,11 @@ __global__ void __launch_bounds__(kFwdBlock) k_mc_forward(
     const long long k = blockIdx.x * static_cast<long long>(kFwdBlock) + threadIdx.x;
     int acc = 0;
     if (k < m) {
-        double r[CHILI_MAX_DIMS + 1];
-        if (u_in) {
-            for (int j = 0; j <= dims; ++j) r[j] = __ldg(u_in + k * (dims + 1) + j);
-        } else {
-            load_uniforms(seed, ctr0 + k, nullptr, dims + 1, r);
-        }
-        const int c = select_channel(cp, nch, r[dims]);
-        const double *g = grids + static_cast<size_t>(c) * dims * (bins + 1);
-        double jac;
         V4 mom[CHILI_MAX_SLOTS];
-        double m2[CHILI_MAX_SLOTS];
-        if (grid_map_checked(g, dims, bins, r, jac)) {
-            fs_generate(progs + c, r, mom, m2);
-        } else {
-            for (int s = 0; s < n_ext; ++s) mom[s] = V4{CUDART_NAN, CUDART_NAN, CUDART_NAN, CUDART_NAN};
-        }
+        const int c = draw_point(progs, grids, cp, nch, dims, bins, seed, u_in ? k : ctr0 + k, u_in, n_ext, mom);
         acc = preprocess(f, mom) ? 1 : 0;
         if (acc) {
-            for (int s = 0; s < n_ext; ++s) {
-                mom_soa[(4 * s + 0) * m + k] = mom[s].e;
-                mom_soa[(4 * s + 1) * m + k] = mom[s].x;
-                mom_soa[(4 * s + 2) * m + k] = mom[s].y;
-                mom_soa[(4 * s + 3) * m + k] = mom[s].z;
-            }
+            for (int s = 0; s < n_ext; ++s) store_v4(mom_soa, s, m, k, mom[s]);
         }
         ich_out[k] = c;
         flag[k] = static_cast<uint8_t>(acc);

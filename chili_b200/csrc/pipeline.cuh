@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) k_pp_given(const PointProgram *__restrict
 // Tile of drawn points (counters ctr0 + base + i): channel, VEGAS map,
 // FSMapper; nodes, the tile's channels and count, and the points' momenta
 // and channels where asked for.  No PreProcess.
-__global__ void __launch_bounds__(kFwdBlock) k_pp_drawn(
+__global__ void __launch_bounds__(kFwdBlock, 3) k_pp_drawn(
     const PointProgram *__restrict__ pp, const ChannelProgram *__restrict__ progs, const double *__restrict__ grids,
     const double *__restrict__ cp, int dims, int bins, uint64_t seed, uint64_t ctr0, long long base, long long n,
     long long m, double *__restrict__ node_soa, int32_t *__restrict__ ich_tile, double *__restrict__ mom_out,
@@ -148,16 +148,8 @@ __global__ void __launch_bounds__(kFwdBlock) k_pp_drawn(
     if (i == 0) *count = n;
     if (i >= m || base + i >= n) return;
     const int ne = pp->n_ext;
-    double r[CHILI_MAX_DIMS + 1], jac;
-    load_uniforms(seed, ctr0 + base + i, nullptr, dims + 1, r);
-    const int c = select_channel(cp, pp->nch, r[dims]);
     V4 mom[CHILI_MAX_SLOTS];
-    double m2[CHILI_MAX_SLOTS];
-    if (grid_map_checked(grids + static_cast<size_t>(c) * dims * (bins + 1), dims, bins, r, jac)) {
-        fs_generate(progs + c, r, mom, m2);
-    } else {
-        for (int s = 0; s < ne; ++s) mom[s] = V4{CUDART_NAN, CUDART_NAN, CUDART_NAN, CUDART_NAN};
-    }
+    const int c = draw_point(progs, grids, cp, pp->nch, dims, bins, seed, ctr0 + base + i, nullptr, ne, mom);
     if (mom_out) {
         double *o = mom_out + (base + i) * ne * 4;
         if (aligned16(mom_out)) {
