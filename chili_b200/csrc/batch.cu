@@ -158,8 +158,9 @@ __global__ void __launch_bounds__(256) k_batch_eval(BatchDev B) {
                     double r[CHILI_MAX_DIMS];
                     load_uniforms(T.key, ctr, nullptr, D, r);
                     const double *g = B.grids + T.grid_off;
+                    const double s2 = f->p[0] * f->p[0];
                     double jac;
-                    if (grid_map_checked(g, D, bins, r, jac)) val = camel(f, r, D) * jac;
+                    if (grid_map_checked(g, D, bins, r, jac)) val = camel(f, r, D, s2, 1. / s2) * jac;
                     else val = CUDART_NAN;
                     const double v2 = val * val;
                     double *H = B.hist + T.hist_off;

@@ -383,7 +383,8 @@ int chili_gpu_create(int device, chili_ctx **out) {
     constexpr size_t kCtl = 2 * sizeof(RoundCtl), kIter = sizeof(long long) * kIterCtl;
     static_assert(kCtl % 8 == 0 && kIter % 8 == 0, "8-byte aligned parts");
     char *pinned = nullptr;
-    if (cudaMallocHost(reinterpret_cast<void **>(&pinned), kCtl + kIter + sizeof(IterAcc)) != cudaSuccess) {
+    if (cudaMallocHost(reinterpret_cast<void **>(&pinned), kCtl + kIter + sizeof(IterAcc) + sizeof(chili_stats)) !=
+        cudaSuccess) {
         cudaStreamDestroy(ctx->stream);
         delete ctx;
         return fail(nullptr, CHILI_ERR_CUDA, "cudaMallocHost failed");
@@ -391,11 +392,12 @@ int chili_gpu_create(int device, chili_ctx **out) {
     ctx->ctl_host = reinterpret_cast<RoundCtl *>(pinned);
     ctx->iter_host = reinterpret_cast<long long *>(pinned + kCtl);
     ctx->acc_host = reinterpret_cast<IterAcc *>(pinned + kCtl + kIter);
+    ctx->stats_host = reinterpret_cast<chili_stats *>(pinned + kCtl + kIter + sizeof(IterAcc));
     cudaDeviceGetAttribute(&ctx->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device);
     cudaFuncSetAttribute(k_mc_accum, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin);
     cudaFuncSetAttribute(k_mc_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin);
-    cudaFuncSetAttribute(k_vegas_iter<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin);
+    cudaFuncSetAttribute(k_vegas_iter<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin);
     cudaFuncSetAttribute(k_grid_adapt, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin);
     cudaGetLastError();
     *out = ctx;
@@ -804,10 +806,13 @@ int chili_gpu_vegas_iterate(chili_ctx *ctx, uint64_t ncalls, uint64_t seed, uint
     const bool smem = hist_bytes <= 48 * 1024;
     if (smem && adapt && ctx->vegas_fused && ctx->g_nch == 1 &&
         sizeof(double) * B * (kVegasBlock / 32) <= 48 * 1024) {
-        const size_t step_smem = std::max(hist_bytes, adapt_scratch_bytes(B) * (kVegasBlock / 32));
+        const size_t grid_bytes = sizeof(double) * D * (B + 1);
+        const size_t step_smem = std::max(hist_bytes + (vegas_stages_grid(D, B) ? grid_bytes : 0),
+                                          adapt_scratch_bytes(B) * (kVegasBlock / 32));
         // the whole iteration in one launch (k_vegas_step): points, a
         // two-level ordered fold and the adaptation
-        const long long nb = std::min<long long>(grid_for(n, kVegasBlock), static_cast<long long>(sms) * 4);
+        const long long nb = std::min<long long>({grid_for(n, kVegasBlock), static_cast<long long>(sms) * 4,
+                                                  static_cast<long long>(kStepGroup) * kMaxStepGroups});
         const long long ngrp = (nb + kStepGroup - 1) / kStepGroup;
         CK(ctx->v_part.ensure(sizeof(double) * 6 * (nb + ngrp)));
         CK(ctx->v_hist.ensure(hist_bytes * (nb + ngrp)));
@@ -823,20 +828,24 @@ int chili_gpu_vegas_iterate(chili_ctx *ctx, uint64_t ncalls, uint64_t seed, uint
         using StepKernel = void (*)(const double *, double *, int, int, uint64_t, uint64_t, const double *, long long,
                                     const IntegrandDesc *, double *, double *, double *, double *, double *, double *,
                                     double, int, unsigned *, int *);
-        StepKernel kern = k_vegas_step<0>;
+        const bool stage = vegas_stages_grid(D, B);
+        StepKernel kern = stage ? k_vegas_step<0, true> : k_vegas_step<0, false>;
         switch (D) {
 #define CHILI_ST(d) \
-    case d: kern = k_vegas_step<d>; break;
+    case d: kern = stage ? k_vegas_step<d, true> : k_vegas_step<d, false>; break;
             CHILI_ST(1) CHILI_ST(2) CHILI_ST(3) CHILI_ST(4) CHILI_ST(5) CHILI_ST(6) CHILI_ST(7) CHILI_ST(8)
             CHILI_ST(10) CHILI_ST(12) CHILI_ST(16)
 #undef CHILI_ST
             default: break;
         }
         double *train_dev = train_out ? static_cast<double *>(atr.dev) : ctx->v_train.as<double>();
-        double *out_dev = stats_out ? static_cast<double *>(ast.dev) : ctx->v_out.as<double>();
+        // host StatsData: the kernel writes the six numbers to pinned host
+        // memory, no copy follows
+        double *out_dev = !stats_out ? ctx->v_out.as<double>()
+                                     : (ast.host ? reinterpret_cast<double *>(ctx->stats_host) : static_cast<double *>(ast.dev));
         {
             KTimer kt_(ctx, KT_VEGAS_STEP);
-            if (step_smem > 48 * 1024)
+            if (step_smem > 40 * 1024)  // with the kernel's own (static) 4.6 KB above 48 KB
                 CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(step_smem)));
             kern<<<static_cast<unsigned>(nb), kVegasBlock, step_smem, ctx->stream>>>(
                 ctx->edges.as<double>(), ctx->edges_tmp.as<double>(), D, B, seed, counter_base,
@@ -847,8 +856,10 @@ int chili_gpu_vegas_iterate(chili_ctx *ctx, uint64_t ncalls, uint64_t seed, uint
         LAUNCHED();
         std::swap(ctx->edges, ctx->edges_tmp);
         ctx->hints_stale = true;  // rebuilt where a bin search uses them
-        if ((rc = finish_out(ctx, ast)) || (rc = finish_out(ctx, atr))) return rc;
-        return sync_if_host(ctx, {&au, &ast, &atr});
+        if ((rc = finish_out(ctx, atr))) return rc;
+        if ((rc = sync_if_host(ctx, {&au, &ast, &atr}))) return rc;
+        if (ast.host) std::memcpy(stats_out, ctx->stats_host, sizeof(chili_stats));
+        return CHILI_OK;
     }
     long long nblocks = std::min<long long>(grid_for(n, kVegasBlock), static_cast<long long>(sms) * 4);
     CK(ctx->v_part.ensure(sizeof(double) * 6 * nblocks));
@@ -859,17 +870,21 @@ int chili_gpu_vegas_iterate(chili_ctx *ctx, uint64_t ncalls, uint64_t seed, uint
     {
     using IterKernel = void (*)(const double *, int, int, uint64_t, uint64_t, const double *, long long,
                                 const IntegrandDesc *, double *, double *, int);
-    IterKernel kern = k_vegas_iter<0>;  // the histogram stays below 48 KB of shared memory here
+    const bool stage = smem && vegas_stages_grid(D, B);
+    IterKernel kern = stage ? k_vegas_iter<0, true> : k_vegas_iter<0, false>;  // at most 48 KB of shared memory
     switch (D) {
 #define CHILI_IT(d) \
-    case d: kern = k_vegas_iter<d>; break;
+    case d: kern = stage ? k_vegas_iter<d, true> : k_vegas_iter<d, false>; break;
         CHILI_IT(1) CHILI_IT(2) CHILI_IT(3) CHILI_IT(4) CHILI_IT(5) CHILI_IT(6) CHILI_IT(7) CHILI_IT(8)
         CHILI_IT(10) CHILI_IT(12) CHILI_IT(16)
 #undef CHILI_IT
         default: break;
     }
     KTimer kt_(ctx, KT_VEGAS);
-    kern<<<static_cast<unsigned>(nblocks), kVegasBlock, smem ? hist_bytes : 0, ctx->stream>>>(
+    const size_t it_smem = (smem ? hist_bytes : 0) + (stage ? sizeof(double) * D * (B + 1) : 0);
+    if (it_smem > 40 * 1024)  // with the kernel's own (static) 1.5 KB above 48 KB
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(it_smem)));
+    kern<<<static_cast<unsigned>(nblocks), kVegasBlock, it_smem, ctx->stream>>>(
         ctx->edges.as<double>(), D, B, seed, counter_base, static_cast<const double *>(au.dev), n,
         ctx->f_dev.as<IntegrandDesc>(), ctx->v_part.as<double>(), ctx->v_hist.as<double>(), smem ? 1 : 0);
     }
@@ -901,11 +916,11 @@ int chili_gpu_vegas_generate(chili_ctx *ctx, uint64_t n, uint64_t seed, uint64_t
     if (n == 0) return CHILI_OK;
     if (n > (1ull << 40)) return fail(ctx, CHILI_ERR_LIMIT, "n must be at most 2^40");
     const int D = ctx->dims, B = ctx->bins;
-    // points per thread: 4 where the staged tile stays small, else 1
+    // the option's points per thread where the staged tile stays small, else 1
     const size_t grid_doubles = (static_cast<size_t>(D) * (B + 1) + 1) / 2 * 2;
     int ppt = static_cast<int>(ctx->gen_ppt);
     if (sizeof(double) * (grid_doubles + static_cast<size_t>(kGenTile) * ppt * (D + 1)) > 64 * 1024) ppt = 1;
-    const size_t smem = sizeof(double) * (grid_doubles + static_cast<size_t>(kGenTile) * ppt * (D + 1));
+    size_t smem = sizeof(double) * (grid_doubles + static_cast<size_t>(kGenTile) * ppt * (D + 1));
     if (smem > 200 * 1024) return fail(ctx, CHILI_ERR_LIMIT, "grid too large for the shared-memory staging");
     const long long nn = static_cast<long long>(n);
     Arg ax, aw;
@@ -913,16 +928,28 @@ int chili_gpu_vegas_generate(chili_ctx *ctx, uint64_t n, uint64_t seed, uint64_t
     if ((rc = resolve(ctx, w_out, sizeof(double) * nn, 1, false, aw))) return rc;
     using GenKernel = void (*)(const double *, int, int, uint64_t, uint64_t, long long, const IntegrandDesc *,
                                double *, double *);
-    GenKernel kern = k_vegas_generate<0, 1>;
-    switch (D * 8 + ppt) {
-#define CHILI_GEN(d)                                             \
-    case d * 8 + 1: kern = k_vegas_generate<d, 1>; break;       \
-    case d * 8 + 2: kern = k_vegas_generate<d, 2>; break;       \
-    case d * 8 + 4: kern = k_vegas_generate<d, 4>; break;
+    // rows straight from the threads where their stores are aligned
+    const uintptr_t at = reinterpret_cast<uintptr_t>(ax.dev);
+    const bool row = D % 4 == 0 ? at % 32 == 0 : (D % 2 == 0 && at % 16 == 0);
+    GenKernel kern = nullptr;
+    switch (D) {
+#define CHILI_GEN(d)                                                                                            \
+    case d:                                                                                                     \
+        if (row)                                                                                                \
+            kern = ppt == 1 ? k_vegas_generate<d, 1, d % 2 == 0>                                                \
+                            : (ppt == 2 ? k_vegas_generate<d, 2, d % 2 == 0> : k_vegas_generate<d, 4, d % 2 == 0>); \
+        else                                                                                                    \
+            kern = ppt == 1 ? k_vegas_generate<d, 1, false>                                                     \
+                            : (ppt == 2 ? k_vegas_generate<d, 2, false> : k_vegas_generate<d, 4, false>);       \
+        if (row) smem = sizeof(double) * grid_doubles;                                                          \
+        break;
         CHILI_GEN(1) CHILI_GEN(2) CHILI_GEN(3) CHILI_GEN(4) CHILI_GEN(5) CHILI_GEN(6) CHILI_GEN(7) CHILI_GEN(8)
         CHILI_GEN(10) CHILI_GEN(12) CHILI_GEN(16)
 #undef CHILI_GEN
-        default: ppt = 1; break;
+        default:
+            kern = k_vegas_generate<0, 1, false>;
+            ppt = 1;
+            break;
     }
     if (smem > 48 * 1024)
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
@@ -1819,7 +1846,7 @@ extern "C" int chili_gpu_vegas_iterate_noalloc(void *stream, const double *edges
     const long long n = static_cast<long long>(ncalls);
     const long long nblocks = std::min<long long>(std::min<long long>(grid_for(n, kVegasBlock), sms * 4ll),
                                                   kNoAllocMaxBlocks);
-    k_vegas_iter<0><<<static_cast<unsigned>(nblocks), kVegasBlock, 0, st>>>(edges, dims, bins, seed, counter_base,
+    k_vegas_iter<0, false><<<static_cast<unsigned>(nblocks), kVegasBlock, 0, st>>>(edges, dims, bins, seed, counter_base,
                                                                           nullptr, n, desc_dev, part, train_out, 0);
     CK(cudaGetLastError());
     k_vegas_finalize<<<1, 256, 0, st>>>(part, static_cast<int>(nblocks), nullptr, 0, nh, train_out, stats_out);

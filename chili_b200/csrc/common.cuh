@@ -53,6 +53,12 @@ __device__ __forceinline__ double div_by(double a, double b, double rb) {
     if ((static_cast<uint32_t>(__double2hiint(q)) & 0x7fffffffu) - 0x03d00000u >= 0x77c00000u) return __ddiv_rn(a, b);
     return __fma_rn(__fma_rn(-q, b, a), rb, q);
 }
+// floor(v) of v in [0, 2^31), as integer and double (exact; no conversion).
+__device__ __forceinline__ int floor_index(double v, double &floor_v) {
+    const double t = __dadd_rd(v, 0x1p52);
+    floor_v = __dsub_rn(t, 0x1p52);
+    return __double2loint(t);
+}
 constexpr double kRcpPi = 1.0 / kPi, kRcpTwoPi = 1.0 / kTwoPi, kEightPi = 8. * kPi, kRcpEightPi = 1.0 / kEightPi;
 
 __device__ __forceinline__ double rapidity(V4 a) {
@@ -101,8 +107,15 @@ __host__ __device__ __forceinline__ U4 philox4x32_10(U4 ctr, uint32_t k0, uint32
 
 // 53 random bits -> [0, 1): (hi << 21 | lo >> 11) * 2^-53
 __host__ __device__ __forceinline__ double u53(uint32_t hi, uint32_t lo) {
+#ifdef __CUDA_ARCH__
+    // the same 53 bits without a 64-bit conversion: hi as the low word of
+    // 2^52 + hi, lo >> 11 as that of 2^31 + (lo >> 11) 2^-21; both sums exact
+    const double a = __hiloint2double(0x43300000, static_cast<int>(hi)) - (0x1p52 + 0x1p31);
+    return (a + __hiloint2double(0x41e00000, static_cast<int>(lo >> 11))) * 0x1p-32;
+#else
     const uint64_t bits = (static_cast<uint64_t>(hi) << 21) | (lo >> 11);
     return static_cast<double>(bits) * 0x1.0p-53;
+#endif
 }
 
 // Uniforms 2q and 2q+1 of point `k` of stream `stream`.

@@ -171,6 +171,7 @@ struct chili_ctx {
     RoundCtl *ctl_host = nullptr;  // pinned, two records: the round, the PreProcess count
     long long *iter_host = nullptr;  // pinned, the queued rounds' state (k_iter_init)
     IterAcc *acc_host = nullptr;     // pinned, the iteration's accumulator
+    chili_stats *stats_host = nullptr;  // pinned, a fused Vegas iteration's StatsData
     DevBuf iter_ctl;                 // device copy of that state
     double accept_rate = 0.5, nan_rate = 0.0;
     DevBuf rec, ctl3;

@@ -35,9 +35,10 @@ inline void set_cut_bounds(IntegrandDesc &f) {
     f.sure[2] = r > 3.0 ? -1.0 : (1.0 - std::cos(r)) * (1.0 - 1e-6) - 1e-9;
 }
 
-// f(x) = N [exp(-|x-a|^2/s^2) + exp(-|x-b|^2/s^2)]; params {s, N, a[D], b[D]}.
-__device__ __forceinline__ double camel(const IntegrandDesc *__restrict__ f, const double *x, int dims) {
-    const double s = f->p[0], norm = f->p[1];
+// f(x) = N [exp(-|x-a|^2/s^2) + exp(-|x-b|^2/s^2)]; params {s, N, a[D], b[D]};
+// s2 = s^2 and its reciprocal given (once per thread, not per point).
+__device__ __forceinline__ double camel(const IntegrandDesc *__restrict__ f, const double *x, int dims, double s2,
+                                        double rs2) {
     double d1 = 0, d2 = 0;
     for (int i = 0; i < dims; ++i) {
         double t = x[i] - f->p[2 + i];
@@ -45,8 +46,7 @@ __device__ __forceinline__ double camel(const IntegrandDesc *__restrict__ f, con
         t = x[i] - f->p[2 + dims + i];
         d2 += t * t;
     }
-    const double s2 = s * s;
-    return norm * (exp(-d1 / s2) + exp(-d2 / s2));
+    return f->p[1] * (exp(div_by(-d1, s2, rs2)) + exp(div_by(-d2, s2, rs2)));
 }
 
 // Pair Breit-Wigner sum (or product of the two largest) times the t-channel

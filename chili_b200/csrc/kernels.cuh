@@ -141,11 +141,25 @@ __global__ void k_grid_split(const double *__restrict__ g_old, double *__restric
 }
 
 // ------------------------------------------------------------- plain VEGAS
+// Dynamic shared memory of a block's points: its histogram, and (where both
+// fit 48 KB) the grid's edges behind it.
+__host__ __device__ inline bool vegas_stages_grid(int dims, int bins) {
+    return sizeof(double) * dims * (2 * bins + 1) <= 48 * 1024;
+}
+
 // One Vegas::operator() over n points (grid-stride).  Histogram in shared
 // memory when it fits (smem_hist), else global atomics into hist.
 // DIMS > 0: the dimension fixed at compile time (coordinates in registers);
-// DIMS == 0: `dims` at run time (a local array).
-template <int DIMS>
+// DIMS == 0: `dims` at run time (a local array).  STAGE: the edges in shared
+// memory behind the histogram; on a monotone grid FindBin of a mapped point
+// is then the bin it was mapped through whenever e[bin] < x <= e[bin + 1] (the
+// lower_bound of x is unique), and the binary search, six dependent loads per
+// dimension, is left to the other points.  A whole adapting call of 1e5 4-d
+// points 71 -> 52 us, of 3e6 228 -> 152 us (16 dims, 128 bins: 757 -> 409 us)
+// together with the folds' loads in flight and the StatsData written to host
+// memory by the kernel; latency bound below 1e5 points (launch, two folds
+// behind the points, adaptation), by issue above.
+template <int DIMS, bool STAGE>
 __device__ __forceinline__ void vegas_points(const double *__restrict__ g, int dims_rt, int bins, uint64_t seed,
                                              uint64_t ctr0, const double *__restrict__ u_in, long long n,
                                              const IntegrandDesc *__restrict__ f, double *__restrict__ part,
@@ -155,22 +169,59 @@ __device__ __forceinline__ void vegas_points(const double *__restrict__ g, int d
     const int nh = dims * bins;
     if (smem_hist)
         for (int k = threadIdx.x; k < nh; k += blockDim.x) sh[k] = 0.0;
-    __syncthreads();
+    bool monotone = false;
+    if constexpr (STAGE) {
+        double *es = sh + nh;
+        int bad = 0;
+        for (int d = 0; d < dims; ++d)
+            for (int k = threadIdx.x; k <= bins; k += blockDim.x) {
+                const double e = __ldg(g + d * (bins + 1) + k);
+                es[d * (bins + 1) + k] = e;
+                bad |= k < bins && !(e <= __ldg(g + d * (bins + 1) + k + 1));
+            }
+        monotone = !__syncthreads_or(bad);
+    } else {
+        __syncthreads();
+    }
     double* H = smem_hist ? sh : hist;
+    const double fb = static_cast<double>(bins), s2 = f->p[0] * f->p[0], rs2 = 1. / s2;
     double cnt = 0, sum = 0, sum2 = 0, mn = 1.7976931348623157e308, mx = 2.2250738585072014e-308, nf = 0;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         double r[DIMS > 0 ? DIMS : CHILI_MAX_DIMS];
+        int bin[DIMS > 0 ? DIMS : CHILI_MAX_DIMS];
         if (u_in) {
 #pragma unroll
             for (int d = 0; d < dims; ++d) r[d] = __ldg(u_in + i * dims + d);
         } else {
             load_uniforms(seed, ctr0 + i, nullptr, dims, r);
         }
-        double jac;
-        double val;
-        if (grid_map_checked(g, dims, bins, r, jac)) val = camel(f, r, dims) * jac;
-        else val = CUDART_NAN;
+        // AdaptiveMap::operator() (AdaptiveMap.cc:40-56), as grid_map_checked
+        double jac = 1.0;
+        bool ok = true;
+#pragma unroll
+        for (int d = 0; d < dims; ++d) {
+            const double pos = __dmul_rn(r[d], fb);
+            ok = ok && pos >= 0.0 && pos < fb;  // the dimensions after a uniform outside keep their uniforms
+            bin[d] = -2;
+            if (ok) {
+                double whole;
+                const int idx = floor_index(pos, whole);
+                double left, right;
+                if constexpr (STAGE) {
+                    left = sh[nh + d * (bins + 1) + idx];
+                    right = sh[nh + d * (bins + 1) + idx + 1];
+                } else {
+                    left = __ldg(g + d * (bins + 1) + idx);
+                    right = __ldg(g + d * (bins + 1) + idx + 1);
+                }
+                const double size = __dsub_rn(right, left);
+                r[d] = __dadd_rn(left, __dmul_rn(__dsub_rn(pos, whole), size));
+                jac = __dmul_rn(jac, __dmul_rn(size, fb));
+                if (monotone && left < r[d] && r[d] <= right) bin[d] = idx;
+            }
+        }
+        const double val = ok ? camel(f, r, dims, s2, rs2) * jac : CUDART_NAN;
         const double val2 = val * val;
         cnt += 1;
         sum += val;
@@ -180,7 +231,7 @@ __device__ __forceinline__ void vegas_points(const double *__restrict__ g, int d
         nf += (val != 0);
 #pragma unroll
         for (int j = 0; j < dims; ++j) {
-            const int b = find_bin(g + j * (bins + 1), bins, r[j]);
+            const int b = bin[j] >= 0 ? bin[j] : find_bin(g + j * (bins + 1), bins, r[j]);
             const int s = j * bins + b;
             if (s >= 0) atomicAdd(H + s, val2);
         }
@@ -211,26 +262,37 @@ __device__ __forceinline__ void vegas_points(const double *__restrict__ g, int d
     }
 }
 
-template <int DIMS>
+template <int DIMS, bool STAGE>
 __global__ void k_vegas_iter(const double *__restrict__ g, int dims_rt, int bins, uint64_t seed, uint64_t ctr0,
                              const double *__restrict__ u_in, long long n, const IntegrandDesc *__restrict__ f,
                              double *__restrict__ part, double *__restrict__ hist, int smem_hist) {
-    vegas_points<DIMS>(g, dims_rt, bins, seed, ctr0, u_in, n, f, part, hist, smem_hist);
+    vegas_points<DIMS, STAGE>(g, dims_rt, bins, seed, ctr0, u_in, n, f, part, hist, smem_hist);
 }
 
 // Materialised VEGAS points on the camel: point i's uniforms (the counter
 // stream of k_vegas_iter, ctr0 + i) through the grid, x_out[i][dims] and the
 // point's weight f(x) J(u) to w_out[i].  The grid (dims x (bins+1) edges) is
-// staged in shared memory; a block's points are assembled in shared memory
-// and leave as contiguous 16-byte stores, so the only HBM traffic is the
-// 8 (dims + 1) bytes written per point.  Persistent grid-stride over tiles
-// of kGenTile points.
+// staged in shared memory, so the only HBM traffic is the 8 (dims + 1) bytes
+// written per point.  Persistent grid-stride over tiles of kGenTile points.
 // DIMS > 0 fixes the dimension at compile time (the point's coordinates stay
 // in registers); DIMS == 0 takes `dims` at run time (a local array).  PPT
 // points per thread (independent dependency chains the scheduler overlaps):
-// a tile is kGenTile * PPT points.
+// a tile is kGenTile * PPT points.  ROW: a point's row leaves straight from
+// its thread, as 32-byte (dims a multiple of 4) or 16-byte stores (even dims)
+// on aligned buffers; the other rows are assembled in shared memory and leave
+// as contiguous 16-byte stores.
+// Bound by instruction issue (two Philox blocks, two exponentials; 450 issued
+// instructions per 4-d point before).  2e7 4-d points: 0.319 ms with every row
+// assembled in shared memory (half of its wavefronts bank conflicts), integer
+// and double conversions and two divisions; 0.276 ms with rows from the
+// threads, conversions through 2^52 and a reciprocal; 3e6 16-d points 244 ->
+// 168 us.  The stores alone take 0.122 ms.
 constexpr int kGenTile = 256;
-template <int DIMS, int PPT>
+__device__ __forceinline__ void store_row4(double *p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+template <int DIMS, int PPT, bool ROW>
 __global__ void __launch_bounds__(kGenTile) k_vegas_generate(const double *__restrict__ g, int dims_rt, int bins,
                                                              uint64_t seed, uint64_t ctr0, long long n,
                                                              const IntegrandDesc *__restrict__ f,
@@ -239,11 +301,11 @@ __global__ void __launch_bounds__(kGenTile) k_vegas_generate(const double *__res
     constexpr int kTile = kGenTile * PPT;
     const int dims = DIMS > 0 ? DIMS : dims_rt;
     const int ne = dims * (bins + 1);
-    double *xt = gsh + ((ne + 1) & ~1);  // kTile * dims x values, 16-byte aligned
+    double *xt = gsh + ((ne + 1) & ~1);  // kTile * dims x values, 16-byte aligned (ROW: none)
     double *wt = xt + kTile * dims;      // kTile weights
     for (int k = threadIdx.x; k < ne; k += blockDim.x) gsh[k] = g[k];
     __syncthreads();
-    const double fb = static_cast<double>(bins);
+    const double fb = static_cast<double>(bins), s2 = f->p[0] * f->p[0], rs2 = 1. / s2;
     const long long ntiles = (n + kTile - 1) / kTile;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const long long i0 = t * kTile;
@@ -261,39 +323,56 @@ __global__ void __launch_bounds__(kGenTile) k_vegas_generate(const double *__res
 #pragma unroll
                 for (int d = 0; d < dims; ++d) {
                     const double pos = __dmul_rn(r[d], fb);
-                    if (!(pos >= 0.0 && pos < fb)) {
-                        ok = false;
-                        break;
-                    }
-                    const int idx = static_cast<int>(pos);
-                    const double loc = __dsub_rn(pos, static_cast<double>(idx));
+                    ok = ok && pos >= 0.0 && pos < fb;
+                    double whole;
+                    const int idx = floor_index(ok ? pos : 0.0, whole);
                     const double *e = gsh + d * (bins + 1);
                     const double left = e[idx];
                     const double size = __dsub_rn(e[idx + 1], left);
-                    r[d] = __dadd_rn(left, __dmul_rn(loc, size));
+                    r[d] = __dadd_rn(left, __dmul_rn(__dsub_rn(pos, whole), size));
                     jac = __dmul_rn(jac, __dmul_rn(size, fb));
                 }
-                const double w = ok ? camel(f, r, dims) * jac : CUDART_NAN;
+                double w = camel(f, r, dims, s2, rs2) * jac;
+                if (!ok) {
+                    w = CUDART_NAN;
 #pragma unroll
-                for (int d = 0; d < dims; ++d) xt[l * dims + d] = ok ? r[d] : CUDART_NAN;
-                wt[l] = w;
+                    for (int d = 0; d < dims; ++d) r[d] = CUDART_NAN;
+                }
+                if constexpr (ROW) {
+                    double *o = x_out + (i0 + l) * DIMS;
+                    if constexpr (DIMS % 4 == 0) {
+#pragma unroll
+                        for (int d = 0; d < DIMS; d += 4) store_row4(o + d, r[d], r[d + 1], r[d + 2], r[d + 3]);
+                    } else {
+#pragma unroll
+                        for (int d = 0; d < DIMS; d += 2)
+                            reinterpret_cast<double2 *>(o)[d / 2] = make_double2(r[d], r[d + 1]);
+                    }
+                    w_out[i0 + l] = w;
+                } else {
+#pragma unroll
+                    for (int d = 0; d < dims; ++d) xt[l * dims + d] = r[d];
+                    wt[l] = w;
+                }
             }
         }
-        __syncthreads();
-        // the tile's rows are contiguous in x_out: cnt * dims doubles from
-        // i0 * dims, written as double2 where both ends allow it
-        double *xo = x_out + i0 * dims;
-        const int nx = cnt * dims;
-        const bool vec = ((reinterpret_cast<uintptr_t>(xo) & 15) == 0) && ((nx & 1) == 0);
-        if (vec) {
-            const double2 *src = reinterpret_cast<const double2 *>(xt);
-            double2 *dst = reinterpret_cast<double2 *>(xo);
-            for (int k = threadIdx.x; k < (nx >> 1); k += blockDim.x) dst[k] = src[k];
-        } else {
-            for (int k = threadIdx.x; k < nx; k += blockDim.x) xo[k] = xt[k];
+        if constexpr (!ROW) {
+            __syncthreads();
+            // the tile's rows are contiguous in x_out: cnt * dims doubles from
+            // i0 * dims, written as double2 where both ends allow it
+            double *xo = x_out + i0 * dims;
+            const int nx = cnt * dims;
+            const bool vec = ((reinterpret_cast<uintptr_t>(xo) & 15) == 0) && ((nx & 1) == 0);
+            if (vec) {
+                const double2 *src = reinterpret_cast<const double2 *>(xt);
+                double2 *dst = reinterpret_cast<double2 *>(xo);
+                for (int k = threadIdx.x; k < (nx >> 1); k += blockDim.x) dst[k] = src[k];
+            } else {
+                for (int k = threadIdx.x; k < nx; k += blockDim.x) xo[k] = xt[k];
+            }
+            for (int k = threadIdx.x; k < cnt; k += blockDim.x) w_out[i0 + k] = wt[k];
+            __syncthreads();
         }
-        for (int k = threadIdx.x; k < cnt; k += blockDim.x) w_out[i0 + k] = wt[k];
-        __syncthreads();
     }
 }
 
@@ -340,29 +419,42 @@ __global__ void k_vegas_finalize(const double *__restrict__ part, int nblocks, c
 // Ordered fold of the partials of blocks [b0, b1) (StatsData with Kahan sums,
 // histogram bin by bin) into one partial: out6 and out_hist[nh].  The
 // partials were written by other blocks of the same launch: read from L2.
+// ps: 6 doubles per partial of shared memory (the StatsData partials are
+// loaded by all threads at once; thread 0 loading them one after the other
+// took longer than the histogram).
 __device__ __forceinline__ void vegas_fold_range(const double *part, const double *hist_part, int b0, int b1, int nh,
-                                                 double *__restrict__ out_hist, double *__restrict__ out6) {
+                                                 double *__restrict__ out_hist, double *__restrict__ out6,
+                                                 double *ps) {
+    for (int k = threadIdx.x; k < 6 * (b1 - b0); k += blockDim.x) ps[k] = __ldcg(part + b0 * 6 + k);
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
         double s = 0;
-        for (int b = b0; b < b1; ++b) s += __ldcg(hist_part + static_cast<size_t>(b) * nh + k);
+        for (int b = b0; b < b1; b += 16) {
+            double v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = b + q < b1 ? __ldcg(hist_part + static_cast<size_t>(b + q) * nh + k) : 0.0;
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+                if (b + q < b1) s += v[q];
+        }
         out_hist[k] = s;
     }
+    __syncthreads();
     if (threadIdx.x == 0) {
         double n = 0, mn = 1.7976931348623157e308, mx = 2.2250738585072014e-308, sum = 0, csum = 0, sum2 = 0,
                csum2 = 0, nf = 0;
         for (int b = b0; b < b1; ++b) {
-            const double *p = part + b * 6;
-            n += __ldcg(p);
-            mn = std_min(mn, __ldcg(p + 1));
-            mx = std_max(mx, __ldcg(p + 2));
-            double y = __ldcg(p + 3) - csum, t = sum + y;  // Kahan
+            const double *p = ps + (b - b0) * 6;
+            n += p[0];
+            mn = std_min(mn, p[1]);
+            mx = std_max(mx, p[2]);
+            double y = p[3] - csum, t = sum + y;  // Kahan
             csum = (t - sum) - y;
             sum = t;
-            y = __ldcg(p + 4) - csum2;
+            y = p[4] - csum2;
             t = sum2 + y;
             csum2 = (t - sum2) - y;
             sum2 = t;
-            nf += __ldcg(p + 5);
+            nf += p[5];
         }
         out6[0] = n; out6[1] = mn; out6[2] = mx; out6[3] = sum; out6[4] = sum2; out6[5] = nf;
     }
@@ -380,14 +472,16 @@ __device__ __forceinline__ void vegas_fold_range(const double *part, const doubl
 // completes them; no block waits for another.  The fixed grouping keeps the
 // sums deterministic.
 constexpr int kStepGroup = 16;
-template <int DIMS>
+constexpr int kMaxStepGroups = 64;  // groups of an iteration's blocks (148 SMs: 592 blocks, 37 groups)
+template <int DIMS, bool STAGE>
 __global__ void k_vegas_step(const double *__restrict__ g, double *__restrict__ g_new, int dims_rt, int bins,
                              uint64_t seed, uint64_t ctr0, const double *__restrict__ u_in, long long n,
                              const IntegrandDesc *__restrict__ f, double *part, double *hist_part, double *gpart,
                              double *ghist, double *__restrict__ train, double *__restrict__ out6, double alpha,
                              int adapt, unsigned *__restrict__ arrive, int *__restrict__ status) {
     extern __shared__ double sh[];
-    vegas_points<DIMS>(g, dims_rt, bins, seed, ctr0, u_in, n, f, part, hist_part, 1);
+    __shared__ double ps[6 * kMaxStepGroups];
+    vegas_points<DIMS, STAGE>(g, dims_rt, bins, seed, ctr0, u_in, n, f, part, hist_part, 1);
     const int dims = DIMS > 0 ? DIMS : dims_rt;
     const int nh = dims * bins;
     const int grp = blockIdx.x / kStepGroup, ngrp = (gridDim.x + kStepGroup - 1) / kStepGroup;
@@ -399,7 +493,7 @@ __global__ void k_vegas_step(const double *__restrict__ g, double *__restrict__ 
     __syncthreads();
     if (!last) return;
     __threadfence();
-    vegas_fold_range(part, hist_part, b0, b1, nh, ghist + static_cast<size_t>(grp) * nh, gpart + grp * 6);
+    vegas_fold_range(part, hist_part, b0, b1, nh, ghist + static_cast<size_t>(grp) * nh, gpart + grp * 6, ps);
     if (threadIdx.x == 0) arrive[1 + grp] = 0u;
     __threadfence();  // the group partial visible before the group's arrival
     __syncthreads();
@@ -407,7 +501,7 @@ __global__ void k_vegas_step(const double *__restrict__ g, double *__restrict__ 
     __syncthreads();
     if (!last) return;
     __threadfence();
-    vegas_fold_range(gpart, ghist, 0, ngrp, nh, train, out6);
+    vegas_fold_range(gpart, ghist, 0, ngrp, nh, train, out6, ps);
     __syncthreads();  // train complete (and the points' shared histogram no longer needed)
     if (adapt) {
         // one warp per dimension (each with its own scratch in shared

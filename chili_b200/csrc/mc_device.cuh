@@ -105,8 +105,9 @@ __device__ __forceinline__ bool grid_map_checked(const double *__restrict__ g, i
     for (int d = 0; d < dims; ++d) {
         const double pos = __dmul_rn(x[d], fb);
         if (!(pos >= 0.0 && pos < fb)) return false;
-        const int idx = static_cast<int>(pos);
-        const double loc = __dsub_rn(pos, static_cast<double>(idx));
+        double whole;
+        const int idx = floor_index(pos, whole);
+        const double loc = __dsub_rn(pos, whole);
         const double *e = g + d * (bins + 1);
         const double left = __ldg(e + idx);
         const double size = __dsub_rn(__ldg(e + idx + 1), left);
