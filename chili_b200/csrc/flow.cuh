@@ -334,6 +334,24 @@ __device__ __forceinline__ void load_row32(const uint8_t *tile, int R, int r, in
     }
 }
 
+// The same 32 columns as packed pairs; and v[j] times the leaky ReLU's slope
+// at such a column's value.
+__device__ __forceinline__ void load_packed32(const uint8_t *tile, int R, int r, int c0, uint4 (&v)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = *reinterpret_cast<const uint4 *>(tile + sw128_off(r, c0 + 8 * q, R));
+}
+__device__ __forceinline__ void lrelu_slopes(const uint4 (&h)[4], float (&v)[32]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint32_t w[4] = {h[q].x, h[q].y, h[q].z, h[q].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[8 * q + 2 * i] *= bf16_lo(w[i]) > 0.f ? 1.f : kSlope;
+            v[8 * q + 2 * i + 1] *= bf16_hi(w[i]) > 0.f ? 1.f : kSlope;
+        }
+    }
+}
+
 // Cooperative copy of `bytes` (a multiple of 16 * blockDim.x) between
 // 16-byte aligned buffers.
 __device__ __forceinline__ void copy_block(void *dst, const void *src, int bytes) {
@@ -367,6 +385,9 @@ struct LayerArgs {
 // epilogues, group j evaluates the spline of dimension j.
 constexpr int kFwdGroups = 5;
 constexpr int kFwdThreads = 128 * kFwdGroups;
+// Issues and awaits the bulk copies of saved tiles: of the fifth group, which
+// has no part in the epilogues (thread 0 issues the products).
+constexpr int kCopyThread = 512;
 constexpr int kFwdSmem = kW1Bytes + kW2Bytes + kW3FBytes + 128 * 64 * 2 + kHTile + (kFwdGroups - 1) * 128 * 4 +
                          kMaxDA * 128 * 4 + 128 * 4 + 64 + 1024;
 
@@ -548,7 +569,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_flow_layer(LayerArgs a) {
             for (int k = 0; k < 8; ++k) mma_bf16(tbase, desc_k(aH, 128, 16 * k), desc_k(aW2, 128, 16 * k), id_h, k > 0);
             mma_commit(bar + 2);
         }
-        if (SAVE && cur) copy_block(a.h1s + tile * kHTile, sH, kHTile);
+        if (SAVE && cur && t == kCopyThread) {
+            bulk_s2g(a.h1s + tile * kHTile, sH, kHTile);
+            bulk_commit();
+        }
         float lsum = 0.f;
         if (due) {
             if (grp < DB) {
@@ -562,7 +586,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_flow_layer(LayerArgs a) {
         if (cur) {
             ok = mbar_wait(bar + 2, phase, kWaitLimit) && ok;
             tc_fence_after();
-            if (SAVE) __syncthreads();  // the copy of h1 is complete before h2 overwrites it
+            if (SAVE) {  // the copy has read h1 before h2 overwrites it
+                if (t == kCopyThread) bulk_wait_read();
+                __syncthreads();
+            }
             epilogue();                 // h2's accumulator reuses h1's columns
         }
         cp_async_wait_all();  // the next tile's copies of this thread, before the barrier publishes them
@@ -587,9 +614,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_flow_layer(LayerArgs a) {
         prow = tile * 128 + r;
         xsp = (prow < n && grp < DB) ? a.xin[dsp * n + prow] : 0.5f;
         lq0 = (prow < n && grp == 0) ? a.logq[prow] : 0.f;
-        if (SAVE) copy_block(a.h2s + tile * kHTile, sH, kHTile);
+        if (SAVE && t == kCopyThread) {
+            bulk_s2g(a.h2s + tile * kHTile, sH, kHTile);
+            bulk_commit();
+        }
         tile += step;
         if (tile < ntiles) build_a(tile);
+        if (SAVE && t == kCopyThread) bulk_wait_read();  // h2 is read before the next tile's h1 overwrites it
         tc_fence_before();
         run = __syncthreads_and(ok);
         if (run && tile < ntiles) {
@@ -599,6 +630,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_flow_layer(LayerArgs a) {
         if (!run) mbar_wait(bar + 3, phase, kWaitLimit);  // the third product's end, before its memory is released
         phase ^= 1;
     }
+    if (SAVE && t == kCopyThread) bulk_wait();
     if (!ok && t == 0) atomicExch(a.err, 1);
     // every issued MMA has been waited for (or the wait gave up): release TMEM
     tc_fence_before();
@@ -628,8 +660,12 @@ struct BwdArgs {
 
 // Five thread groups of 128 (one thread per point each, as in the forward
 // kernel): group j runs the spline backward of dimension j; groups 0-3 split
-// the epilogues' 128 hidden columns. The g_a partials of groups 1-3 reuse the
-// g_theta tile's memory once its product and copy are done.
+// the epilogues' 128 hidden columns and g_a's 16.  The saved tiles leave
+// shared memory by bulk copies, h2 and h1 are loaded behind the products, and
+// g_a is a third product.  With the tiles copied by all threads, h loaded when
+// needed and g_a on the CUDA cores (1100 of about 3800 instructions a thread)
+// a 65536-point layer took 100 us; so 74 us.  Bound by the issue of the spline
+// backward (two-byte stores of its 49 gradients) and the chain of the products.
 constexpr int kBwdGroups = 5;
 constexpr int kBwdThreads = 128 * kBwdGroups;
 constexpr int kBwdSmem = kWBytes + kGTile + kHTile + 64 + 1024;
@@ -642,7 +678,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_flow_layer_bwd(BwdArgs a) {
     uint8_t *sW1 = sm, *sW2 = sm + kW1Bytes, *sW3 = sm + kW1Bytes + kW2Bytes;
     uint8_t *sG = sm + kWBytes;
     uint8_t *sP = sG + kGTile;
-    float *sGA = reinterpret_cast<float *>(sG);  // [3][16][128] g_a partials of groups 1-3 (after g_theta's use)
     uint64_t *bar = reinterpret_cast<uint64_t *>(sP + kHTile);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 2);
     const int t = threadIdx.x, wp = t >> 5;
@@ -666,8 +701,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_flow_layer_bwd(BwdArgs a) {
         bulk_g2s(sm, a.L.wt, kWBytes, bar);
     }
     bool ok = mbar_wait(bar, 0, kWaitLimit);
-    const uint32_t aW2 = smem_u32(sW2), aW3 = smem_u32(sW3), aG = smem_u32(sG), aP = smem_u32(sP);
+    const uint32_t aW1 = smem_u32(sW1), aW2 = smem_u32(sW2), aW3 = smem_u32(sW3), aG = smem_u32(sG), aP = smem_u32(sP);
     constexpr uint32_t id_mn = idesc_bf16(128, 128, false, true);
+    constexpr uint32_t id_ga = idesc_bf16(128, 64, false, true);  // W1's 64 columns; g_a is the first da
     uint32_t phase = 0;
     const int da = a.L.da;
     // the group that zeroes g_theta's padding columns DB*49 .. 255
@@ -692,6 +728,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_flow_layer_bwd(BwdArgs a) {
         if (grp == kPadGroup)
             for (int col = DB * kPerDim; col < kP; ++col)
                 *reinterpret_cast<uint16_t *>(sG + sw128_off(r, col, 128)) = 0;
+        if (t == kCopyThread) bulk_wait_read();  // the previous tile's g_p1, before sP is written again
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -702,22 +739,24 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_flow_layer_bwd(BwdArgs a) {
                 mma_bf16(tbase, desc_k(aG, 128, 16 * k), desc_mn(aW3, kP, 16 * k), id_mn, k > 0);
             mma_commit(bar + 1);
         }
-        copy_block(a.gths + tile * kGTile, sG, kGTile);
+        if (t == kCopyThread) {
+            bulk_s2g(a.gths + tile * kGTile, sG, kGTile);
+            bulk_commit();
+        }
+        uint4 hv[4];  // this group's 32 columns of h2, then of h1, loaded behind the products
+        if (grp < 4) load_packed32(a.h2s + tile * kHTile, 128, r, 32 * grp, hv);
         ok = mbar_wait(bar + 1, phase, kWaitLimit) && ok;
         phase ^= 1;
         tc_fence_after();
         // g_p2 = g_h2 * lrelu'(h2), unit 127 -> 0; groups 0-3, 32 columns each
         if (grp < 4) {
-            const uint8_t *h2t = a.h2s + tile * kHTile;
             const int c0 = 32 * grp;
-            float v[32], hv[32];
+            float v[32];
             tmem_ld32(lane_addr + c0, v);
-            load_row32(h2t, 128, r, c0, hv);
+            lrelu_slopes(hv, v);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                v[j] *= hv[j] > 0.f ? 1.f : kSlope;
+            for (int j = 0; j < 32; ++j)
                 if (c0 + j == kH - 1 || !valid) v[j] = 0.f;
-            }
             store_row32(sP, 128, r, c0, v);
         }
         fence_async_smem();
@@ -729,62 +768,61 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_flow_layer_bwd(BwdArgs a) {
             for (int k = 0; k < 8; ++k) mma_bf16(tbase, desc_k(aP, 128, 16 * k), desc_mn(aW2, 128, 16 * k), id_mn, k > 0);
             mma_commit(bar + 1);
         }
-        copy_block(a.gp2s + tile * kHTile, sP, kHTile);
+        if (t == kCopyThread) {
+            bulk_s2g(a.gp2s + tile * kHTile, sP, kHTile);
+            bulk_commit();
+        }
+        if (grp < 4) load_packed32(a.h1s + tile * kHTile, 128, r, 32 * grp, hv);
         ok = mbar_wait(bar + 1, phase, kWaitLimit) && ok;
         phase ^= 1;
         tc_fence_after();
-        __syncthreads();  // the copies of g_theta and g_p2 are complete before their tiles are reused
-        // g_p1 = g_h1 * lrelu'(h1); g_a = bf16(g_p1) W1 on the CUDA cores,
-        // this group's 32 units
-        float ga[kMaxDA];
-#pragma unroll
-        for (int i = 0; i < kMaxDA; ++i) ga[i] = 0.f;
+        if (t == kCopyThread) bulk_wait_read();
+        __syncthreads();  // g_theta and g_p2 are read before their tiles are reused
+        // g_p1 = g_h1 * lrelu'(h1); g_a = bf16(g_p1) W1
         if (grp < 4) {
-            const uint8_t *h1t = a.h1s + tile * kHTile;
             const int c0 = 32 * grp;
-            float v[32], hv[32];
+            float v[32];
             tmem_ld32(lane_addr + c0, v);
-            load_row32(h1t, 128, r, c0, hv);
+            lrelu_slopes(hv, v);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                v[j] *= hv[j] > 0.f ? 1.f : kSlope;
+            for (int j = 0; j < 32; ++j)
                 if (c0 + j == kH - 1 || !valid) v[j] = 0.f;
-            }
             store_row32(sP, 128, r, c0, v);
-#pragma unroll 4
-            for (int j = 0; j < 32; ++j) {
-                const int hcol = c0 + j;
-                const float gq = bf16_hi(pack_bf16x2(0.f, v[j]));
-                // W1[hcol][0..15]: two 16-byte chunks of row hcol of the W1 tile
-                const uint4 w0 = *reinterpret_cast<const uint4 *>(sW1 + sw128_off(hcol, 0, 128));
-                const uint4 w1 = *reinterpret_cast<const uint4 *>(sW1 + sw128_off(hcol, 8, 128));
-                ga[0] += gq * bf16_lo(w0.x); ga[1] += gq * bf16_hi(w0.x);
-                ga[2] += gq * bf16_lo(w0.y); ga[3] += gq * bf16_hi(w0.y);
-                ga[4] += gq * bf16_lo(w0.z); ga[5] += gq * bf16_hi(w0.z);
-                ga[6] += gq * bf16_lo(w0.w); ga[7] += gq * bf16_hi(w0.w);
-                ga[8] += gq * bf16_lo(w1.x); ga[9] += gq * bf16_hi(w1.x);
-                ga[10] += gq * bf16_lo(w1.y); ga[11] += gq * bf16_hi(w1.y);
-                ga[12] += gq * bf16_lo(w1.z); ga[13] += gq * bf16_hi(w1.z);
-                ga[14] += gq * bf16_lo(w1.w); ga[15] += gq * bf16_hi(w1.w);
-            }
-            if (grp > 0) {
-#pragma unroll
-                for (int i = 0; i < kMaxDA; ++i) sGA[((grp - 1) * kMaxDA + i) * 128 + r] = ga[i];
-            }
         }
+        fence_async_smem();
+        tc_fence_before();
         __syncthreads();
-        copy_block(a.gp1s + tile * kHTile, sP, kHTile);
-        if (grp == 0 && valid) {
+        if (t == 0) {
+            tc_fence_after();
 #pragma unroll
-            for (int i = 0; i < kMaxDA; ++i)
-                if (i < da) {
-                    const int d = a.L.cond[i];
-                    const float s3 = sGA[i * 128 + r] + sGA[(kMaxDA + i) * 128 + r] + sGA[(2 * kMaxDA + i) * 128 + r];
-                    a.gin[d * n + row] = (a.gout ? a.gout[d * n + row] : 0.f) + 2.f * (ga[i] + s3);
-                }
+            for (int k = 0; k < 8; ++k) mma_bf16(tbase, desc_k(aP, 128, 16 * k), desc_mn(aW1, 128, 16 * k), id_ga, k > 0);
+            mma_commit(bar + 1);
+        }
+        if (t == kCopyThread) {
+            bulk_s2g(a.gp1s + tile * kHTile, sP, kHTile);
+            bulk_commit();
+        }
+        float gp[4];  // the pass-through part of the input's gradient
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = 4 * grp + q;
+            gp[q] = (a.gout && valid && i < da) ? a.gout[a.L.cond[i] * n + row] : 0.f;
+        }
+        ok = mbar_wait(bar + 1, phase, kWaitLimit) && ok;
+        phase ^= 1;
+        tc_fence_after();
+        if (grp < 4) {
+            float ga[4];
+            tmem_ld4(lane_addr + 4 * grp, ga);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = 4 * grp + q;
+                if (i < da && valid) a.gin[a.L.cond[i] * n + row] = gp[q] + 2.f * ga[q];
+            }
         }
         tc_fence_before();
     }
+    if (t == kCopyThread) bulk_wait();
     if (!ok && t == 0) atomicExch(a.err, 2);
     tc_fence_before();
     __syncthreads();
@@ -860,31 +898,38 @@ __global__ void __launch_bounds__(128, 1) k_flow_wgrad(WgradArgs a) {
             if (srcB) bulk_g2s(sB[s], srcB + tile * strideB, bbytes, bar + s);
         }
     };
+    // product 2: this thread's row of a tile, all loads in flight at once and
+    // a tile ahead (loaded one after the other at the tile's start they set the
+    // kernel's time: 73 us for 65536 points, so 37.6)
+    float bx[kMaxDA];
+    int bc = 0;
+    bool bvalid = false;  // the row is not past the end
+    auto load_rows = [&](long long tl) {
+        const long long row = tl * 128 + t;
+        bvalid = row < n;
+        bc = bvalid ? a.ch[row] : 0;
+#pragma unroll
+        for (int i = 0; i < kMaxDA; ++i) bx[i] = bvalid && i < a.da ? a.xin[a.cond[i] * n + row] : 0.f;
+    };
     long long tile = blockIdx.x;
     if (tile < ntiles) issue_load(tile, 0);
+    if (p == 2 && tile < ntiles) load_rows(tile);
     int s = 0;
     for (; __syncthreads_and(ok) && tile < ntiles; tile += gridDim.x, s ^= 1) {
         if (p == 2) {
-            // B tile: [a (da columns) | 0 | onehot(c) at column 16 + c], bf16
-            const long long row = tile * 128 + t;
-            const bool valid = row < n;
-            const int c = valid ? a.ch[row] : -1;
+            // B tile: [a (da columns) | 0 | onehot(c) at column 16 + c], bf16,
+            // from the values loaded behind the tile before
             for (int c0 = 0; c0 < ncols; c0 += 32) {
                 float v[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
-                    const int col = c0 + j;
-                    float x = 0.f;
-                    if (valid) {
-                        if (col < a.da)
-                            x = 2.f * fminf(fmaxf(a.xin[a.cond[col] * n + row], 0.f), 1.f) - 1.f;
-                        else if (col == 16 + c)
-                            x = 1.f;
-                    }
-                    v[j] = x;
+                    v[j] = bvalid && c0 + j == 16 + bc ? 1.f : 0.f;
+                    if (j < kMaxDA && c0 == 0 && bvalid && j < a.da)
+                        v[j] = 2.f * fminf(fmaxf(bx[j], 0.f), 1.f) - 1.f;
                 }
                 store_row32(sB[s], 128, t, c0, v);
             }
+            if (tile + gridDim.x < ntiles) load_rows(tile + gridDim.x);
             fence_async_smem();
         }
         ok = mbar_wait(bar + s, ph_load[s], kWaitLimit) && ok;
