@@ -456,19 +456,19 @@ def compact_other_workloads(args, dev, rank):
 # counters for the forward kernel (it runs over every drawn point of a
 # chunk), weighted points for the rest.
 KERNEL_COUNTERS = {
-    "k_mc_forward": {"fp64_ops_per_point": 1868.7, "dram_bytes_per_point": 424.4, "basis": "drawn",
+    "k_mc_forward": {"fp64_ops_per_point": 1506.9, "dram_bytes_per_point": 445.5, "basis": "drawn",
                      "source": "profiles/multichannel_2to4_kernels.md"},
-    "k_pp_nodes": {"fp64_ops_per_point": 24.0, "dram_bytes_per_point": 838.1, "basis": "weighted",
+    "k_pp_nodes": {"fp64_ops_per_point": 24.0, "dram_bytes_per_point": 840.1, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
-    "k_pp_items": {"fp64_ops_per_point": 9343.5, "dram_bytes_per_point": 1316.3, "basis": "weighted",
+    "k_pp_items": {"fp64_ops_per_point": 7453.3, "dram_bytes_per_point": 1332.5, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
-    "k_pp_chains": {"fp64_ops_per_point": 3684.0, "dram_bytes_per_point": 597.0, "basis": "weighted",
+    "k_pp_chains": {"fp64_ops_per_point": 2926.0, "dram_bytes_per_point": 624.6, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
-    "k_pp_channel": {"fp64_ops_per_point": 684.0, "dram_bytes_per_point": 1077.4, "basis": "weighted",
+    "k_pp_channel": {"fp64_ops_per_point": 510.6, "dram_bytes_per_point": 970.5, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
-    "k_pp_combine": {"fp64_ops_per_point": 724.0, "dram_bytes_per_point": 416.2, "basis": "weighted",
+    "k_pp_combine": {"fp64_ops_per_point": 724.0, "dram_bytes_per_point": 415.5, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
-    "k_mc_accum": {"fp64_ops_per_point": 300.0, "dram_bytes_per_point": 32.3, "basis": "weighted",
+    "k_mc_accum": {"fp64_ops_per_point": 252.7, "dram_bytes_per_point": 137.6, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"}
 }
 
