@@ -278,21 +278,38 @@ __device__ __forceinline__ float rqs_backward_st(const float *th, float x, float
         dotw += (scw * gw) * smw[m];
         doth += (sch * gh) * smh[m];
     }
+    const float s0 = sigmoid_f(b.t0), s1 = sigmoid_f(b.t1);
+    auto grad = [&](int i) -> float {  // parameter i's gradient
+        if (i < kBins) {
+            const float gw = (i < b.k ? g_x0 : 0.f) + (i == b.k ? g_wk : 0.f);
+            return smw[i] * (scw * gw - dotw);
+        }
+        if (i < 2 * kBins) {
+            const int m = i - kBins;
+            const float gh = (m < b.k ? g_y0 : 0.f) + (m == b.k ? g_hk : 0.f);
+            return smh[m] * (sch * gh - doth);
+        }
+        const int m = i - 2 * kBins;
+        return (m == b.k ? g_d0 * s0 : 0.f) + (m == b.k + 1 ? g_d1 * s1 : 0.f);
+    };
+    // columns in aligned pairs (a 4-byte store; half the stores and their
+    // address arithmetic), the odd one alone: last of an even c0, first of an odd
     auto put = [&](int col, float v) {
         *reinterpret_cast<uint16_t *>(tile + sw128_off(r, c0 + col, 128)) =
             static_cast<uint16_t>(pack_bf16x2(v, 0.f) & 0xFFFFu);
     };
+    auto put2 = [&](int col, float lo, float hi) {
+        *reinterpret_cast<uint32_t *>(tile + sw128_off(r, c0 + col, 128)) = pack_bf16x2(lo, hi);
+    };
+    if (c0 & 1) {
+        put(0, grad(0));
 #pragma unroll
-    for (int m = 0; m < kBins; ++m) {
-        const float gw = (m < b.k ? g_x0 : 0.f) + (m == b.k ? g_wk : 0.f);
-        const float gh = (m < b.k ? g_y0 : 0.f) + (m == b.k ? g_hk : 0.f);
-        put(m, smw[m] * (scw * gw - dotw));
-        put(kBins + m, smh[m] * (sch * gh - doth));
+        for (int i = 1; i < kPerDim; i += 2) put2(i, grad(i), grad(i + 1));
+    } else {
+#pragma unroll
+        for (int i = 0; i + 1 < kPerDim; i += 2) put2(i, grad(i), grad(i + 1));
+        put(kPerDim - 1, grad(kPerDim - 1));
     }
-    const float s0 = sigmoid_f(b.t0), s1 = sigmoid_f(b.t1);
-#pragma unroll
-    for (int m = 0; m <= kBins; ++m)
-        put(2 * kBins + m, (m == b.k ? g_d0 * s0 : 0.f) + (m == b.k + 1 ? g_d1 * s1 : 0.f));
     return g_xi / b.wk;
 }
 
