@@ -681,8 +681,10 @@ struct BwdArgs {
 // shared memory by bulk copies, h2 and h1 are loaded behind the products, and
 // g_a is a third product.  With the tiles copied by all threads, h loaded when
 // needed and g_a on the CUDA cores (1100 of about 3800 instructions a thread)
-// a 65536-point layer took 100 us; so 74 us.  Bound by the issue of the spline
-// backward (two-byte stores of its 49 gradients) and the chain of the products.
+// a 65536-point layer took 100 us; so 74 us, with the parameter gradients stored
+// in pairs 70.  Bound by the loads of theta at a tile's start (long scoreboard 5.0
+// stalls per issue, issue 36% busy; prefetching the next tile's to L2 gained
+// nothing) and the chain of the products.
 constexpr int kBwdGroups = 5;
 constexpr int kBwdThreads = 128 * kBwdGroups;
 constexpr int kBwdSmem = kWBytes + kGTile + kHTile + 64 + 1024;
