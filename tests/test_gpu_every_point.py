@@ -65,3 +65,17 @@ def test_outputs_are_optional(ctx_factory):
     ctx.call("chili_gpu_multichannel_weight", C.c_void_p(mom.ctypes.data), C.c_void_p(ch.ctypes.data),
              C.c_void_p(alone.ctypes.data), None, None, 300)
     assert np.array_equal(alone, full, equal_nan=True)
+
+
+@pytest.mark.parametrize("n_out,n", [(3, 513), (4, 257), (5, 300), (6, 1001), (4, 262145)])
+def test_both_routes_round_every_point_the_same(ctx_factory, n_out, n):
+    """Every density, weight and event value of the tiled pass has the bits of
+    the per-thread kernel: the running product of a channel's decay weights is
+    divided by 2 pi once per decay (Channel.cc:111) on both, so the bound at
+    every point, cancelling channel sums included, is zero."""
+    ctxs = [_context(ctx_factory, n_out, p) for p in (0, 1)]
+    events = [c.generate(n, seed=29, counter=7) for c in ctxs]
+    for a, b in zip(*events):
+        assert np.array_equal(a, b, equal_nan=True)
+    for a, b in zip(*(c.multichannel_weight(events[0][0], events[0][2]) for c in ctxs)):
+        assert np.array_equal(a, b, equal_nan=True)
