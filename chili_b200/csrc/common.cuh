@@ -45,9 +45,11 @@ __device__ __forceinline__ double dot3(V4 a, V4 b) { return dadd(dadd(dmul(a.x, 
 // Markstein's correction q + (a - q b) rb of q = a rb ("Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34 (1990)) is the correctly rounded quotient (but for about one pair
-// in 2^50, half an ulp by a hair).  Three FP64 operations instead of about
-// ten; quotients outside 2^-962 .. 2^957 (zeros, infinities, NaN among them)
-// take the division.
+// in 2^50, half an ulp by a hair) where nothing underflows: |a| at least
+// 2^-968, so that a - q b is exact, and rb normal.  Three FP64 operations
+// instead of about ten.  Quotients outside 2^-962 .. 2^954 (zeros, infinities,
+// NaN among them) take the division; a smaller |a| over a b below 2^-6 keeps
+// the quotient within an ulp.
 __device__ __forceinline__ double div_by(double a, double b, double rb) {
     const double q = __dmul_rn(a, rb);
     if ((static_cast<uint32_t>(__double2hiint(q)) & 0x7fffffffu) - 0x03d00000u >= 0x77c00000u) return __ddiv_rn(a, b);
