@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(256) k_g_channel(WaveDev W, int lo, int hi, lo
         pp_channel_block<DIMS, TAB, 11, true>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms,
                                         Densities{P.dens, P.ms}, P.vwv, P.bin_rec, 0, i0, i1, c, smem);
     else
-        pp_channel_block<DIMS, TAB, 9, true>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms,
+        pp_channel_block<DIMS, TAB, 8, true>(P.pp, P.tables, P.bins, P.memo, P.cfail, P.ich_tile, P.ms,
                                         Densities{P.dens, P.ms}, P.vwv, P.bin_rec, 0, i0, i1, c, smem);
 }
 

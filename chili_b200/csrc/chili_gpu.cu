@@ -64,8 +64,8 @@ int launch_channel(chili_ctx *ctx, const PointProgram *pp, const GridTables &G, 
     const bool f11 = cell_fbits(bins) == 11;
     auto pick = [&](auto rec) {
         constexpr bool R = decltype(rec)::value;
-        return tab ? (f11 ? k_pp_channel<D, true, 11, R> : k_pp_channel<D, true, 9, R>)
-                   : (f11 ? k_pp_channel<D, false, 11, R> : k_pp_channel<D, false, 9, R>);
+        return tab ? (f11 ? k_pp_channel<D, true, 11, R> : k_pp_channel<D, true, 8, R>)
+                   : (f11 ? k_pp_channel<D, false, 11, R> : k_pp_channel<D, false, 8, R>);
     };
     auto kern = rec_bins ? pick(std::true_type{}) : pick(std::false_type{});
     if (smem > 48 * 1024)

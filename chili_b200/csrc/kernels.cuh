@@ -97,10 +97,10 @@ __global__ void k_grid_weight(const double *__restrict__ g, const uint32_t *__re
         const double v = x[i * dims + d];
         bool slow;
         int k = cell_fbits(bins) == 11 ? cell_count<true, 11>(en, cells, cells * 2048.0, v, slow)
-                                       : cell_count<true, 9>(en, cells, cells * 512.0, v, slow);
+                                       : cell_count<true, 8>(en, cells, cells * 256.0, v, slow);
         if (slow)
             k = cell_fbits(bins) == 11 ? cell_count_slow<true, 11>(e, en, bins, cells, cells * 2048.0, v)
-                                       : cell_count_slow<true, 9>(e, en, bins, cells, cells * 512.0, v);
+                                       : cell_count_slow<true, 8>(e, en, bins, cells, cells * 256.0, v);
         if (bin) bin[i * dims + d] = k - 1;
         jac = __dmul_rn(jac, __ldg(ws + d * width_row(bins) + k));
     }

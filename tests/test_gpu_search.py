@@ -35,3 +35,37 @@ def test_bins_match_lower_bound(ctx_factory, bins):
     for d in range(4):
         jac = jac * (width[:, d] * float(bins))
     assert np.array_equal(w[ok], jac)
+
+
+def test_crowded_cells_are_searched_by_bisection(ctx_factory):
+    """A trained peak puts most edges, and so most points, into few cells.  The
+    search among a cell's edges takes a logarithm of their number: with all
+    1000 edges in one cell a coordinate between them costs at most six times
+    one on equidistant edges (read one after the other: 44 times)."""
+    import ctypes as C
+
+    import torch
+
+    bins, n = 1000, 1 << 20
+    rng = np.random.default_rng(4)
+    crowded = np.concatenate([[0.0], np.sort(0.3 + 1e-5 * rng.random(bins - 1)), [1.0]])
+    x = torch.from_numpy(0.3 + 1e-5 * rng.random((n, 4))).cuda()
+    w = torch.empty(n, dtype=torch.float64, device="cuda")
+    times = []
+    stream = torch.cuda.Stream()
+    for row in (np.linspace(0, 1, bins + 1), crowded):
+        ctx = ctx_factory()
+        ctx.set_stream(stream.cuda_stream)
+        ctx.set_grids(np.tile(row, (1, 4, 1)))
+        span = x if row is crowded else torch.from_numpy(rng.random((n, 4))).cuda()
+        torch.cuda.synchronize()
+        best = np.inf
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            ctx.call("chili_gpu_grid_weight", 0, C.c_void_p(span.data_ptr()), C.c_void_p(w.data_ptr()), None, n)
+            b.record(stream)
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times.append(best)
+    assert times[1] <= 6 * times[0], times
