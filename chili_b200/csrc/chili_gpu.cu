@@ -37,9 +37,17 @@ namespace {
 
 int rebuild_hints(chili_ctx *ctx);
 
-// Largest table of one channel (entries and widths) staged in shared memory
-// by the channel step; larger ones are read from global memory.
-constexpr size_t kMaxChannelTab = 200 * 1024;
+// Dynamic shared memory that kernels with tables of the grid's size may take;
+// channel tables (entries and widths) beyond it are read from global memory.
+constexpr size_t kMaxDynSmem = 200 * 1024;
+
+// A kernel's limit is one value per process and device, so every launch that
+// needs more than the default sets this same one: the size of the call at hand
+// could be lowered by another thread, with a smaller grid, before its launch.
+template <class K>
+cudaError_t allow_dyn_smem(K kern) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxDynSmem));
+}
 
 GridTables grid_tables(const chili_ctx *ctx) {
     return GridTables{ctx->edges.as<double>(), ctx->cells.as<uint32_t>(), ctx->widths.as<double>()};
@@ -51,7 +59,7 @@ template <int D>
 int launch_channel(chili_ctx *ctx, const PointProgram *pp, const GridTables &G, int bins, const double *memo,
                    const uint8_t *cfail, const int32_t *ich_tile, const long long *n_list, long long base, long long T,
                    Densities dens, double *vwv, uint4 *rec_bins, double *x_own, int nch, long long n) {
-    const bool tab = ctx->channel_tables && channel_smem_bytes(D, bins, true) <= kMaxChannelTab;
+    const bool tab = ctx->channel_tables && channel_smem_bytes(D, bins, true) <= kMaxDynSmem;
     const size_t smem = channel_smem_bytes(D, bins, tab);
     // as many threads per block as keep 32 warps on an SM beside the tables
     const int threads = !tab || smem <= 54 * 1024 ? 256 : (smem <= 110 * 1024 ? 512 : channel_max_threads(D));
@@ -68,8 +76,7 @@ int launch_channel(chili_ctx *ctx, const PointProgram *pp, const GridTables &G, 
                    : (f11 ? k_pp_channel<D, false, 11, R> : k_pp_channel<D, false, 8, R>);
     };
     auto kern = rec_bins ? pick(std::true_type{}) : pick(std::false_type{});
-    if (smem > 48 * 1024)
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    if (smem > 48 * 1024) CK(allow_dyn_smem(kern));
     kern<<<grid, threads, smem, ctx->stream>>>(pp, G, bins, memo, cfail, ich_tile, n_list, base, T, dens, vwv,
                                                rec_bins ? static_cast<void *>(rec_bins) : x_own, static_cast<int>(points));
     LAUNCHED();
@@ -845,8 +852,7 @@ int chili_gpu_vegas_iterate(chili_ctx *ctx, uint64_t ncalls, uint64_t seed, uint
                                      : (ast.host ? reinterpret_cast<double *>(ctx->stats_host) : static_cast<double *>(ast.dev));
         {
             KTimer kt_(ctx, KT_VEGAS_STEP);
-            if (step_smem > 40 * 1024)  // with the kernel's own (static) 4.6 KB above 48 KB
-                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(step_smem)));
+            if (step_smem > 40 * 1024) CK(allow_dyn_smem(kern));  // with the kernel's own (static) 4.6 KB above 48 KB
             kern<<<static_cast<unsigned>(nb), kVegasBlock, step_smem, ctx->stream>>>(
                 ctx->edges.as<double>(), ctx->edges_tmp.as<double>(), D, B, seed, counter_base,
                 static_cast<const double *>(au.dev), n, ctx->f_dev.as<IntegrandDesc>(), ctx->v_part.as<double>(),
@@ -882,8 +888,7 @@ int chili_gpu_vegas_iterate(chili_ctx *ctx, uint64_t ncalls, uint64_t seed, uint
     }
     KTimer kt_(ctx, KT_VEGAS);
     const size_t it_smem = (smem ? hist_bytes : 0) + (stage ? sizeof(double) * D * (B + 1) : 0);
-    if (it_smem > 40 * 1024)  // with the kernel's own (static) 1.5 KB above 48 KB
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(it_smem)));
+    if (it_smem > 40 * 1024) CK(allow_dyn_smem(kern));  // with the kernel's own (static) 1.5 KB above 48 KB
     kern<<<static_cast<unsigned>(nblocks), kVegasBlock, it_smem, ctx->stream>>>(
         ctx->edges.as<double>(), D, B, seed, counter_base, static_cast<const double *>(au.dev), n,
         ctx->f_dev.as<IntegrandDesc>(), ctx->v_part.as<double>(), ctx->v_hist.as<double>(), smem ? 1 : 0);
@@ -921,7 +926,7 @@ int chili_gpu_vegas_generate(chili_ctx *ctx, uint64_t n, uint64_t seed, uint64_t
     int ppt = static_cast<int>(ctx->gen_ppt);
     if (sizeof(double) * (grid_doubles + static_cast<size_t>(kGenTile) * ppt * (D + 1)) > 64 * 1024) ppt = 1;
     size_t smem = sizeof(double) * (grid_doubles + static_cast<size_t>(kGenTile) * ppt * (D + 1));
-    if (smem > 200 * 1024) return fail(ctx, CHILI_ERR_LIMIT, "grid too large for the shared-memory staging");
+    if (smem > kMaxDynSmem) return fail(ctx, CHILI_ERR_LIMIT, "grid too large for the shared-memory staging");
     const long long nn = static_cast<long long>(n);
     Arg ax, aw;
     if ((rc = resolve(ctx, x_out, sizeof(double) * nn * D, 0, false, ax))) return rc;
@@ -951,8 +956,7 @@ int chili_gpu_vegas_generate(chili_ctx *ctx, uint64_t n, uint64_t seed, uint64_t
             ppt = 1;
             break;
     }
-    if (smem > 48 * 1024)
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    if (smem > 48 * 1024) CK(allow_dyn_smem(kern));
     int sms = 148, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGenTile, smem));
