@@ -103,26 +103,32 @@ int launch_channel_dims(chili_ctx *ctx, int dims, A... a) {
 
 namespace {
 
-// The tile buffers of the phased pass for T points, for a whole number of
-// 2^16 points: the accepted count of a chunk varies from call to call, and a
-// buffer that grew by a few points each time would be reallocated (a device
-// synchronisation) each time.
-cudaError_t pipeline_buffers(chili_ctx *ctx, long long T, bool own_dens) {
-    const PointProgram &P = ctx->pp_host;
-    const long long Ta = (T + 65535) / 65536 * 65536;
-    const std::pair<DevView *, size_t> want[] = {
-        {&ctx->node_soa, sizeof(double) * 4 * P.n_nodes * Ta},
-        {&ctx->memo, sizeof(double) * std::max(1, P.n_memo) * Ta},
-        {&ctx->vwv, sizeof(double) * ctx->nch * Ta},
-        {&ctx->dcv, own_dens ? sizeof(double) * ctx->nch * Ta : 0},
-        {&ctx->ich_tile, sizeof(int32_t) * Ta},
-        {&ctx->cfail, static_cast<size_t>(std::max(1, P.n_chains)) * Ta}};
+// The tile buffers of the phased pass for `points` points (a multiple of 64)
+// in one allocation: a cudaMalloc that needs new memory takes 0.35 ms whatever
+// its size.
+struct TileParts {
+    std::pair<DevView *, size_t> part[7];
     size_t total = 0;
-    for (const auto &w : want) total += w.second;  // Ta keeps every part a multiple of 2^16 bytes
-    const cudaError_t e = ctx->tile.ensure(total);
+};
+
+TileParts tile_parts(chili_ctx *ctx, long long points, bool own_dens) {
+    const PointProgram &P = ctx->pp_host;
+    TileParts t{{{&ctx->every_count, 256},
+                 {&ctx->node_soa, sizeof(double) * 4 * P.n_nodes * points},
+                 {&ctx->memo, sizeof(double) * std::max(1, P.n_memo) * points},
+                 {&ctx->vwv, sizeof(double) * ctx->nch * points},
+                 {&ctx->dcv, own_dens ? sizeof(double) * ctx->nch * points : 0},
+                 {&ctx->ich_tile, sizeof(int32_t) * points},
+                 {&ctx->cfail, static_cast<size_t>(std::max(1, P.n_chains)) * points}}};
+    for (const auto &w : t.part) t.total += w.second;  // every part but the last a multiple of 256 bytes
+    return t;
+}
+
+cudaError_t pipeline_buffers(chili_ctx *ctx, const TileParts &t) {
+    const cudaError_t e = ctx->tile.ensure(t.total);
     if (e != cudaSuccess) return e;
     char *at = ctx->tile.as<char>();
-    for (const auto &w : want) {
+    for (const auto &w : t.part) {
         w.first->p = w.second ? at : nullptr;
         at += w.second;
     }
@@ -170,26 +176,45 @@ int pipeline_tile(chili_ctx *ctx, const long long *n_list, long long base, long 
                                ctx->vwv.as<double>(), rec_bins, x_own, ctx->nch, n);
 }
 
-// Tiles of entry points that weight every one of n points (k_pp_given,
-// k_pp_drawn): points per tile, or 0 where the per-thread kernels take the
-// call -- a set without shared program or phased kernels, the option
-// "pipeline" 0, a stream that is being captured (the tile buffers may move
-// later, and the per-thread kernels need none), or no memory for the tile.
-// 2^18 points: 0.4 GB of buffers for the 2->4 set; larger tiles are no
-// faster, smaller ones lose to launch tails.
-long long every_point_tile(chili_ctx *ctx, long long n) {
-    if (!(pipeline_dims_ok(ctx->ndims) && ctx->have_pp && ctx->use_pp && ctx->use_pipeline)) return 0;
+// Whether entry points that take every one of their points (k_pp_given,
+// k_pp_drawn) may run the tiled pass.  The per-thread kernels keep sets without
+// shared program or phased kernels, the option "pipeline" 0, and a stream that
+// is being captured (the tile buffers may move later, and the per-thread
+// kernels need none).  Both give the same bits, so the rules of
+// every_point_tile are about time alone.
+bool every_point_tiled(chili_ctx *ctx) {
+    if (!(pipeline_dims_ok(ctx->ndims) && ctx->have_pp && ctx->use_pp && ctx->use_pipeline)) return false;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return 0;
-    }
+    if (cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) return true;
+    cudaGetLastError();
+    return false;
+}
+
+// Points per tile of a call that weights every one of n points, or 0 where the
+// per-thread kernels take it: every_point_tiled, no memory for the tile, and
+// a context's first short call, which would allocate the tile: the 0.35 ms come
+// back only where the per-thread pass takes about 0.9 ms, 5.8 us per channel and
+// outgoing leg and 2^16 points (15 2->4 channels, 20,000 points: 0.35 ms against
+// 0.12 and the allocation).
+// 2^18 points: 0.4 GB of buffers for the 2->4 set; larger tiles are no faster,
+// smaller ones lose to launch tails.  A short call's buffers hold the next
+// power of two of its points: up to about 1 MB come from memory that the
+// context has mapped, and calls of growing size move them seldom.
+long long every_point_tile(chili_ctx *ctx, long long n) {
+    const long long legs = ctx->nch * (ctx->n_ext - 2ll);
+    if (!every_point_tiled(ctx)) return 0;
     const long long tiles = (n + (1ll << 18) - 1) >> 18, T = (n + tiles - 1) / tiles;  // tiles of one size
-    if (ctx->every_count.ensure(sizeof(long long)) != cudaSuccess || pipeline_buffers(ctx, T, true) != cudaSuccess) {
-        cudaGetLastError();
+    long long room = 64;
+    while (room < T && room < (1 << 16)) room <<= 1;
+    const TileParts parts = tile_parts(ctx, (T + room - 1) / room * room, true);
+    if (parts.total > ctx->tile.cap && parts.total > (1u << 20) && !ctx->every_called &&
+        legs * ((n + 65535) >> 16) < 150) {
+        ctx->every_called = true;
         return 0;
     }
-    return T;
+    if (pipeline_buffers(ctx, parts) == cudaSuccess) return T;
+    cudaGetLastError();
+    return 0;
 }
 
 }  // namespace
@@ -209,7 +234,10 @@ int pipeline_run(chili_ctx *ctx, const double *mom_soa, long long m, const int32
     // gridDim.y (point blocks of 128) stays below 65536
     const long long T = std::min<long long>(std::min<long long>(ctx->pipe_tile, 65535ll * 128),
                                             std::max<long long>(n_pre, 1));
-    CK(pipeline_buffers(ctx, T, !rec_dens));
+    // room for a whole number of 2^16 points: the accepted count of a chunk
+    // varies from call to call, and a buffer that grew by a few points each
+    // time would be reallocated (a device synchronisation) each time
+    CK(pipeline_buffers(ctx, tile_parts(ctx, (T + 65535) / 65536 * 65536, !rec_dens)));
     const unsigned gx = static_cast<unsigned>((T + 255) / 256);
     for (long long base = 0; base < n_pre; base += T) {
         // the densities go straight to the records, or to a tile buffer
@@ -418,7 +446,7 @@ int chili_gpu_destroy(chili_ctx *ctx) {
     DevBuf *bufs[] = {&ctx->edges, &ctx->edges_tmp, &ctx->progs, &ctx->point_prog, &ctx->tile, &ctx->cells, &ctx->widths, &ctx->alpha_buf, &ctx->f_dev, &ctx->mom_soa,
                       &ctx->ich, &ctx->flag, &ctx->list, &ctx->block_count, &ctx->block_off, &ctx->part,
                       &ctx->hist, &ctx->round_res, &ctx->acc, &ctx->ctl, &ctx->status, &ctx->v_part,
-                      &ctx->v_hist, &ctx->v_train, &ctx->v_out, &ctx->rec, &ctx->ctl3, &ctx->unw, &ctx->iter_ctl, &ctx->every_count,
+                      &ctx->v_hist, &ctx->v_train, &ctx->v_out, &ctx->rec, &ctx->ctl3, &ctx->unw, &ctx->iter_ctl,
                       &ctx->mom_soa_alt, &ctx->ich_alt, &ctx->flag_alt, &ctx->block_count_alt,
                       &ctx->v_arrive};
     for (DevBuf *b : bufs) b->release();
@@ -1580,7 +1608,8 @@ int chili_gpu_generate(chili_ctx *ctx, int64_t n, uint64_t seed, uint64_t counte
     if ((rc = resolve(ctx, mom, sizeof(double) * n * ctx->n_ext * 4, 0, false, am))) return rc;
     if ((rc = resolve(ctx, wgt, sizeof(double) * n, 1, false, aw))) return rc;
     if ((rc = resolve(ctx, ch, sizeof(int32_t) * n, 2, false, ac))) return rc;
-    const long long T = every_point_tile(ctx, n);
+    // without weights the points are drawn in one launch and need no buffers
+    const long long T = wgt ? every_point_tile(ctx, n) : (every_point_tiled(ctx) ? static_cast<long long>(n) : 0);
     for (long long base = 0; T > 0 && base < n; base += T) {
         const Densities dd{ctx->dcv.as<double>(), T};
         {

@@ -151,9 +151,10 @@ struct chili_ctx {
     PointProgram pp_host;      // host copy (sizes of the memo buffers)
     DevBuf tile;  // buffers of a tile of the phased pass, in one allocation (a cudaMalloc takes 0.35 ms here)
     DevView node_soa, memo, cfail, dcv, vwv, ich_tile;
+    bool every_called = false;  // a short call has run without the tile (every_point_tile)
+    DevView every_count;  // point count of a call that weights every point (the tile steps read it)
     DevBuf v_arrive;  // the fused Vegas iteration's arrival counter (zero between launches)
     DevBuf cells, widths;  // search entries and scaled bin widths of the grids (grid.cuh)
-    DevBuf every_count;  // point count of a call that weights every point (the tile steps read it)
     // channel weights: alpha[CH], best[CH], cp[CH], min_diff
     DevBuf alpha_buf;
     bool alpha_set = false;

@@ -137,15 +137,15 @@ __global__ void __launch_bounds__(256) k_pp_given(const PointProgram *__restrict
 }
 
 // Tile of drawn points (counters ctr0 + base + i): channel, VEGAS map,
-// FSMapper; nodes, the tile's channels and count, and the points' momenta
-// and channels where asked for.  No PreProcess.
+// FSMapper; nodes, the tile's channels and count (node_soa null: none of
+// them), and the points' momenta and channels where asked for.  No PreProcess.
 __global__ void __launch_bounds__(kFwdBlock, 3) k_pp_drawn(
     const PointProgram *__restrict__ pp, const ChannelProgram *__restrict__ progs, const double *__restrict__ grids,
     const double *__restrict__ cp, int dims, int bins, uint64_t seed, uint64_t ctr0, long long base, long long n,
     long long m, double *__restrict__ node_soa, int32_t *__restrict__ ich_tile, double *__restrict__ mom_out,
     int32_t *__restrict__ ch_out, long long *__restrict__ count) {
     const long long i = blockIdx.x * static_cast<long long>(kFwdBlock) + threadIdx.x;
-    if (i == 0) *count = n;
+    if (i == 0 && node_soa) *count = n;
     if (i >= m || base + i >= n) return;
     const int ne = pp->n_ext;
     V4 mom[CHILI_MAX_SLOTS];

@@ -74,8 +74,72 @@ def test_both_routes_round_every_point_the_same(ctx_factory, n_out, n):
     divided by 2 pi once per decay (Channel.cc:111) on both, so the bound at
     every point, cancelling channel sums included, is zero."""
     ctxs = [_context(ctx_factory, n_out, p) for p in (0, 1)]
+    ctxs[1].generate(n, seed=1)  # a context's first short call is not tiled
     events = [c.generate(n, seed=29, counter=7) for c in ctxs]
     for a, b in zip(*events):
         assert np.array_equal(a, b, equal_nan=True)
     for a, b in zip(*(c.multichannel_weight(events[0][0], events[0][2]) for c in ctxs)):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+def _grown(call):
+    """Device memory that the call leaves allocated."""
+    import torch
+
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    call()
+    torch.cuda.synchronize()
+    return before - torch.cuda.mem_get_info()[0]
+
+
+def _device_points(ctx, n):
+    import torch
+
+    mom, _, ich = ctx.generate(n, seed=3)
+    return [torch.from_numpy(a).cuda() for a in (mom, ich, np.zeros(n))]
+
+
+def _weigh(ctx, dev):
+    ctx.call("chili_gpu_multichannel_weight", *(C.c_void_p(t.data_ptr()) for t in dev), None, None, dev[1].shape[0])
+    ctx.synchronize()
+    return dev[2].cpu().numpy()
+
+
+def test_work_space_follows_the_call(ctx_factory):
+    """A call of one point holds no buffers for 2^16 of them (0.25 GB for the
+    2->6 set), a context's first short call holds none, and drawing points
+    without weights holds none either."""
+    import torch
+
+    mb = 1 << 20
+    warm = _context(ctx_factory, 6, 1)  # the kernels' code is loaded once
+    one, some = _device_points(warm, 1), _device_points(_context(ctx_factory, 4, 0), 20000)
+    out = torch.empty(300000, 8, 4, dtype=torch.float64, device="cuda")
+
+    def points_alone(ctx):
+        ctx.call("chili_gpu_generate", out.shape[0], 2, 0, C.c_void_p(out.data_ptr()), None, None)
+
+    for _ in range(2):
+        _weigh(warm, one)
+        _weigh(_context(ctx_factory, 4, 1), some)
+    points_alone(warm)
+    ctx = _context(ctx_factory, 6, 1)
+    assert _grown(lambda: _weigh(ctx, one)) <= 8 * mb
+    assert _grown(lambda: points_alone(ctx)) <= 8 * mb
+    want = _context(ctx_factory, 6, 0).generate(out.shape[0], seed=2)[0]
+    assert np.array_equal(out.cpu().numpy(), want, equal_nan=True)
+    ctx = _context(ctx_factory, 4, 1)
+    got = []
+    assert _grown(lambda: got.append(_weigh(ctx, some))) <= 8 * mb
+    assert _grown(lambda: got.append(_weigh(ctx, some))) > 8 * mb  # the second one is tiled
+    assert np.array_equal(got[0], got[1], equal_nan=True)
+
+
+def test_calls_of_changing_size_on_one_context(ctx_factory):
+    """The tile's parts are laid out anew by every call."""
+    ctx, ref = _context(ctx_factory, 4, 1), _context(ctx_factory, 4, 0)
+    for n in (1, 64, 65, 5000, 3, 70000, 300, 262145, 2):
+        got, want = ctx.generate(n, seed=n), ref.generate(n, seed=n)
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b, equal_nan=True)
