@@ -192,17 +192,24 @@ bool every_point_tiled(chili_ctx *ctx) {
 
 // Points per tile of a call that weights every one of n points, or 0 where the
 // per-thread kernels take it: every_point_tiled, no memory for the tile, and
-// a context's first short call, which would allocate the tile: the 0.35 ms come
-// back only where the per-thread pass takes about 0.9 ms, 5.8 us per channel and
-// outgoing leg and 2^16 points (15 2->4 channels, 20,000 points: 0.35 ms against
-// 0.12 and the allocation).
+//  - one or two channels at up to 2^16 points, one wave of the per-thread
+//    kernel: their few items do not pay for seven launches (two 2->2 channels,
+//    given momenta: 300 points 34 against 37 us, 60,000 points 38 against 44;
+//    100,000 points, two waves, 66 against 48; three 2->4 channels, 300 points:
+//    69 against 42), and sets of fewer than four outgoing legs over all
+//    channels at any size (one 2->2 channel, 1e6 points: 202 against 239; two,
+//    four legs: 309 against 292);
+//  - a context's first short call, which would allocate the tile: the 0.35 ms
+//    come back only where the per-thread pass takes about 0.9 ms, 5.8 us per
+//    channel and outgoing leg and 2^16 points (15 2->4 channels, 20,000 points:
+//    0.35 ms against 0.12 and the allocation).
 // 2^18 points: 0.4 GB of buffers for the 2->4 set; larger tiles are no faster,
 // smaller ones lose to launch tails.  A short call's buffers hold the next
 // power of two of its points: up to about 1 MB come from memory that the
 // context has mapped, and calls of growing size move them seldom.
 long long every_point_tile(chili_ctx *ctx, long long n) {
     const long long legs = ctx->nch * (ctx->n_ext - 2ll);
-    if (!every_point_tiled(ctx)) return 0;
+    if (!every_point_tiled(ctx) || legs < 4 || (ctx->nch <= 2 && n <= (1 << 16))) return 0;
     const long long tiles = (n + (1ll << 18) - 1) >> 18, T = (n + tiles - 1) / tiles;  // tiles of one size
     long long room = 64;
     while (room < T && room < (1 << 16)) room <<= 1;

@@ -136,6 +136,19 @@ def test_work_space_follows_the_call(ctx_factory):
     assert np.array_equal(got[0], got[1], equal_nan=True)
 
 
+def test_two_channels_are_tiled_beyond_one_wave(ctx_factory):
+    """Two channels' few items pay for the tiled pass's launches only where the
+    per-thread kernel needs more than one wave; the bits are the same."""
+    ctx, ref = _context(ctx_factory, 2, 1), _context(ctx_factory, 2, 0)
+    for n, tiled in ((65536, False), (65537, True)):
+        dev = _device_points(ref, n)
+        want = _weigh(ref, dev)
+        for k in range(3):
+            before = ctx.launches
+            assert np.array_equal(_weigh(ctx, dev), want, equal_nan=True)
+            assert (ctx.launches - before > 1) == (tiled and k > 0)  # the first short call allocates nothing
+
+
 def test_calls_of_changing_size_on_one_context(ctx_factory):
     """The tile's parts are laid out anew by every call."""
     ctx, ref = _context(ctx_factory, 4, 1), _context(ctx_factory, 4, 0)
