@@ -553,7 +553,8 @@ __global__ void __launch_bounds__(256) k_g_chains(WaveDev W, int lo, int hi, lon
 // points of one channel c of one piece (pp_channel_block; TAB: the channel's
 // tables in dynamic shared memory).
 template <int DIMS, bool TAB>
-__global__ void __launch_bounds__(256) k_g_channel(WaveDev W, int lo, int hi, long long blk0) {
+__global__ void __launch_bounds__(channel_max_threads(DIMS), DIMS > 16 ? 1 : 1024 / channel_max_threads(DIMS))
+    k_g_channel(WaveDev W, int lo, int hi, long long blk0) {
     extern __shared__ __align__(16) char smem[];
     CHILI_PIECE(GS_CHANNEL)
     const int c = static_cast<int>(lb % P.nch);
@@ -807,7 +808,15 @@ struct BatchState {
         int sidx = 0;                                // stream (and arena) of the wave
         long long prefix_off = 0;                    // into d_prefix
         std::vector<long long> blocks;               // per step: total blocks
-        std::vector<std::array<int, 4>> dgroups;     // (dims, k0, k1, bins): pieces [k0, k1) of one dimension, their most bins
+        // (dims, k0, k1, bins): pieces [k0, k1) of one dimension and size of
+        // cell table, their most bins
+        std::vector<std::array<int, 4>> dgroups;
+        void add(const Piece &P, int k) {
+            if (dgroups.empty() || dgroups.back()[0] != P.dims || grid_cells(dgroups.back()[3]) != grid_cells(P.bins))
+                dgroups.push_back({P.dims, k, k, P.bins});
+            dgroups.back()[2] = k + 1;
+            dgroups.back()[3] = std::max(dgroups.back()[3], P.bins);
+        }
     };
     std::vector<Piece> pieces;
     std::vector<WaveHost> waves;
@@ -1009,18 +1018,15 @@ int enqueue_waves(chili_ctx *ctx, const BatchDev &B, const std::vector<BatchStat
         for (const auto &g : w.dgroups) {
             const long long b0 = pc[g[1]], nbk = pc[g[2]] - b0;
             if (nbk <= 0) continue;
-            // one channel's entries and widths in shared memory when they
-            // fit the default 48 KB
-            const bool use_tab = ctx->channel_tables && channel_smem_bytes(g[0], g[3], true) <= 48 * 1024;
-            const size_t smem = channel_smem_bytes(g[0], g[3], use_tab);
+            const ChannelShape cs = grouped_channel_shape(g[0], g[3], ctx->channel_tables);
             switch (g[0]) {
-#define CHILI_GCH(D)                                                                                         \
-    case D:                                                                                                  \
-        if (use_tab)                                                                                         \
-            k_g_channel<D, true><<<static_cast<unsigned>(nbk), 256, smem, ctx->stream>>>(W, g[1], g[2], b0);  \
-        else                                                                                                 \
-            k_g_channel<D, false><<<static_cast<unsigned>(nbk), 256, smem, ctx->stream>>>(W, g[1], g[2], b0); \
-        break;
+#define CHILI_GCH(D)                                                                                       \
+    case D: {                                                                                              \
+        auto kern = cs.tables ? k_g_channel<D, true> : k_g_channel<D, false>;                              \
+        if (cs.smem > 48 * 1024) CK(allow_dyn_smem(kern));                                                 \
+        kern<<<static_cast<unsigned>(nbk), cs.threads, cs.smem, ctx->stream>>>(W, g[1], g[2], b0);         \
+        break;                                                                                             \
+    }
                 CHILI_GCH(1) CHILI_GCH(4) CHILI_GCH(7) CHILI_GCH(10) CHILI_GCH(13) CHILI_GCH(16) CHILI_GCH(19)
                 CHILI_GCH(22)
 #undef CHILI_GCH
@@ -1077,13 +1083,7 @@ int run_retry_round(chili_ctx *ctx) {
         for (size_t j = 0; j < keep.size(); ++j) {
             const Piece &P = S.pieces[static_cast<size_t>(w.first + keep[j])];
             S.top_pieces.push_back(P);
-            const int kj = static_cast<int>(j);
-            if (fw.dgroups.empty() || fw.dgroups.back()[0] != P.dims) {
-                fw.dgroups.push_back({P.dims, kj, kj + 1, P.bins});
-            } else {
-                fw.dgroups.back()[2] = kj + 1;
-                fw.dgroups.back()[3] = std::max(fw.dgroups.back()[3], P.bins);
-            }
+            fw.add(P, static_cast<int>(j));
         }
         S.top_waves.push_back(fw);
     }
@@ -1417,9 +1417,10 @@ int plan_waves(chili_ctx *ctx, const std::vector<PointProgram> &pps) {
     S.prefix_host.clear();
     for (size_t wi = 0; wi < waves.size(); ++wi) {
         auto &w = waves[wi];
-        // pieces of one dimension together
+        // pieces of one dimension and size of cell table together
         std::stable_sort(w.begin(), w.end(), [&](const Piece &a, const Piece &b) {
-            return S.tasks[static_cast<size_t>(a.ti)].dims < S.tasks[static_cast<size_t>(b.ti)].dims;
+            const BatchTask &p = S.tasks[static_cast<size_t>(a.ti)], &q = S.tasks[static_cast<size_t>(b.ti)];
+            return p.dims != q.dims ? p.dims < q.dims : grid_cells(p.bins) < grid_cells(q.bins);
         });
         BatchState::WaveHost wh;
         wh.sidx = static_cast<int>(wi % ns);
@@ -1473,12 +1474,7 @@ int plan_waves(chili_ctx *ctx, const std::vector<PointProgram> &pps) {
             const long long nblk[kGroupSteps] = {P.nb, P.nb, gx, P.n_items[0] * gx, P.n_items[1] * gx,
                                                  P.n_items[2] * gx, P.n_chains * gx, P.nch * gy, gx, P.nb};
             for (int st = 0; st < kGroupSteps; ++st) pre[static_cast<size_t>(st)][k + 1] = pre[st][k] + nblk[st];
-            if (wh.dgroups.empty() || wh.dgroups.back()[0] != P.dims) {
-                wh.dgroups.push_back({P.dims, static_cast<int>(k), static_cast<int>(k) + 1, P.bins});
-            } else {
-                wh.dgroups.back()[2] = static_cast<int>(k) + 1;
-                wh.dgroups.back()[3] = std::max(wh.dgroups.back()[3], P.bins);
-            }
+            wh.add(P, static_cast<int>(k));
         }
         for (int st = 0; st < kGroupSteps; ++st) {
             wh.blocks.push_back(pre[static_cast<size_t>(st)][w.size()]);

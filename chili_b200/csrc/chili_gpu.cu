@@ -37,18 +37,6 @@ namespace {
 
 int rebuild_hints(chili_ctx *ctx);
 
-// Dynamic shared memory that kernels with tables of the grid's size may take;
-// channel tables (entries and widths) beyond it are read from global memory.
-constexpr size_t kMaxDynSmem = 200 * 1024;
-
-// A kernel's limit is one value per process and device, so every launch that
-// needs more than the default sets this same one: the size of the call at hand
-// could be lowered by another thread, with a smaller grid, before its launch.
-template <class K>
-cudaError_t allow_dyn_smem(K kern) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxDynSmem));
-}
-
 GridTables grid_tables(const chili_ctx *ctx) {
     return GridTables{ctx->edges.as<double>(), ctx->cells.as<uint32_t>(), ctx->widths.as<double>()};
 }
@@ -59,10 +47,7 @@ template <int D>
 int launch_channel(chili_ctx *ctx, const PointProgram *pp, const GridTables &G, int bins, const double *memo,
                    const uint8_t *cfail, const int32_t *ich_tile, const long long *n_list, long long base, long long T,
                    Densities dens, double *vwv, uint4 *rec_bins, double *x_own, int nch, long long n) {
-    const bool tab = ctx->channel_tables && channel_smem_bytes(D, bins, true) <= kMaxDynSmem;
-    const size_t smem = channel_smem_bytes(D, bins, tab);
-    // as many threads per block as keep 32 warps on an SM beside the tables
-    const int threads = !tab || smem <= 54 * 1024 ? 256 : (smem <= 110 * 1024 ? 512 : channel_max_threads(D));
+    const auto [tab, smem, threads] = channel_shape(D, bins, ctx->channel_tables);
     // points per block: enough for the table copy to be small beside them,
     // few enough for about four blocks per SM
     long long points = n * nch / (4 * ctx->sms);
@@ -70,7 +55,7 @@ int launch_channel(chili_ctx *ctx, const PointProgram *pp, const GridTables &G, 
     points = std::max(points, (T / 65535 / threads + 1) * threads);  // gridDim.y stays below 65536
     const dim3 grid(static_cast<unsigned>(nch), static_cast<unsigned>((T + points - 1) / points));
     const bool f11 = cell_fbits(bins) == 11;
-    auto pick = [&](auto rec) {
+    auto pick = [f11, tab = tab](auto rec) {
         constexpr bool R = decltype(rec)::value;
         return tab ? (f11 ? k_pp_channel<D, true, 11, R> : k_pp_channel<D, true, 8, R>)
                    : (f11 ? k_pp_channel<D, false, 11, R> : k_pp_channel<D, false, 8, R>);

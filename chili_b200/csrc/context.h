@@ -297,6 +297,15 @@ bool is_device_ptr(const void *p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// A kernel's dynamic shared-memory limit is one value per process and device,
+// so every launch that needs more than the default sets this same one: the size
+// of the call at hand could be lowered by another thread, with a smaller grid,
+// before its launch.
+template <class K>
+cudaError_t allow_dyn_smem(K kern) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxDynSmem));
+}
+
 // Resolves a caller buffer to a device pointer: device buffers pass through,
 // host buffers are staged in slot `slot` (copied in when `in`).
 struct Arg {

@@ -292,6 +292,33 @@ __host__ __device__ inline size_t channel_smem_bytes(int dims, int bins, bool ta
     return rows + (tables ? static_cast<size_t>(dims) * (4 * static_cast<size_t>(grid_cells(bins)) + 8 * width_row(bins)) : 0);
 }
 
+// Dynamic shared memory that kernels with tables of the grid's size may take.
+constexpr size_t kMaxDynSmem = 200 * 1024;
+
+// Launch shape of the channel step: one channel's tables in shared memory
+// where they fit, and as many threads per block as keep 32 warps on an SM
+// beside them.
+constexpr int channel_max_threads(int dims) { return dims > 10 && dims <= 16 ? 1024 : 512; }
+struct ChannelShape {
+    bool tables;
+    size_t smem;
+    int threads;
+};
+inline ChannelShape channel_shape(int dims, int bins, bool want_tables) {
+    const bool tab = want_tables && channel_smem_bytes(dims, bins, true) <= kMaxDynSmem;
+    const size_t smem = channel_smem_bytes(dims, bins, tab);
+    return {tab, smem, !tab || smem <= 54 * 1024 ? 256 : (smem <= 110 * 1024 ? 512 : channel_max_threads(dims))};
+}
+// The same for the grouped launches of batched tasks, whose blocks take a
+// couple of thousand points: tables that leave no room for 32 warps are read
+// from global memory (14 tasks of 10 dimensions at 300 bins, 196 KB: 2.54 ms an
+// iteration staged, 2.32 read from there; 200 bins, 98 KB: 2.10 against 2.15; 11
+// tasks of 13 dimensions at 200 bins, 127 KB and 32 warps: 1.32 against 1.35).
+inline ChannelShape grouped_channel_shape(int dims, int bins, bool want_tables) {
+    const ChannelShape s = channel_shape(dims, bins, want_tables);
+    return s.smem > 110 * 1024 && s.threads < 1024 ? channel_shape(dims, bins, false) : s;
+}
+
 // 16 bytes from global to shared memory (both 16-byte aligned), and the wait
 // for this thread's copies.
 __device__ __forceinline__ void copy16_async(uint32_t dst, const void *src) {

@@ -70,8 +70,6 @@ __global__ void __launch_bounds__(256) k_pp_chains(const PointProgram *__restric
 // shared-memory bank conflicts.  Per iteration of 1e6 points: 2->4, 15 x 10
 // searches per point, 0.43 ms; 2->6, 45 x 16 searches, 1.57 ms (the hinted
 // binary searches this replaces: 0.58 and 4.89 ms).
-constexpr int channel_max_threads(int dims) { return dims > 10 && dims <= 16 ? 1024 : 512; }
-
 template <int DIMS, bool TAB, int F, bool REC>
 __global__ void __launch_bounds__(channel_max_threads(DIMS), DIMS > 16 ? 1 : 1024 / channel_max_threads(DIMS)) k_pp_channel(
     const PointProgram *__restrict__ pp, GridTables T, int bins, const double *__restrict__ memo,

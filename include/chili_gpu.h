@@ -221,8 +221,10 @@ uint64_t chili_gpu_launch_count(const chili_ctx *ctx);
  * rejected points and NaN values counting as zero-valued calls.  Read by
  * chili_gpu_batch_set.
  * "channel_tables": 1 (default) stages each channel's cell and width tables
- * in shared memory for the bin searches of the phased weight pass (where they
- * fit a block), 0 reads them from global memory; the same numbers.
+ * in shared memory for the bin searches of the phased weight pass, 0 reads them
+ * from global memory; the same numbers.  Tables above 200 KB are always read
+ * from global memory, and those of batched tasks above 110 KB unless the task
+ * has 11 to 16 dimensions.
  * "flow_streamed": 1 runs a learned proposal of 2 x 128 hidden units on the
  * streamed-weight coupling kernels that wider or deeper conditioners always
  * use (the same function; a cross-check of the two kernel families), 0

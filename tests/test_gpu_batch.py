@@ -233,3 +233,22 @@ def test_graph_recapture_on_changed_calls(ctx_factory):
         ea, aa = a.batch_get_grid(k)
         eb, ab = b.batch_get_grid(k)
         assert np.max(rel(ea, eb)) < 1e-7 and np.max(rel(aa, ab)) < 1e-7
+
+
+@pytest.mark.parametrize("retry", [0, 1])
+def test_tasks_of_many_table_sizes_in_one_wave(ctx_factory, retry):
+    """Tasks of one dimension whose channel tables take 25 to 390 KB, some in
+    shared memory and some not: the values of the first iteration are those of
+    the same tasks with every table in global memory, bit for bit."""
+    tasks = [mc_task(n_out, 1000.0, 3000 + 37 * k, bins, cuts=retry == 1)
+             for k, (n_out, bins) in enumerate([(4, 50), (4, 300), (3, 400), (4, 100), (5, 200), (4, 255), (4, 256),
+                                                (5, 64), (4, 1000), (3, 65)])]
+    got = []
+    for tables in (1, 0):
+        ctx = ctx_factory()
+        ctx.set_option("channel_tables", tables)
+        ctx.set_option("batch_retry", retry)
+        ctx.batch_set(tasks)
+        got.append(ctx.batch_iterate(1, seed=11)[0])
+    assert np.array_equal(got[0], got[1])
+    assert (got[0][0, :, 0] > 0).all() and (got[0][0, :, 5] > 0).all()
