@@ -365,17 +365,23 @@ int launch_pipeline(chili_ctx *ctx, const double *mom_soa, const int32_t *ich, l
                         });
 }
 
-// The search tables of the grid set (grid.cuh), rebuilt after every change of
-// the edges.
-int rebuild_hints(chili_ctx *ctx) {
-    ctx->hints_stale = false;
+// Memory for the search tables of the grid set (grid.cuh).
+cudaError_t size_tables(chili_ctx *ctx) {
     const size_t rows = static_cast<size_t>(ctx->g_nch) * ctx->dims;
-    CK(ctx->cells.ensure(sizeof(uint32_t) * rows * grid_cells(ctx->bins)));
-    CK(ctx->widths.ensure(sizeof(double) * rows * width_row(ctx->bins)));
+    const cudaError_t e = ctx->cells.ensure(sizeof(uint32_t) * rows * grid_cells(ctx->bins));
+    return e != cudaSuccess ? e : ctx->widths.ensure(sizeof(double) * rows * width_row(ctx->bins));
+}
+
+// The search tables, rebuilt after every change of the edges; they stay marked
+// stale when this fails.
+int rebuild_hints(chili_ctx *ctx) {
+    ctx->hints_stale = true;
+    CK(size_tables(ctx));
     k_build_cells<<<dim3(ctx->dims, ctx->g_nch), 256, 0, ctx->stream>>>(
         ctx->edges.as<double>(), ctx->dims, ctx->bins, ctx->cells.as<uint32_t>(), ctx->widths.as<double>(),
         TrainGate{});
     LAUNCHED();
+    ctx->hints_stale = false;
     return CHILI_OK;
 }
 
@@ -710,6 +716,7 @@ static int adapt_grids(chili_ctx *ctx, int first, int count, double alpha, const
 // The caller swaps the edge buffers once it knows that the gate was open.
 static int queue_training(chili_ctx *ctx, const chili_multichannel_params *params, TrainGate gate) {
     const int D = ctx->dims, B = ctx->bins;
+    CK(size_tables(ctx));  // an iteration without the phased pass has not used them
     KTimer kt_(ctx, KT_ITER_END);
     k_alpha_update<<<1, 256, 0, ctx->stream>>>(alpha_ptr(ctx), best_ptr(ctx), mindiff_ptr(ctx), cp_ptr(ctx),
                                                acc_train_ptr(ctx), ctx->nch, params->beta, params->min_alpha, 1, gate);
