@@ -156,3 +156,39 @@ def test_calls_of_changing_size_on_one_context(ctx_factory):
         got, want = ctx.generate(n, seed=n), ref.generate(n, seed=n)
         for a, b in zip(got, want):
             assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [1000, 70000])
+def test_captured_calls_allocate_nothing_and_replay_the_same_bits(ctx_factory, n):
+    """On a stream that is being captured the calls take the per-thread
+    kernels, which need no buffers of the context; a replay on other inputs in
+    the same buffers gives what an eager, tiled call gives."""
+    import torch
+
+    ctx = _context(ctx_factory, 4, 1)
+    dev = _device_points(ctx, n)
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    eager = [_weigh(ctx, dev), _weigh(ctx, dev)]
+    out = [torch.zeros(n, 6, 4, dtype=torch.float64, device="cuda"), torch.zeros(n, dtype=torch.float64, device="cuda"),
+           torch.zeros(n, dtype=torch.int32, device="cuda")]
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        before = ctx.launches
+        ctx.call("chili_gpu_multichannel_weight", *(C.c_void_p(t.data_ptr()) for t in dev), None, None, n)
+        ctx.call("chili_gpu_generate", n, 5, 9, *(C.c_void_p(t.data_ptr()) for t in out))
+        assert ctx.launches - before == 2
+    for seed in (3, 4):
+        mom, w, ich = ctx.generate(n, seed=seed)
+        dev[0].copy_(torch.from_numpy(mom))
+        dev[1].copy_(torch.from_numpy(ich))
+        dev[2].zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        want = eager[1] if seed == 3 else ctx.multichannel_weight(mom, ich)[0]
+        assert np.array_equal(dev[2].cpu().numpy(), want, equal_nan=True)
+    assert np.array_equal(eager[0], eager[1], equal_nan=True)
+    for a, b in zip(out, ctx.generate(n, seed=5, counter=9)):
+        assert np.array_equal(a.cpu().numpy(), b, equal_nan=True)
