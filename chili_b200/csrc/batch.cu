@@ -1188,10 +1188,8 @@ int enqueue_final(chili_ctx *ctx, bool adapt) {
     k_batch_finalize<<<static_cast<unsigned>(S.tasks.size()), kFoldThreads, 0, ctx->stream>>>(B, adapt ? 1 : 0);
     LAUNCHED();
     if (adapt && !S.jobs.empty()) {
-        const size_t scratch = adapt_scratch_bytes(S.max_bins);
-        if (scratch > 48 * 1024)
-            CK(cudaFuncSetAttribute(k_batch_adapt, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scratch)));
-        k_batch_adapt<<<static_cast<unsigned>(S.jobs.size()), 64, scratch, ctx->stream>>>(
+        static_assert(adapt_scratch_bytes(CHILI_MAX_BINS) <= 48 * 1024, "within the default limit");
+        k_batch_adapt<<<static_cast<unsigned>(S.jobs.size()), 64, adapt_scratch_bytes(S.max_bins), ctx->stream>>>(
             B, S.d_jobs.as<AdaptJob>(), static_cast<int>(S.jobs.size()), S.d_status.as<int>());
         LAUNCHED();
         k_batch_commit<<<static_cast<unsigned>(S.jobs.size()), 128, 0, ctx->stream>>>(

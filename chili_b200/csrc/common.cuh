@@ -72,15 +72,6 @@ __device__ __forceinline__ double phi_0_2pi(V4 a) {
     if (p < 0) return p + kTwoPi;
     return p;
 }
-__device__ __forceinline__ double comp(const V4 &a, int i) {
-    return i == 0 ? a.e : (i == 1 ? a.x : (i == 2 ? a.y : a.z));
-}
-__device__ __forceinline__ void set_comp(V4 &a, int i, double v) {
-    if (i == 0) a.e = v;
-    else if (i == 1) a.x = v;
-    else if (i == 2) a.y = v;
-    else a.z = v;
-}
 
 // ---------------------------------------------------------------- Philox
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, "Parallel random numbers: as easy

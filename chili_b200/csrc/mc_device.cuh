@@ -249,7 +249,7 @@ __device__ __forceinline__ void alpha_update(double *__restrict__ alpha, double 
 
 // Shared-memory bytes of the adaptation of one row: the factors (doubles)
 // and the bins that the edges fall in (halfwords).
-__host__ __device__ inline size_t adapt_scratch_bytes(int bins) {
+__host__ __device__ constexpr size_t adapt_scratch_bytes(int bins) {
     return sizeof(double) * (static_cast<size_t>(bins) + (bins + 3) / 4);
 }
 
