@@ -460,11 +460,11 @@ KERNEL_COUNTERS = {
                      "source": "profiles/multichannel_2to4_kernels.md"},
     "k_pp_nodes": {"fp64_ops_per_point": 24.0, "dram_bytes_per_point": 840.1, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
-    "k_pp_items": {"fp64_ops_per_point": 7453.3, "dram_bytes_per_point": 1332.5, "basis": "weighted",
+    "k_pp_items": {"fp64_ops_per_point": 7393.3, "dram_bytes_per_point": 1327.9, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
     "k_pp_chains": {"fp64_ops_per_point": 2926.0, "dram_bytes_per_point": 624.6, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
-    "k_pp_channel": {"fp64_ops_per_point": 510.6, "dram_bytes_per_point": 970.5, "basis": "weighted",
+    "k_pp_channel": {"fp64_ops_per_point": 555.6, "dram_bytes_per_point": 969.8, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
     "k_pp_combine": {"fp64_ops_per_point": 724.0, "dram_bytes_per_point": 415.5, "basis": "weighted",
                      "source": "profiles/multichannel_2to4_kernels.md"},
